@@ -45,8 +45,8 @@ struct BlendCtl {
     unsigned long long sum1[3], sum2[3], n_ov, sq;
     float gain[3];
     int have_ov, vertical, first_side;  // first_side: image 1 left of (vertical) / above the seam
-    int line0, line1;                   // first and last DP line holding overlap
     int n_lines, seam_end;              // overlap lines; seam position on the last one
+    int band_lo, band_hi;               // union of the overlap lines' ranges
     int chunk;                          // backtrack chunk length
     int hist;                           // colour matching: 0 gain, 1 histograms (pysift/core.py:3694-3699)
     unsigned int hist1[3][256], hist2[3][256];  // overlap histograms of images 1 and 2
@@ -224,10 +224,13 @@ __device__ void block_sum6(long long v[6], long long* sh /* [32][6] */) {
 
 // gain (pysift/core.py:3692-3699) and the seam orientation (pysift/core.py:3424-3438)
 __global__ void __launch_bounds__(1024) k_blend_decide(BlendCtl* ctl, const int* __restrict__ rowf,
-                                                       const int* __restrict__ colf, int cw, int ch, int hist) {
+                                                       const int* __restrict__ colf, const int* __restrict__ rlo,
+                                                       const int* __restrict__ rhi, const int* __restrict__ clo,
+                                                       const int* __restrict__ chi, int cw, int ch, int hist,
+                                                       int* __restrict__ ovl) {
     __shared__ long long sh[32 * 6];
     __shared__ long long s_rows[6];
-    __shared__ int s_lo, s_hi;
+    __shared__ int s_lo, s_hi, s_scan[33];
     // rows: {n overlap rows, n rows with image 1 only, sum of their indices, same for image 2, -}
     long long v[6] = {0, 0, 0, 0, 0, 0};
     for (int r = threadIdx.x; r < ch; r += blockDim.x) {
@@ -275,18 +278,33 @@ __global__ void __launch_bounds__(1024) k_blend_decide(BlendCtl* ctl, const int*
         s_hi = -1;
     }
     __syncthreads();
+    // the overlap lines in order and the band they cover
     const bool vert = ctl->vertical != 0;
     const int L = vert ? ch : cw;
     const int* lf = vert ? rowf : colf;
-    for (int i = threadIdx.x; i < L; i += blockDim.x)
-        if (lf[i] & 1) {
-            atomicMin(&s_lo, i);
-            atomicMax(&s_hi, i);
-        }
+    const int* lo_of = vert ? rlo : clo;
+    const int* hi_of = vert ? rhi : chi;
+    int lo = 0x7fffffff, hi = -1;
+    const int nL = block_compact<2, int>(
+        L, [&](int i) { return (lf[i] & 1) ? i : -1; }, [](int line) { return line >= 0; },
+        [&](int pos, int line) {
+            ovl[pos] = line;
+            lo = min(lo, lo_of[line]);
+            hi = max(hi, hi_of[line]);
+        },
+        s_scan);
+    if (hi >= 0) {
+        atomicMin(&s_lo, lo);
+        atomicMax(&s_hi, hi);
+    }
     __syncthreads();
     if (threadIdx.x == 0) {
-        ctl->line0 = s_lo;
-        ctl->line1 = s_hi;
+        ctl->n_lines = nL;
+        ctl->band_lo = s_lo;
+        ctl->band_hi = s_hi;
+        int R = 16;
+        while (2 * R * R < nL) R *= 2;
+        ctl->chunk = R;
     }
 }
 
@@ -392,12 +410,18 @@ __global__ void k_blend_prepare(const Img1 w1, const uint8_t* __restrict__ m1,
 // axis (antisymmetric: x[i+1] - x[i-1]) rounded to float32, then [1, 2, 1]
 // along the other (2 x[i] + (x[i-1] + x[i+1])), both in float64 with
 // half-sample reflection.  The DP reads `dpc`: the cost where both images
-// cover the canvas, else -1, line by line (transposed for a horizontal seam).
+// cover the canvas, else -1, line by line (transposed for a horizontal seam),
+// at a pitch of a multiple of 4 with -1 in the padding.
 __global__ void k_sobel_cost(const float* __restrict__ avg, const float* __restrict__ color,
                              const uint8_t* __restrict__ m1, const uint8_t* __restrict__ m2, const BlendCtl* ctl,
                              float* __restrict__ dpc, int W, int H) {
     const int x = blockIdx.x * blockDim.x + threadIdx.x, y = blockIdx.y;
-    if (x >= W) return;
+    const bool vert = ctl->vertical != 0;
+    const int Wp = (W + 3) & ~3, Hp = (H + 3) & ~3;
+    if (x >= W) {
+        if (vert && x < Wp) dpc[(long long)y * Wp + x] = -1.0f;
+        return;
+    }
     const long long p = (long long)y * W + x;
     const int xl = refl_half(x - 1, W), xr = refl_half(x + 1, W);
     const int yu = refl_half(y - 1, H), yd = refl_half(y + 1, H);
@@ -411,172 +435,244 @@ __global__ void k_sobel_cost(const float* __restrict__ avg, const float* __restr
     const float gy = (float)(2.0 * dyc(x) + (dyc(xl) + dyc(xr)));
     const float c = color[p] + 0.05f * sqrtf(gx * gx + gy * gy);
     const float out = (m1[p] && m2[p]) ? c : -1.0f;
-    if (ctl->vertical) dpc[p] = out;
-    else dpc[(long long)x * H + y] = out;
+    if (vert) {
+        dpc[(long long)y * Wp + x] = out;
+    } else {
+        dpc[(long long)x * Hp + y] = out;
+        if (y == H - 1)
+            for (int t = H; t < Hp; ++t) dpc[(long long)x * Hp + t] = -1.0f;
+    }
 }
 
-__device__ __forceinline__ void bl_cp_async4(void* dst, const void* src) {
-    const unsigned d = (unsigned)__cvta_generic_to_shared(dst);
-    asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(d), "l"(src) : "memory");
+// ---------------------------------------------------------------------------
+// Dynamic-programming seam, forward pass (pysift/core.py:3286-3383): the
+// overlap lines in order (rows for a vertical seam, columns for a horizontal
+// one), D[q][j] = cost + min(D[q-1][j-1], D[q-1][j], D[q-1][j+1]) in float64
+// with numpy's first-minimum order; INF where the images do not both cover
+// the canvas.  dir[line][j] = argmin (0 left, 1 centre, 2 right).
+//
+// The lines are a serial chain, so the time is (lines) x (latency of one
+// line).  One cluster of DP_CTAS CTAs holds the band (the union of the
+// overlap ranges; every value outside it is INF) in registers: a warp keeps
+// 32 E consecutive positions, E a lane, neighbours by shuffle, and advances
+// DP_B lines without any synchronisation while its outermost positions go
+// stale one per line and side; then it hands the DP_B positions at each of
+// its net ends to the neighbouring warps through (distributed) shared memory
+// and one cluster barrier.  The cost lines are loaded DP_B lines ahead into
+// registers.  Spreading the warps over eight SMs leaves a scheduler at most
+// two of them, so a line costs its own shuffle -> 2 x (compare, select) ->
+// add chain and not the issue slots of the whole line: a line took 0.37 us
+// with the band in one CTA's shared memory and a block barrier per line.
+// ---------------------------------------------------------------------------
+constexpr int DP_CTAS = 8, DP_WARPS = 4, DP_T = 32 * DP_WARPS, DP_B = 16;
+template <int E>
+__host__ __device__ constexpr int dp_net() { return 32 * E - 2 * DP_B; }
+
+__device__ __forceinline__ void dp_cluster_sync() {
+    asm volatile("barrier.cluster.arrive.release.aligned;\nbarrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
-__device__ __forceinline__ void bl_cp_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
-template <int N>
-__device__ __forceinline__ void bl_cp_wait() {
-    asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory");
+__device__ __forceinline__ unsigned dp_cluster_rank() {
+    unsigned r;
+    asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
+    return r;
+}
+// store into the shared memory of CTA `rank` of the cluster, at the place of this CTA's `p`
+__device__ __forceinline__ void dp_remote_store(double* p, unsigned rank, double v) {
+    const unsigned a = (unsigned)__cvta_generic_to_shared(p);
+    unsigned r;
+    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(a), "r"(rank));
+    asm volatile("st.shared::cluster.f64 [%0], %1;" ::"r"(r), "d"(v) : "memory");
 }
 
-// Dynamic-programming seam, forward pass (pysift/core.py:3286-3383), in one
-// CTA: overlap lines in order (rows for a vertical seam, columns for a
-// horizontal one), positions in parallel.  Line q only computes its window:
-// its own overlap range widened to one past the previous overlap line's range.
-// Outside it all three predecessors are INF, so the DP value is INF and the
-// argmin is 0 (dir is cleared beforehand).  The DP lines hold INF outside the
-// window (positions of the line before last that fall outside are reset) and
-// carry one INF sentinel at each end.  With K > 0 the cost lines stream
-// through a K-deep cp.async ring, each thread copying the positions it reads.
-// Outputs: dir[line][pos] = argmin (0 left, 1 centre, 2 right), the compacted
-// overlap lines, and in ctl their count and the seam position on the last one
-// (numpy's first minimum over the whole line).
-template <int K>
-__global__ void __launch_bounds__(1024) k_blend_dp(const float* __restrict__ dpc, const int* __restrict__ rowf,
-                                                   const int* __restrict__ colf, const int* __restrict__ rlo,
-                                                   const int* __restrict__ rhi, const int* __restrict__ clo,
-                                                   const int* __restrict__ chi, int cw, int ch, BlendCtl* ctl,
-                                                   double* __restrict__ gA, double* __restrict__ gB,
-                                                   int4* __restrict__ gwin, int in_global,
-                                                   uint8_t* __restrict__ dir, int* __restrict__ ovl) {
-    extern __shared__ __align__(16) unsigned char dsm[];
-    __shared__ int s_sh[33];
-    __shared__ double s_best[32];
-    __shared__ int s_idx[32];
-    if (!ctl->have_ov) return;
-    const bool vert = ctl->vertical != 0;
-    const int L = vert ? ch : cw, M = vert ? cw : ch;
-    const int* lf = vert ? rowf : colf;
-    const int* lo_of = vert ? rlo : clo;
-    const int* hi_of = vert ? rhi : chi;
-    const int nfw = (L + 31) >> 5;
-    const int tid = threadIdx.x, nt = blockDim.x;
-    // shared layout: line bitmask | windows {lo, hi, line} | the two DP lines (M + 2 each) | ring
-    unsigned* fl = reinterpret_cast<unsigned*>(dsm);
-    size_t off = ((size_t)nfw * 4 + 15) & ~(size_t)15;
-    int4* win = in_global ? gwin : reinterpret_cast<int4*>(dsm + off);
-    if (!in_global) off += (size_t)L * 16;
-    double* lineA = in_global ? gA : reinterpret_cast<double*>(dsm + off);
-    double* lineB = in_global ? gB : lineA + (M + 2);
-    if (!in_global) off += (size_t)(M + 2) * 16;
-    float* ring = reinterpret_cast<float*>(dsm + off);
-    // overlap-line bitmask and the compacted list of overlap lines
-    const int per = (nfw + nt - 1) / nt;
-    const int w0 = min(nfw, tid * per), w1 = min(nfw, (tid + 1) * per);
-    int cnt = 0;
-    for (int w = w0; w < w1; ++w) {
-        unsigned b = 0u;
-        for (int k = 0; k < 32; ++k) {
-            const int i = (w << 5) + k;
-            if (i < L && (lf[i] & 1)) b |= 1u << k;
-        }
-        fl[w] = b;
-        cnt += __popc(b);
-    }
-    int nL;
-    int base = block_excl_scan(cnt, &nL, s_sh);
-    for (int w = w0; w < w1; ++w) {
-        unsigned b = fl[w];
-        while (b) {
-            const int k = __ffs(b) - 1;
-            b &= b - 1u;
-            const int line = (w << 5) + k;
-            const int lo = lo_of[line], hi = hi_of[line];
-            int4 wn = make_int4(lo, hi, line, 0);
-            if (base > 0) {
-                // the previous overlap line: the highest set bit below `line`
-                int pw = line >> 5;
-                unsigned pb = fl[pw] & ((1u << (line & 31)) - 1u);
-                while (!pb) pb = fl[--pw];  // base > 0: an earlier overlap line exists
-                const int pline = (pw << 5) + 31 - __clz(pb);
-                wn.x = max(0, min(lo_of[pline] - 1, lo));
-                wn.y = min(M - 1, max(hi_of[pline] + 1, hi));
-            }
-            win[base] = wn;
-            ovl[base++] = line;
-        }
-    }
-    for (int j = tid; j < M + 2; j += nt) {
-        lineA[j] = BL_INF;
-        lineB[j] = BL_INF;
-    }
-    __syncthreads();
-    double* prev = lineA + 1;  // prev[-1] and prev[M] stay INF
-    double* cur = lineB + 1;
+struct DpBand {
+    const float* dpc;  // cost lines, pitch Mp floats (a multiple of 4), -1 outside the overlap and past M
+    const int* ovl;    // overlap lines in order
+    int nL, M, Mp;
+    int lo, hi;        // band, lo a multiple of 4
+    uint8_t* dir;      // pitch Mp
+    double* end;       // D of the last line, written inside the band
+};
+
+// halo[parity][side][warp]: the DP_B values left (side 0) / right (side 1) of a warp's net positions
+typedef double DpHalo[2][2][DP_WARPS][DP_B];
+
+template <int E>
+__device__ __forceinline__ void dp_band(const DpBand& a, DpHalo& halo) {
+    constexpr int NET = dp_net<E>(), NQ = E / 4, HL = DP_B / E;  // HL lanes hold a halo
+    const unsigned rank = dp_cluster_rank();
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int nseg = (a.hi - a.lo) / NET + 1, per = (nseg + DP_CTAS - 1) / DP_CTAS;
+    const int seg = (int)rank * per + warp;
+    const bool on = warp < per && seg < nseg;  // other warps only take part in the barriers
+    const int pos = a.lo + seg * NET - DP_B + lane * E;
+    const bool net = on && lane >= HL && lane < 32 - HL;
+    bool in[NQ];
+#pragma unroll
+    for (int k = 0; k < NQ; ++k) in[k] = on && pos + 4 * k >= 0 && pos + 4 * k < a.Mp;
+    auto load = [&](int line, float4 c[NQ]) {
+        const float* src = a.dpc + (long long)line * a.Mp + pos;
+#pragma unroll
+        for (int k = 0; k < NQ; ++k)
+            c[k] = in[k] ? __ldg(reinterpret_cast<const float4*>(src) + k) : make_float4(-1.0f, -1.0f, -1.0f, -1.0f);
+    };
+    double p[E];
+    float4 ring[DP_B][NQ];
     {
-        const int4 w = win[0];
-        const float* crow = dpc + (long long)w.z * M;
-        for (int j = w.x + tid; j <= w.y; j += nt) {
-            const float c = crow[j];
-            prev[j] = c >= 0.0f ? (double)c : BL_INF;
+        float4 c[NQ];
+        load(a.ovl[0], c);
+#pragma unroll
+        for (int k = 0; k < NQ; ++k) {
+            const float v[4] = {c[k].x, c[k].y, c[k].z, c[k].w};
+#pragma unroll
+            for (int e = 0; e < 4; ++e) p[4 * k + e] = v[e] >= 0.0f ? (double)v[e] : BL_INF;
         }
     }
-    constexpr int KR = K > 0 ? K : 1;
-    if (K > 0) {
-        for (int s = 0; s < K - 1; ++s) {
-            const int q = 1 + s;
-            if (q < nL) {
-                const int4 w = win[q];
-                const float* src = dpc + (long long)w.z * M;
-                float* slot = ring + (size_t)s * M;
-                for (int j = w.x + tid; j <= w.y; j += nt) bl_cp_async4(slot + j, src + j);
+    int ids = lane < DP_B && 1 + lane < a.nL ? a.ovl[1 + lane] : -1;  // this block's lines
+#pragma unroll
+    for (int t = 0; t < DP_B; ++t) {
+        const int line = __shfl_sync(0xffffffffu, ids, t);
+        if (line >= 0) load(line, ring[t]);
+    }
+    int parity = 0;
+    for (int q0 = 1; q0 < a.nL; q0 += DP_B) {
+        const int qn = q0 + DP_B + lane;
+        const int next = lane < DP_B && qn < a.nL ? a.ovl[qn] : -1;
+#pragma unroll
+        for (int t = 0; t < DP_B; ++t) {
+            if (q0 + t >= a.nL) break;
+            const int line = __shfl_sync(0xffffffffu, ids, t);
+            // the outermost lanes read themselves: those positions are stale by now
+            const double left = __shfl_up_sync(0xffffffffu, p[E - 1], 1);
+            const double right = __shfl_down_sync(0xffffffffu, p[0], 1);
+            double o[E];
+            unsigned d[NQ];
+#pragma unroll
+            for (int k = 0; k < NQ; ++k) {
+                const float v[4] = {ring[t][k].x, ring[t][k].y, ring[t][k].z, ring[t][k].w};
+                d[k] = 0u;
+#pragma unroll
+                for (int e = 0; e < 4; ++e) {
+                    const int i = 4 * k + e;
+                    const double pl = i ? p[i - 1] : left, pm = p[i], pr = i + 1 < E ? p[i + 1] : right;
+                    unsigned m = 0u;
+                    double best = pl;
+                    if (pm < best) { best = pm; m = 1u << (8 * e); }
+                    if (pr < best) { best = pr; m = 2u << (8 * e); }
+                    d[k] |= m;
+                    o[i] = v[e] >= 0.0f ? (double)v[e] + best : BL_INF;
+                }
             }
-            bl_cp_commit();
+#pragma unroll
+            for (int i = 0; i < E; ++i) p[i] = o[i];
+            if (net) {
+                uint8_t* row = a.dir + (long long)line * a.Mp + pos;
+#pragma unroll
+                for (int k = 0; k < NQ; ++k)
+                    if (in[k]) reinterpret_cast<unsigned*>(row)[k] = d[k];
+            }
+            const int after = __shfl_sync(0xffffffffu, next, t);
+            if (after >= 0) load(after, ring[t]);
+        }
+        ids = next;
+        if (q0 + DP_B < a.nL) {
+            // the values written at one exchange are read before the next
+            // barrier, so two sets of slots are enough
+            if (on) {
+                if (lane >= HL && lane < 2 * HL && seg > 0) {
+                    const int s = seg - 1;
+#pragma unroll
+                    for (int i = 0; i < E; ++i)
+                        dp_remote_store(&halo[parity][1][s % per][(lane - HL) * E + i], (unsigned)(s / per), p[i]);
+                }
+                if (lane >= 32 - 2 * HL && lane < 32 - HL && seg + 1 < nseg) {
+                    const int s = seg + 1;
+#pragma unroll
+                    for (int i = 0; i < E; ++i)
+                        dp_remote_store(&halo[parity][0][s % per][(lane - 32 + 2 * HL) * E + i], (unsigned)(s / per),
+                                        p[i]);
+                }
+            }
+            dp_cluster_sync();
+            // past the first and last warp lies no band: INF
+            if (on && lane < HL) {
+#pragma unroll
+                for (int i = 0; i < E; ++i) p[i] = seg > 0 ? halo[parity][0][warp][lane * E + i] : BL_INF;
+            }
+            if (on && lane >= 32 - HL) {
+#pragma unroll
+                for (int i = 0; i < E; ++i)
+                    p[i] = seg + 1 < nseg ? halo[parity][1][warp][(lane - 32 + HL) * E + i] : BL_INF;
+            }
+            parity ^= 1;
         }
     }
-    __syncthreads();
-    for (int q = 1; q < nL; ++q) {
-        const int4 w = win[q];
-        const float* crow;
-        if (K > 0) {
-            const int qn = q + K - 1;
-            if (qn < nL) {
-                const int4 wn = win[qn];
-                const float* src = dpc + (long long)wn.z * M;
-                float* slot = ring + (size_t)((q + K - 2) % KR) * M;
-                for (int j = wn.x + tid; j <= wn.y; j += nt) bl_cp_async4(slot + j, src + j);
+    if (net) {
+#pragma unroll
+        for (int i = 0; i < E; ++i)
+            if (pos + i < a.M) a.end[pos + i] = p[i];
+    }
+}
+
+// Bands wider than the cluster's registers: one CTA, the two DP lines in
+// global memory, a block barrier per line.
+__device__ __noinline__ void dp_wide(const DpBand& a, double* prev, double* cur) {
+    const int tid = threadIdx.x;
+    for (int q = 0; q < a.nL; ++q) {
+        const long long row = (long long)a.ovl[q] * a.Mp;
+        for (int j = a.lo + tid; j <= a.hi; j += DP_T) {
+            const float c = a.dpc[row + j];
+            double best = 0.0;
+            if (q > 0) {
+                const double pl = j > a.lo ? prev[j - 1] : BL_INF, pm = prev[j], pr = j < a.hi ? prev[j + 1] : BL_INF;
+                int m = 0;
+                best = pl;
+                if (pm < best) { best = pm; m = 1; }
+                if (pr < best) { best = pr; m = 2; }
+                a.dir[row + j] = (uint8_t)m;
             }
-            bl_cp_commit();
-            bl_cp_wait<KR - 1>();
-            crow = ring + (size_t)((q - 1) % KR) * M;
-        } else {
-            crow = dpc + (long long)w.z * M;
-        }
-        // positions of the line before last outside this window go back to INF
-        if (q >= 2) {
-            const int4 o = win[q - 2];
-            for (int j = o.x + tid; j < min(o.y + 1, w.x); j += nt) cur[j] = BL_INF;
-            for (int j = max(o.x, w.y + 1) + tid; j <= o.y; j += nt) cur[j] = BL_INF;
-        }
-        uint8_t* drow = dir + (long long)w.z * M;
-        for (int j = w.x + tid; j <= w.y; j += nt) {
-            const float c = crow[j];
-            const double pl = prev[j - 1], pm = prev[j], pr = prev[j + 1];
-            int a = 0;
-            double best = pl;
-            if (pm < best) { best = pm; a = 1; }
-            if (pr < best) { best = pr; a = 2; }
             cur[j] = c >= 0.0f ? (double)c + best : BL_INF;
-            if (a) drow[j] = (uint8_t)a;
         }
         __syncthreads();
         double* t = prev;
         prev = cur;
         cur = t;
     }
-    if (K > 0) bl_cp_wait<0>();
+    if (prev != a.end)
+        for (int j = a.lo + tid; j <= a.hi; j += DP_T) a.end[j] = prev[j];
+}
+
+__global__ void __cluster_dims__(DP_CTAS, 1, 1) __launch_bounds__(DP_T)
+    k_blend_dp(const float* __restrict__ dpc, const int* __restrict__ ovl, int cw, int ch, BlendCtl* ctl, double* gA,
+               double* gB, uint8_t* __restrict__ dir) {
+    __shared__ DpHalo halo;
+    __shared__ double s_best[DP_WARPS];
+    __shared__ int s_idx[DP_WARPS];
+    if (!ctl->have_ov) return;
+    const int tid = threadIdx.x;
+    DpBand a;
+    a.dpc = dpc;
+    a.ovl = ovl;
+    a.nL = ctl->n_lines;
+    a.M = ctl->vertical ? cw : ch;
+    a.Mp = (a.M + 3) & ~3;
+    a.lo = ctl->band_lo & ~3;
+    a.hi = ctl->band_hi;
+    a.dir = dir;
+    a.end = gA;
+    const unsigned rank = dp_cluster_rank();
+    dp_cluster_sync();  // every CTA of the cluster has started before its shared memory is written
+    const int width = a.hi - a.lo + 1;
+    if (width <= DP_CTAS * DP_WARPS * dp_net<4>()) dp_band<4>(a, halo);
+    else if (width <= DP_CTAS * DP_WARPS * dp_net<8>()) dp_band<8>(a, halo);
+    else if (rank == 0) dp_wide(a, gB, gA);
+    dp_cluster_sync();
+    if (rank != 0) return;
     // first minimum of the last overlap line (non-overlap positions count as INF)
-    const int last = win[nL - 1].z;
+    const float* last = dpc + (long long)ovl[a.nL - 1] * a.Mp;
     double bv = BL_INF * 4.0;
     int bj = 0x7fffffff;
-    for (int j = tid; j < M; j += nt) {
-        const double vv = dpc[(long long)last * M + j] >= 0.0f ? prev[j] : BL_INF;
+    for (int j = tid; j < a.M; j += DP_T) {
+        const double vv = last[j] >= 0.0f ? gA[j] : BL_INF;
         if (vv < bv) { bv = vv; bj = j; }
     }
 #pragma unroll
@@ -591,20 +687,16 @@ __global__ void __launch_bounds__(1024) k_blend_dp(const float* __restrict__ dpc
     }
     __syncthreads();
     if (tid == 0) {
-        for (int w = 1; w < (nt >> 5); ++w)
+        for (int w = 1; w < DP_WARPS; ++w)
             if (s_best[w] < bv || (s_best[w] == bv && s_idx[w] < bj)) { bv = s_best[w]; bj = s_idx[w]; }
         ctl->seam_end = bj;
-        ctl->n_lines = nL;
-        int R = 16;
-        while (2 * R * R < nL) R *= 2;
-        ctl->chunk = R;
     }
 }
 
 // one backtrack step from overlap line q (position p) to overlap line q - 1
 __device__ __forceinline__ int bt_step(const uint8_t* __restrict__ dir, const int* __restrict__ ovl, int M, int q,
                                        int p) {
-    const int k = p + (int)dir[(long long)ovl[q] * M + p] - 1;
+    const int k = p + (int)dir[(long long)ovl[q] * ((M + 3) & ~3) + p] - 1;
     return k < 0 ? 0 : (k > M - 1 ? M - 1 : k);
 }
 
@@ -1022,9 +1114,6 @@ __global__ void k_place_image(const uint8_t* __restrict__ img, int h, int w, int
     if (mask) mask[p] = in;
 }
 
-constexpr int DP_SMEM_MAX = 200 * 1024;
-constexpr int DP_THREADS = 256;
-
 // backtrack chunks: the chunk length R (a power of two, at least 16, with
 // 2 R^2 >= the number of overlap lines, which balances the sequential walk of
 // about 2 R + lines / R steps) is chosen on the device, so there are at most
@@ -1053,7 +1142,7 @@ static cudaStream_t side_stream() {
 }
 
 struct BlendLayout {
-    size_t off_ctl, off_rowf, off_colf, off_rlo, off_rhi, off_clo, off_chi, off_win, off_color, off_avg, off_dpc,
+    size_t off_ctl, off_rowf, off_colf, off_rlo, off_rhi, off_clo, off_chi, off_color, off_avg, off_dpc,
         off_rowA, off_rowB, off_dir, off_seam, off_ovl, off_jump, off_entry, off_srow, off_t1,
         off_t2, off_tm;
     int nchunk;
@@ -1081,13 +1170,14 @@ static BlendLayout blend_layout(int cw, int ch, int levels) {
     l.off_rhi = take((size_t)ch * 4);
     l.off_clo = take((size_t)cw * 4);
     l.off_chi = take((size_t)cw * 4);
-    l.off_win = take((size_t)M * 16);
     l.off_color = take(N * 4);
     l.off_avg = take(N * 4);
-    l.off_dpc = take(N * 4);
-    l.off_rowA = take((size_t)(M + 2) * 8);
-    l.off_rowB = take((size_t)(M + 2) * 8);
-    l.off_dir = take(N);
+    // lines at a pitch of a multiple of 4, either way round
+    const size_t NP = std::max(align_up(cw, 4) * ch, align_up(ch, 4) * cw);
+    l.off_dpc = take(NP * 4);
+    l.off_rowA = take((size_t)M * 8);
+    l.off_rowB = take((size_t)M * 8);
+    l.off_dir = take(NP);
     l.off_seam = take((size_t)M * 4);
     l.off_ovl = take((size_t)M * 4);
     l.nchunk = max_seam_chunks(M);
@@ -1250,7 +1340,8 @@ int pysift_blend_multiband(const void* image1, int32_t image1_f32, const uint8_t
     k_blend_stats<<<dim3(1, ch), 256, 0, st>>>(w1, mask1, canvas2, mask2, cw, ctl, rowf, colf, rlo, rhi, clo, chi,
                                                 hist);
     PYSIFT_LAUNCH_CHECK("k_blend_stats");
-    k_blend_decide<<<1, 1024, 0, st>>>(ctl, rowf, colf, cw, ch, hist);
+    int* ovl = bwp<int>(ws, l.off_ovl);
+    k_blend_decide<<<1, 1024, 0, st>>>(ctl, rowf, colf, rlo, rhi, clo, chi, cw, ch, hist, ovl);
     PYSIFT_LAUNCH_CHECK("k_blend_decide");
     if (hist) {
         k_blend_hist_lut<<<3, 256, 0, st>>>(ctl);
@@ -1299,37 +1390,12 @@ int pysift_blend_multiband(const void* image1, int32_t image1_f32, const uint8_t
     // DP seam and backtrack
     int* seam = bwp<int>(ws, l.off_seam);
     {
-        int* ovl = bwp<int>(ws, l.off_ovl);
         uint8_t* dir = bwp<uint8_t>(ws, l.off_dir);
-        // the orientation is decided on the device: size shared memory for the longer side
         const int M = cw > ch ? cw : ch;
-        const size_t flags = (((size_t)(M + 31) / 32) * 4 + 15) & ~(size_t)15;
-        const size_t wins = (size_t)M * 16;
-        const size_t lines = (size_t)(M + 2) * 16;
-        double* gA = bwp<double>(ws, l.off_rowA);
-        double* gB = bwp<double>(ws, l.off_rowB);
-        int4* gwin = bwp<int4>(ws, l.off_win);
-        PYSIFT_CUDA_TRY(cudaMemsetAsync(dir, 0, (size_t)cw * ch, st));
-        const size_t base = flags + wins + lines;
-        if (base + (size_t)M * 32 <= (size_t)DP_SMEM_MAX) {
-            const size_t sm = base + (size_t)M * 32;
-            PYSIFT_CUDA_TRY(cudaFuncSetAttribute(k_blend_dp<8>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
-            k_blend_dp<8><<<1, DP_THREADS, sm, st>>>(dpc, rowf, colf, rlo, rhi, clo, chi, cw, ch, ctl, gA, gB, gwin, 0, dir,
-                                               ovl);
-        } else if (base + (size_t)M * 16 <= (size_t)DP_SMEM_MAX) {
-            const size_t sm = base + (size_t)M * 16;
-            PYSIFT_CUDA_TRY(cudaFuncSetAttribute(k_blend_dp<4>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
-            k_blend_dp<4><<<1, DP_THREADS, sm, st>>>(dpc, rowf, colf, rlo, rhi, clo, chi, cw, ch, ctl, gA, gB, gwin, 0, dir,
-                                               ovl);
-        } else if (base <= (size_t)DP_SMEM_MAX) {
-            PYSIFT_CUDA_TRY(cudaFuncSetAttribute(k_blend_dp<0>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)base));
-            k_blend_dp<0><<<1, DP_THREADS, base, st>>>(dpc, rowf, colf, rlo, rhi, clo, chi, cw, ch, ctl, gA, gB, gwin, 0, dir,
-                                                 ovl);
-        } else {
-            PYSIFT_CUDA_TRY(cudaFuncSetAttribute(k_blend_dp<0>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)flags));
-            k_blend_dp<0><<<1, DP_THREADS, flags, st>>>(dpc, rowf, colf, rlo, rhi, clo, chi, cw, ch, ctl, gA, gB, gwin, 1,
-                                                  dir, ovl);
-        }
+        const size_t dir_bytes = std::max(align_up(cw, 4) * ch, align_up(ch, 4) * cw);
+        PYSIFT_CUDA_TRY(cudaMemsetAsync(dir, 0, dir_bytes, st));
+        k_blend_dp<<<DP_CTAS, DP_T, 0, st>>>(dpc, ovl, cw, ch, ctl, bwp<double>(ws, l.off_rowA),
+                                             bwp<double>(ws, l.off_rowB), dir);
         PYSIFT_LAUNCH_CHECK("k_blend_dp");
         int* jump = bwp<int>(ws, l.off_jump);
         k_seam_jump<<<dim3(ceil_div(M, 256), l.nchunk), 256, 0, st>>>(dir, ovl, ctl, cw, ch, jump);

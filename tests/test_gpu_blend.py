@@ -148,6 +148,34 @@ def test_blend_degenerate_masks(seed):
     assert np.array_equal(pano, ref)
 
 
+@pytest.mark.parametrize("rows,lo,na,gap,nb", [
+    (97, 5, 93, 0, 0), (97, 4, 96, 0, 0), (98, 4, 97, 0, 0),      # one segment, full, one more
+    (772, 3, 769, 0, 0),                                           # more segments than CTAs
+    (16, 2, 9, 0, 0), (17, 2, 9, 0, 0), (18, 2, 9, 0, 0), (33, 2, 9, 0, 0),  # blocks of lines
+    (40, 1, 20, 3031, 20), (40, 4, 20, 3033, 20),                  # 3071 and 3073: 4 and 8 positions a lane
+    (40, 0, 20, 7128, 20), (40, 0, 20, 7129, 20),                  # 7168 and 7169: the widest band in registers
+])
+def test_blend_seam_band_edges(rows, lo, na, gap, nb):
+    """The DP's band (here columns lo .. lo + na + gap + nb, with no overlap in
+    the gap) at the edges of its segments, line blocks and widths."""
+    from oracle import blend_oracle as bo
+    rng = np.random.default_rng(rows + gap)
+    ch, cw = rows + 3, lo + na + gap + nb + 2
+    xx = np.mgrid[0:ch, 0:cw][1]
+    ov = ((xx >= lo) & (xx < lo + na)) | ((xx >= lo + na + gap) & (xx < lo + na + gap + nb))
+    ov[rows:] = False
+    m1, m2 = ov | (xx < lo), ov | (xx >= lo + na + gap + nb)
+    w1 = rng.integers(0, 256, (ch, cw, 3), dtype=np.uint8)
+    c2 = rng.integers(0, 256, (ch, cw, 3), dtype=np.uint8)
+    w1[~m1] = 0
+    c2[~m2] = 0
+    for a, ma, b, mb in ((w1, m1, c2, m2), (w1.transpose(1, 0, 2), m1.T, c2.transpose(1, 0, 2), m2.T)):
+        pano, both, _ = _run(a, ma, b, mb)
+        ref, ref_both = bo.blend_pair(a, ma, b, mb)
+        assert np.array_equal(both, ref_both)
+        assert np.array_equal(pano, ref)
+
+
 def test_blend_no_overlap_and_edges():
     """No overlap (no gain, no seam), an overlap of one column and one of one row."""
     from oracle import blend_oracle as bo
