@@ -336,6 +336,22 @@ int pysift_desc_f32_backward(const float* level, int32_t H, int32_t W, int32_t p
 int pysift_blur_adjoint(const float* gout, int32_t gout_pitch, float* gin, int32_t gin_pitch, float* tmp,
                         int32_t tmp_pitch, int32_t H, int32_t W, const float* weights_dev, int32_t radius,
                         int32_t accumulate, pysift_stream_t stream);
+/* The whole descriptor function over the keypoints of every level of the
+ * non-doubled pyramid of cfg: kp has n rows of 4 floats [octave *
+ * PYSIFT_MAX_LEVELS + scale index, centre row, centre column, angle in
+ * degrees]; octaves 0 .. n_octaves - 1 and levels 0 .. top (n_scales <= top <=
+ * n_scales + 2) of img (float, pitch in floats) are built in the workspace (a
+ * row of another level yields zeros).  backward rebuilds them and writes
+ * dL/dimg (gimg; each blur radius must be below both sides of its octave). */
+int pysift_desc_levels_workspace_size(const pysift_detect_config* cfg, int32_t H, int32_t W, int32_t n_octaves,
+                                      int32_t top, int32_t backward, size_t* bytes);
+int pysift_desc_levels_forward(const pysift_detect_config* cfg, const float* img, int32_t H, int32_t W, int32_t pitch,
+                               const float* kp, int32_t n, int32_t n_octaves, int32_t top, void* workspace,
+                               size_t workspace_bytes, float* hist, float* desc, pysift_stream_t stream);
+int pysift_desc_levels_backward(const pysift_detect_config* cfg, const float* img, int32_t H, int32_t W, int32_t pitch,
+                                const float* kp, int32_t n, int32_t n_octaves, int32_t top, void* workspace,
+                                size_t workspace_bytes, const float* hist, const float* gdesc, float* gimg,
+                                int32_t gimg_pitch, pysift_stream_t stream);
 int pysift_warp_f32_forward(const float* img1, int32_t hs, int32_t ws, int32_t C, const float* img2, int32_t h2,
                             int32_t w2, int32_t cw, int32_t ch, const double* hinv_host, double ox, double oy,
                             int32_t iox, int32_t ioy, float* out, pysift_stream_t stream);

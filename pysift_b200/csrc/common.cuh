@@ -47,11 +47,26 @@ void count_launch();
         }                                                                                  \
     } while (0)
 
+// One blurred level (detect.cu): in at `step` (1, or 2 to read every second
+// pixel, which copy0, if not null, receives), pitches in floats.
+int blur_level(const float* in, long long in_pitch, int step, float* out, int out_pitch, float* copy0, int H, int W,
+               const float* w, int R, cudaStream_t st);
+
 inline size_t align_up(size_t x, size_t a) { return (x + a - 1) / a * a; }
 __host__ __device__ inline int ceil_div(int a, int b) { return (a + b - 1) / b; }
 inline long long ceil_div_ll(long long a, long long b) { return (a + b - 1) / b; }
 
 __device__ __forceinline__ float round_half(float v) { return __half2float(__float2half_rn(v)); }
+
+// Half-sample-symmetric reflection into [0, n) (period 2n), as the
+// reference's reflect() (pysift/core.py:477-483), without integer division.
+__device__ __forceinline__ int reflect_idx(int i, int n) {
+    while (i < 0 || i >= n) {
+        if (i < 0) i = -i - 1;
+        if (i >= n) i = 2 * n - 1 - i;
+    }
+    return i;
+}
 
 // Exclusive scan of one int per thread across a block of blockDim.x
 // threads (multiple of 32, <= 1024).  sh must hold 33 ints.  Returns the

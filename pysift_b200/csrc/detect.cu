@@ -685,16 +685,6 @@ struct BlurArgs {
     unsigned long long w2[2 * BLUR_PAIR_MAX_R + 1];  // (w[k], w[k]) packed, radii up to BLUR_PAIR_MAX_R
 };
 
-// Half-sample-symmetric reflection into [0, n) (period 2n), as the
-// reference's reflect() (pysift/core.py:477-483), without integer division.
-__device__ __forceinline__ int reflect_idx(int i, int n) {
-    while (i < 0 || i >= n) {
-        if (i < 0) i = -i - 1;
-        if (i >= n) i = 2 * n - 1 - i;
-    }
-    return i;
-}
-
 constexpr int BLUR_TW = 64, BLUR_TH = 32, BLUR_NT = 256;
 
 // Loads input rows [r0-R, r0+TH+R) and columns [c0-RA, c0+TW+RA) (RA >= R,
@@ -1236,6 +1226,21 @@ static int launch_blur(BlurArgs& a, int R, const float* w, cudaStream_t st) {
         PYSIFT_LAUNCH_CHECK("k_blur_generic");
     }
     return PYSIFT_OK;
+}
+
+int blur_level(const float* in, long long in_pitch, int step, float* out, int out_pitch, float* copy0, int H, int W,
+               const float* w, int R, cudaStream_t st) {
+    static thread_local BlurArgs a;  // large (weights by value); not on the stack
+    memset(&a, 0, sizeof(a));
+    a.in = in;
+    a.in_pitch = in_pitch;
+    a.step = step;
+    a.out = out;
+    a.out_pitch = out_pitch;
+    a.copy0 = copy0;
+    a.H = H;
+    a.W = W;
+    return launch_blur(a, R, w, st);
 }
 
 // ---------------------------------------------------------------------------
@@ -2912,16 +2917,8 @@ int pysift_gauss_blur(const float* in, int32_t in_pitch, float* out, int32_t out
     PYSIFT_CHECK_ARG(H > 0 && W > 0 && in_pitch >= W && out_pitch >= W, "bad sizes");
     PYSIFT_CHECK_ARG(radius >= 0 && radius <= PYSIFT_MAX_RADIUS, "radius %d outside 0..%d", radius,
                      PYSIFT_MAX_RADIUS);
-    static thread_local BlurArgs a;
-    memset(&a, 0, sizeof(a));
-    a.in = in;
-    a.in_pitch = in_pitch;
-    a.step = 1;
-    a.out = out;
-    a.out_pitch = out_pitch;
-    a.H = H;
-    a.W = W;
-    return launch_blur(a, radius, weights, reinterpret_cast<cudaStream_t>(stream));
+    return blur_level(in, in_pitch, 1, out, out_pitch, nullptr, H, W, weights, radius,
+                      reinterpret_cast<cudaStream_t>(stream));
 }
 
 int pysift_set_blur_tile_rows(int32_t rows) {

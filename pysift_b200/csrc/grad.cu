@@ -11,7 +11,11 @@
 // histogram, then per sample through mag = |(dx, dy)|, the orientation
 // theta = atan2(dy, dx) (which moves the orientation interpolation weights)
 // into the central differences dx = G[r][c+1] - G[r][c-1],
-// dy = G[r+1][c] - G[r-1][c] (float atomics into the level's gradient).
+// dy = G[r+1][c] - G[r-1][c] (float atomics into a map of (d/ddx, d/ddy) per
+// pixel of the level; the pass that reads the map forms the differences'
+// adjoint).  pysift_desc_levels_* run the whole function over the keypoints
+// of all levels: the pyramid, one descriptor launch, and backward one adjoint
+// launch a level.
 //
 // Blur adjoint: the transpose of the separable blur with half-sample
 // symmetric reflection (pysift/core.py:477-483): a reflected tap folds back
@@ -27,7 +31,9 @@
 // homography terms are computed in float64 (the images and pixel values stay
 // float32): the per-pixel terms of the homography gradient cancel over the
 // canvas.
+#include <algorithm>
 #include <cstdint>
+#include <cstring>
 
 #include "common.cuh"
 
@@ -104,65 +110,149 @@ __device__ __forceinline__ float block_sum_f(float v, float* sh) {
     return t;
 }
 
-// kp: (n, 3) float rows [r0, c0, angle_deg]; hist (n, 128) raw, desc (n, 128)
-__global__ void __launch_bounds__(GD_T) k_desc_f32_fwd(const float* __restrict__ G, int H, int W, long long P,
-                                                       const float* __restrict__ kp, int n, int ph,
-                                                       float* __restrict__ hist, float* __restrict__ desc) {
-    __shared__ float h[128];
-    __shared__ float sh[33];
-    const float scale_sp = 4.0f / (2.0f * (float)ph);
+// The levels keypoints can sit on: entry octave * PYSIFT_MAX_LEVELS + scale
+// index (the single-level entry points use entry 0).
+struct DescLevel {
+    const float* G;  // null: no such level
+    float2* map;     // backward: (dL/ddx, dL/ddy) per pixel, pitch P, accumulated with atomics
+    int H, W, P, ph;
+};
+constexpr int GD_LEVELS = PYSIFT_MAX_OCTAVES * PYSIFT_MAX_LEVELS;
+struct DescTable {
+    DescLevel lv[GD_LEVELS];
+};
+
+// keypoint rows: [r0, c0, angle in degrees], or with `levels` [entry, r0, c0, angle]
+struct DescKp {
+    const DescLevel* lv;
+    int r0, c0;
+    float ang, sin_a, cos_a;
+    float scale_sp, inv_2s2;
+    int side;
+};
+
+__device__ __forceinline__ DescKp desc_kp(const DescTable& tab, const float* __restrict__ kp, int k, bool levels) {
+    DescKp d;
+    const float* row = kp + (long long)k * (levels ? 4 : 3);
+    int e = 0;
+    if (levels) {
+        e = (int)row[0];
+        ++row;
+    }
+    d.lv = e >= 0 && e < GD_LEVELS && tab.lv[e].G ? &tab.lv[e] : nullptr;
+    d.r0 = (int)row[0];
+    d.c0 = (int)row[1];
+    d.ang = row[2] * (GD_PI / 180.0f);
+    sincosf(d.ang, &d.sin_a, &d.cos_a);
+    const int ph = d.lv ? d.lv->ph : 1;
+    d.scale_sp = 4.0f / (2.0f * (float)ph);
     const float sigma_d = (float)ph * 0.5657f;
-    const float inv_2s2 = 1.0f / (2.0f * sigma_d * sigma_d + 1e-12f);
-    const int side = 2 * ph + 1;
+    d.inv_2s2 = 1.0f / (2.0f * sigma_d * sigma_d + 1e-12f);
+    d.side = 2 * ph + 1;
+    return d;
+}
+
+// hist (n, 128) raw, desc (n, 128).  A block per keypoint.  Every lane adds
+// its samples into a histogram of its own, 128 words at a stride of 32 (one
+// bank a lane): a plain load, add and store per corner without conflicts,
+// where a float atomic on shared memory is a compare-and-swap loop (1,068 us
+// for the 2,000 keypoints of a 1024x768 image in twelve launches, 115 us so
+// in one).  The corners that the clamp at the patch's rim maps to one cell
+// are merged first, so a sample's eight words differ and its eight loads can
+// be in flight together.
+constexpr int GF_T = 128;
+constexpr size_t GF_SMEM = (size_t)GF_T * 128 * sizeof(float);
+
+__global__ void __launch_bounds__(GF_T) k_desc_f32_fwd(const __grid_constant__ DescTable tab,
+                                                       const float* __restrict__ kp, int n, bool levels,
+                                                       float* __restrict__ hist, float* __restrict__ desc) {
+    extern __shared__ float lane_hist[];
+    __shared__ float sh[33];
+    const int tid = threadIdx.x;
+    float* const h = lane_hist + (tid >> 5) * (128 * 32) + (tid & 31);
     for (int k = blockIdx.x; k < n; k += gridDim.x) {
-        for (int b = threadIdx.x; b < 128; b += GD_T) h[b] = 0.0f;
-        __syncthreads();
-        const int r0 = (int)kp[3 * k], c0 = (int)kp[3 * k + 1];
-        const float ang = kp[3 * k + 2] * (GD_PI / 180.0f);
-        float sin_a, cos_a;
-        sincosf(ang, &sin_a, &cos_a);
-        for (int idx = threadIdx.x; idx < side * side; idx += GD_T) {
-            const DescSample s = desc_sample(idx, side, ph, r0, c0, H, W, cos_a, sin_a, scale_sp);
-            if (!s.act) continue;
-            const float* gp = G + (long long)s.rr * P + s.cc;
-            const float dx = gp[1] - gp[-1], dy = gp[P] - gp[-P];
-            const float mag = sqrtf(dx * dx + dy * dy);
-            float ori = (atan2f(dy, dx) - ang) * (180.0f / GD_PI) + 360.0f;
-            ori = ori >= 360.0f ? ori - 360.0f : ori;
-            const float gw = expf(-(s.xr * s.xr + s.yr * s.yr) * inv_2s2);
-            const Corners c = desc_corners(s.xb, s.yb, ori);
-            const float wm = mag * gw;
+#pragma unroll 16
+        for (int b = 0; b < 128; ++b) h[b * 32] = 0.0f;
+        const DescKp d = desc_kp(tab, kp, k, levels);
+        if (d.lv) {
+            const float* __restrict__ G = d.lv->G;
+            const int H = d.lv->H, W = d.lv->W, ph = d.lv->ph;
+            const long long P = d.lv->P;
+            for (int idx = tid; idx < d.side * d.side; idx += GF_T) {
+                const DescSample s = desc_sample(idx, d.side, ph, d.r0, d.c0, H, W, d.cos_a, d.sin_a, d.scale_sp);
+                if (!s.act) continue;
+                const float* gp = G + (long long)s.rr * P + s.cc;
+                const float dx = gp[1] - gp[-1], dy = gp[P] - gp[-P];
+                const float mag = sqrtf(dx * dx + dy * dy);
+                float ori = (atan2f(dy, dx) - d.ang) * (180.0f / GD_PI) + 360.0f;
+                ori = ori >= 360.0f ? ori - 360.0f : ori;
+                const float gw = expf(-(s.xr * s.xr + s.yr * s.yr) * d.inv_2s2);
+                const float wm = mag * gw;
+                const float ob = ori * (8.0f / 360.0f);
+                const int oi0 = (int)floorf(ob);
+                const float df = ob - (float)oi0;
+                const int xi = (int)floorf(s.xb), yi = (int)floorf(s.yb);
+                float wx1 = s.xb - (float)xi, wy1 = s.yb - (float)yi;
+                float wx0 = 1.0f - wx1, wy0 = 1.0f - wy1;
+                // xi, yi are in -1 .. 3: at either end both corners clamp to one
+                // cell, which takes the whole weight; its neighbour gets nothing
+                const bool mx = xi < 0 || xi > 2, my = yi < 0 || yi > 2;
+                if (mx) wx0 = 1.0f;
+                if (my) wy0 = 1.0f;
+                const int xa = max(xi, 0), ya = max(yi, 0);
+                const int xc = xi < 0 ? 1 : (xi > 2 ? 2 : xi + 1), yc = yi < 0 ? 1 : (yi > 2 ? 2 : yi + 1);
+                const int o0 = oi0 & 7, o1 = (oi0 + 1) & 7;
+                const float w[4] = {wy0 * wx0, wy0 * wx1, wy1 * wx0, wy1 * wx1};
+                float* const c[4] = {h + (ya * 32 + xa * 8) * 32, h + (ya * 32 + xc * 8) * 32,
+                                     h + (yc * 32 + xa * 8) * 32, h + (yc * 32 + xc * 8) * 32};
+                float v0[4], v1[4];
 #pragma unroll
-            for (int q = 0; q < 4; ++q) {
-                atomicAdd(&h[c.bin[2 * q]], c.wsp[q] * (1.0f - c.df) * wm);
-                atomicAdd(&h[c.bin[2 * q + 1]], c.wsp[q] * c.df * wm);
+                for (int q = 0; q < 4; ++q) {
+                    v0[q] = c[q][o0 * 32];
+                    v1[q] = c[q][o1 * 32];
+                }
+#pragma unroll
+                for (int q = 0; q < 4; ++q) {
+                    if (((q & 1) && mx) || ((q & 2) && my)) continue;
+                    v0[q] += w[q] * (1.0f - df) * wm;
+                    v1[q] += w[q] * df * wm;
+                }
+#pragma unroll
+                for (int q = 0; q < 4; ++q) {
+                    c[q][o0 * 32] = v0[q];
+                    c[q][o1 * 32] = v1[q];
+                }
             }
         }
         __syncthreads();
-        const float v = threadIdx.x < 128 ? h[threadIdx.x] : 0.0f;
+        // thread b sums bin b over the lanes, starting at its own bank
+        float v = 0.0f;
+        for (int w = 0; w < GF_T / 32; ++w) {
+            const float* src = lane_hist + w * (128 * 32) + tid * 32;
+            float part[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+#pragma unroll
+            for (int j = 0; j < 32; ++j) part[j & 3] += src[(j + tid) & 31];
+            v += (part[0] + part[1]) + (part[2] + part[3]);
+        }
         const float n1 = sqrtf(block_sum_f(v * v, sh) + 1e-14f);
         float t = v / n1;
         t = t > 0.2f ? 0.2f : t;
-        const float n2 = sqrtf(block_sum_f(threadIdx.x < 128 ? t * t : 0.0f, sh) + 1e-14f);
-        if (threadIdx.x < 128) {
-            hist[(long long)k * 128 + threadIdx.x] = v;
-            desc[(long long)k * 128 + threadIdx.x] = t / n2;
-        }
-        __syncthreads();
+        const float n2 = sqrtf(block_sum_f(t * t, sh) + 1e-14f);
+        hist[(long long)k * 128 + tid] = v;
+        desc[(long long)k * 128 + tid] = t / n2;
     }
 }
 
-// gdesc: dL/ddesc (n, 128); gG: dL/dG accumulated with atomics (pitch P)
-__global__ void __launch_bounds__(GD_T) k_desc_f32_bwd(const float* __restrict__ G, int H, int W, long long P,
-                                                       const float* __restrict__ kp, int n, int ph,
+// gdesc: dL/ddesc (n, 128).  Into the level's map one vector atomic a sample
+// (four scalar ones on the level's gradient, one a neighbour, were 210 us for
+// 2,000 keypoints at 1024x768, this 99), or with gG != null (the single-level
+// entry point) straight into the level's gradient.
+__global__ void __launch_bounds__(GD_T) k_desc_f32_bwd(const __grid_constant__ DescTable tab,
+                                                       const float* __restrict__ kp, int n, bool levels,
                                                        const float* __restrict__ hist,
                                                        const float* __restrict__ gdesc, float* __restrict__ gG) {
     __shared__ float hb[128];  // dL/dhist
     __shared__ float sh[33];
-    const float scale_sp = 4.0f / (2.0f * (float)ph);
-    const float sigma_d = (float)ph * 0.5657f;
-    const float inv_2s2 = 1.0f / (2.0f * sigma_d * sigma_d + 1e-12f);
-    const int side = 2 * ph + 1;
     for (int k = blockIdx.x; k < n; k += gridDim.x) {
         // backward of L2 -> clip 0.2 -> L2
         const bool own = threadIdx.x < 128;
@@ -179,21 +269,21 @@ __global__ void __launch_bounds__(GD_T) k_desc_f32_bwd(const float* __restrict__
         const float gh = gt / n1 - v * gt_dot / (n1 * n1 * n1);
         if (own) hb[threadIdx.x] = gh;
         __syncthreads();
-        const int r0 = (int)kp[3 * k], c0 = (int)kp[3 * k + 1];
-        const float ang = kp[3 * k + 2] * (GD_PI / 180.0f);
-        float sin_a, cos_a;
-        sincosf(ang, &sin_a, &cos_a);
-        for (int idx = threadIdx.x; idx < side * side; idx += GD_T) {
-            const DescSample s = desc_sample(idx, side, ph, r0, c0, H, W, cos_a, sin_a, scale_sp);
+        const DescKp d = desc_kp(tab, kp, k, levels);
+        const int H = d.lv ? d.lv->H : 0, W = d.lv ? d.lv->W : 0, ph = d.lv ? d.lv->ph : 0;
+        const long long P = d.lv ? d.lv->P : 0;
+        const int ns = d.lv ? d.side * d.side : 0;
+        for (int idx = threadIdx.x; idx < ns; idx += GD_T) {
+            const DescSample s = desc_sample(idx, d.side, ph, d.r0, d.c0, H, W, d.cos_a, d.sin_a, d.scale_sp);
             if (!s.act) continue;
-            const float* gp = G + (long long)s.rr * P + s.cc;
+            const float* gp = d.lv->G + (long long)s.rr * P + s.cc;
             const float dx = gp[1] - gp[-1], dy = gp[P] - gp[-P];
             const float m2 = dx * dx + dy * dy;
             if (!(m2 > 0.0f)) continue;
             const float mag = sqrtf(m2);
-            float ori = (atan2f(dy, dx) - ang) * (180.0f / GD_PI) + 360.0f;
+            float ori = (atan2f(dy, dx) - d.ang) * (180.0f / GD_PI) + 360.0f;
             ori = ori >= 360.0f ? ori - 360.0f : ori;
-            const float gw = expf(-(s.xr * s.xr + s.yr * s.yr) * inv_2s2);
+            const float gw = expf(-(s.xr * s.xr + s.yr * s.yr) * d.inv_2s2);
             const Corners cr = desc_corners(s.xb, s.yb, ori);
             float gmag = 0.0f, gdf = 0.0f;
 #pragma unroll
@@ -207,41 +297,317 @@ __global__ void __launch_bounds__(GD_T) k_desc_f32_bwd(const float* __restrict__
             const float gth = gdf * gw * mag * (4.0f / GD_PI);
             const float gdx = gmag * dx / mag - gth * dy / m2;
             const float gdy = gmag * dy / mag + gth * dx / m2;
-            float* g = gG + (long long)s.rr * P + s.cc;
-            atomicAdd(g + 1, gdx);
-            atomicAdd(g - 1, -gdx);
-            atomicAdd(g + P, gdy);
-            atomicAdd(g - P, -gdy);
+            const long long at = (long long)s.rr * P + s.cc;
+            if (gG) {
+                atomicAdd(gG + at + 1, gdx);
+                atomicAdd(gG + at - 1, -gdx);
+                atomicAdd(gG + at + P, gdy);
+                atomicAdd(gG + at - P, -gdy);
+            } else {
+                atomicAdd(d.lv->map + at, make_float2(gdx, gdy));
+            }
         }
         __syncthreads();
     }
 }
 
+// What is added to a blur adjoint: the adjoint of the central differences of
+// a level's map, and at even rows and columns the gradient of the octave that
+// the level was subsampled into.
+struct AdjTail {
+    const float2* map;
+    int map_pitch;
+    const float* sub;
+    int sub_pitch;
+    __device__ __forceinline__ float at(int y, int x, int H, int W) const {
+        float v = 0.0f;
+        if (map) {
+            const float2* m = map + (long long)y * map_pitch + x;
+            if (x > 0) v += m[-1].x;
+            if (x + 1 < W) v -= m[1].x;
+            if (y > 0) v += m[-(long long)map_pitch].y;
+            if (y + 1 < H) v -= m[map_pitch].y;
+        }
+        if (sub && !((y | x) & 1)) v += sub[(long long)(y >> 1) * sub_pitch + (x >> 1)];
+        return v;
+    }
+};
+
+struct AdjArgs {
+    const float* in;
+    long long in_pitch;
+    float* out;
+    long long out_pitch;
+    int H, W;
+    float w[PYSIFT_MAX_TAPS];
+    const float* wdev;  // device weights in place of w (k_blur_adjoint_axis)
+    bool accumulate;    // out += (k_blur_adjoint_axis)
+    AdjTail tail;
+};
+
 // One axis of the adjoint of y[i] = sum_k w[k] x[refl(i + k - R)] (half-sample
 // symmetric reflection, R < n): x_bar[j] = sum_k w[k] sum over the reads of
-// pixel j.  axis 0: along rows (x), axis 1: along columns (y).  out = in^T-applied.
-__global__ void k_blur_adjoint_axis(const float* __restrict__ in, long long in_pitch, float* __restrict__ out,
-                                    long long out_pitch, int H, int W, const float* __restrict__ w, int R, int axis,
-                                    int accumulate) {
+// pixel j.  axis 0: along rows (x), with the tail; axis 1: along columns (y).
+// For any taps and radius, and in place.
+__global__ void k_blur_adjoint_axis(const __grid_constant__ AdjArgs a, int R, int axis) {
     const int x = blockIdx.x * blockDim.x + threadIdx.x, y = blockIdx.y;
-    if (x >= W || y >= H) return;
-    const int n = axis == 0 ? W : H, j = axis == 0 ? x : y;
+    if (x >= a.W || y >= a.H) return;
+    const int n = axis == 0 ? a.W : a.H, j = axis == 0 ? x : y;
     float acc = 0.0f;
     for (int k = 0; k <= 2 * R; ++k) {
-        const float wk = w[k];
+        const float wk = a.wdev ? a.wdev[k] : a.w[k];
         const int cand[3] = {j - k + R, -1 - j - k + R, 2 * n - 1 - j - k + R};
 #pragma unroll
         for (int q = 0; q < 3; ++q) {
             const int i = cand[q];
             if (i < 0 || i >= n) continue;
-            if (q == 1 && -1 - j == j) continue;            // never (j >= 0)
-            if (q == 2 && 2 * n - 1 - j == j) continue;     // never (j <= n - 1)
-            const float v = axis == 0 ? in[(long long)y * in_pitch + i] : in[(long long)i * in_pitch + x];
-            acc += wk * v;
+            acc += wk * (axis == 0 ? a.in[(long long)y * a.in_pitch + i] : a.in[(long long)i * a.in_pitch + x]);
         }
     }
-    float* o = out + (long long)y * out_pitch + x;
-    *o = accumulate ? *o + acc : acc;
+    float* o = a.out + (long long)y * a.out_pitch + x;
+    if (axis == 0) acc += a.tail.at(y, x, a.H, a.W);
+    *o = axis == 0 && a.accumulate ? *o + acc : acc;
+}
+
+// Both axes of the adjoint of one 64 x 32 tile, for symmetric taps: then
+// B[i][j] = w(j - i) + w(-1 - j - i) + w(2 n - 1 - j - i) is its own transpose
+// (w(t) the tap at offset t), so the adjoint is the reflecting blur itself.
+// Columns first, into a strip of 64 + 2 R columns, then rows; both passes
+// slide a register window over 8 outputs.  One tile pass with the differences
+// and the subsampling in its tail replaces two passes over global memory and
+// their three candidate reads a tap: 286 us for the 16 levels of a
+// 1024x768 image, now 103 with the tails.
+constexpr int ADJ_TW = 64, ADJ_TH = 32, ADJ_T = 256;
+template <int R>
+struct AdjTile {
+    static constexpr int ROWS = ADJ_TH + 2 * R, COLS = ADJ_TW + 2 * R, TS = COLS | 1;
+    static constexpr size_t bytes = (size_t)(ROWS + ADJ_TH) * TS * sizeof(float);
+};
+static_assert(AdjTile<16>::bytes <= 48 * 1024, "the tiles stay within the default dynamic shared memory");
+
+template <int R>
+__global__ void __launch_bounds__(ADJ_T) k_blur_adjoint(const __grid_constant__ AdjArgs a) {
+    using T = AdjTile<R>;
+    extern __shared__ float adj_smem[];
+    float* const tile = adj_smem;             // input rows [r0 - R, r0 + TH + R), columns [c0 - R, c0 + TW + R)
+    float* const mid = adj_smem + T::ROWS * T::TS;
+    const int c0 = blockIdx.x * ADJ_TW, r0 = blockIdx.y * ADJ_TH;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    constexpr int CQ = (T::COLS + 31) / 32;
+    int gc[CQ];
+#pragma unroll
+    for (int q = 0; q < CQ; ++q) gc[q] = reflect_idx(c0 - R + lane + 32 * q, a.W);
+    for (int rr = warp; rr < T::ROWS; rr += ADJ_T / 32) {
+        const float* src = a.in + (long long)reflect_idx(r0 - R + rr, a.H) * a.in_pitch;
+#pragma unroll
+        for (int q = 0; q < CQ; ++q)
+            if (lane + 32 * q < T::COLS) tile[rr * T::TS + lane + 32 * q] = src[gc[q]];
+    }
+    __syncthreads();
+    for (int i = tid; i < T::COLS * (ADJ_TH / 8); i += ADJ_T) {
+        const int cc = i % T::COLS, j0 = (i / T::COLS) * 8;
+        float v[8 + 2 * R];
+#pragma unroll
+        for (int m = 0; m < 8 + 2 * R; ++m) v[m] = tile[(j0 + m) * T::TS + cc];
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+            float acc = 0.0f;
+#pragma unroll
+            for (int k = 0; k <= 2 * R; ++k) acc = fmaf(a.w[k], v[j + k], acc);
+            mid[(j0 + j) * T::TS + cc] = acc;
+        }
+    }
+    __syncthreads();
+    {
+        float v[8 + 2 * R];
+#pragma unroll
+        for (int m = 0; m < 8 + 2 * R; ++m) v[m] = mid[lane * T::TS + warp * 8 + m];
+        // the tile is free: the outputs go through it, so that a warp stores whole rows
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+            float acc = 0.0f;
+#pragma unroll
+            for (int k = 0; k <= 2 * R; ++k) acc = fmaf(a.w[k], v[j + k], acc);
+            tile[lane * T::TS + warp * 8 + j] = acc;
+        }
+    }
+    __syncthreads();
+    for (int i = tid; i < ADJ_TH * ADJ_TW; i += ADJ_T) {
+        const int y = r0 + i / ADJ_TW, x = c0 + i % ADJ_TW;
+        if (y < a.H && x < a.W)
+            a.out[(long long)y * a.out_pitch + x] = tile[(i / ADJ_TW) * T::TS + i % ADJ_TW] + a.tail.at(y, x, a.H, a.W);
+    }
+}
+
+// the tail alone (the top level of an octave)
+__global__ void __launch_bounds__(256) k_adjoint_tail(float* __restrict__ out, int out_pitch, int H, int W,
+                                                      const AdjTail tail) {
+    const int x = blockIdx.x * blockDim.x + threadIdx.x, y = blockIdx.y;
+    if (x < W) out[(long long)y * out_pitch + x] = tail.at(y, x, H, W);
+}
+
+template <int R>
+static void adj_launch(const AdjArgs& a, cudaStream_t st) {
+    k_blur_adjoint<R><<<dim3(ceil_div(a.W, ADJ_TW), ceil_div(a.H, ADJ_TH)), ADJ_T, AdjTile<R>::bytes, st>>>(a);
+}
+
+constexpr int ADJ_MAX_R = 16;  // radii of the tiled kernel
+
+// tmp: as large as the input, for the two-pass form
+static int launch_adjoint_axes(const AdjArgs& a, int R, float* tmp, int tmp_pitch, cudaStream_t st) {
+    const dim3 grid(ceil_div(a.W, 128), a.H);
+    // forward = horizontal then vertical; adjoint = vertical^T then horizontal^T
+    AdjArgs b = a;
+    b.out = tmp;
+    b.out_pitch = tmp_pitch;
+    k_blur_adjoint_axis<<<grid, 128, 0, st>>>(b, R, 1);
+    PYSIFT_LAUNCH_CHECK("k_blur_adjoint_axis");
+    b = a;
+    b.in = tmp;
+    b.in_pitch = tmp_pitch;
+    k_blur_adjoint_axis<<<grid, 128, 0, st>>>(b, R, 0);
+    PYSIFT_LAUNCH_CHECK("k_blur_adjoint_axis");
+    return PYSIFT_OK;
+}
+
+// The tiled kernel for the taps it is right and compiled for (the Gaussian
+// tables are symmetric bit for bit), the two-pass form for the others.
+static int launch_adjoint(const AdjArgs& a, int R, float* tmp, int tmp_pitch, cudaStream_t st) {
+    bool tiled = R <= ADJ_MAX_R;
+    for (int k = 0; k < R; ++k) tiled = tiled && a.w[k] == a.w[2 * R - k];
+    if (!tiled) return launch_adjoint_axes(a, R, tmp, tmp_pitch, st);
+    switch (R) {
+        case 0: adj_launch<0>(a, st); break;
+        case 1: adj_launch<1>(a, st); break;
+        case 2: adj_launch<2>(a, st); break;
+        case 3: adj_launch<3>(a, st); break;
+        case 4: adj_launch<4>(a, st); break;
+        case 5: adj_launch<5>(a, st); break;
+        case 6: adj_launch<6>(a, st); break;
+        case 7: adj_launch<7>(a, st); break;
+        case 8: adj_launch<8>(a, st); break;
+        case 9: adj_launch<9>(a, st); break;
+        case 10: adj_launch<10>(a, st); break;
+        case 11: adj_launch<11>(a, st); break;
+        case 12: adj_launch<12>(a, st); break;
+        case 13: adj_launch<13>(a, st); break;
+        case 14: adj_launch<14>(a, st); break;
+        case 15: adj_launch<15>(a, st); break;
+        default: adj_launch<16>(a, st); break;
+    }
+    PYSIFT_LAUNCH_CHECK("k_blur_adjoint");
+    return PYSIFT_OK;
+}
+
+static int launch_desc_fwd(const DescTable& tab, const float* kp, int n, bool levels, float* hist, float* desc,
+                           cudaStream_t st) {
+    PYSIFT_CUDA_TRY(cudaFuncSetAttribute(k_desc_f32_fwd, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)GF_SMEM));
+    // three resident blocks an SM; more blocks than that keep the tail short
+    k_desc_f32_fwd<<<std::min(n, 148 * 12), GF_T, GF_SMEM, st>>>(tab, kp, n, levels, hist, desc);
+    PYSIFT_LAUNCH_CHECK("k_desc_f32_fwd");
+    return PYSIFT_OK;
+}
+
+static int launch_desc_bwd(const DescTable& tab, const float* kp, int n, bool levels, const float* hist,
+                           const float* gdesc, float* gG, cudaStream_t st) {
+    k_desc_f32_bwd<<<std::min(n, 148 * 8), GD_T, 0, st>>>(tab, kp, n, levels, hist, gdesc, gG);
+    PYSIFT_LAUNCH_CHECK("k_desc_f32_bwd");
+    return PYSIFT_OK;
+}
+
+// Workspace of pysift_desc_levels_*: the Gaussian levels 0 .. top of every
+// octave in use, and backward a map per level from 0 .. top, each octave's
+// level-0 gradient and three buffers for the chain of adjoints.
+struct LevelsLayout {
+    int n_oct, top;
+    int H[PYSIFT_MAX_OCTAVES], W[PYSIFT_MAX_OCTAVES], P[PYSIFT_MAX_OCTAVES];
+    size_t off_lev[PYSIFT_MAX_OCTAVES], off_map[PYSIFT_MAX_OCTAVES], off_g0[PYSIFT_MAX_OCTAVES], off_chain[3];
+    size_t map_begin, map_end, total;
+    size_t plane(int o) const { return (size_t)H[o] * P[o]; }
+};
+
+static int levels_layout(const pysift_detect_config* cfg, int H, int W, int n_oct, int top, bool backward,
+                         LevelsLayout& l) {
+    PYSIFT_CHECK_ARG(cfg, "config is NULL");
+    PYSIFT_CHECK_ARG(H > 2 && W > 2, "image size %dx%d too small", H, W);
+    PYSIFT_CHECK_ARG(n_oct >= 1 && n_oct <= PYSIFT_MAX_OCTAVES, "n_octaves %d outside 1..%d", n_oct,
+                     PYSIFT_MAX_OCTAVES);
+    PYSIFT_CHECK_ARG(cfg->n_scales >= 1 && cfg->n_scales + 3 <= PYSIFT_MAX_LEVELS, "n_scales out of range");
+    PYSIFT_CHECK_ARG(top >= cfg->n_scales && top <= cfg->n_scales + 2, "top level %d outside %d..%d", top,
+                     cfg->n_scales, cfg->n_scales + 2);
+    for (int i = 1; i < 2 + top; ++i)
+        PYSIFT_CHECK_ARG(cfg->blur_radius[i] >= 0 && cfg->blur_radius[i] <= PYSIFT_MAX_RADIUS,
+                         "blur radius %d outside 0..%d", cfg->blur_radius[i], PYSIFT_MAX_RADIUS);
+    size_t off = 0;
+    auto take = [&](size_t bytes) {
+        const size_t r = off;
+        off = align_up(off + bytes, 256);
+        return r;
+    };
+    l.n_oct = n_oct;
+    l.top = top;
+    for (int o = 0; o < n_oct; ++o) {
+        l.H[o] = o ? (l.H[o - 1] + 1) / 2 : H;
+        l.W[o] = o ? (l.W[o - 1] + 1) / 2 : W;
+        PYSIFT_CHECK_ARG(l.H[o] > 2 && l.W[o] > 2, "octave %d of a %dx%d image is too small", o, H, W);
+        l.P[o] = (int)align_up((size_t)l.W[o], 32);
+    }
+    for (int o = 0; o < n_oct; ++o) l.off_lev[o] = take((size_t)(top + 1) * l.plane(o) * sizeof(float));
+    l.map_begin = off;
+    if (backward) {
+        for (int o = 0; o < n_oct; ++o) l.off_map[o] = take((size_t)(top + 1) * l.plane(o) * sizeof(float2));
+        l.map_end = off;
+        for (int o = 0; o < n_oct; ++o) l.off_g0[o] = take(l.plane(o) * sizeof(float));
+        for (size_t& c : l.off_chain) c = take(l.plane(0) * sizeof(float));
+    }
+    l.total = off;
+    return PYSIFT_OK;
+}
+
+static float* lev_at(void* ws, const LevelsLayout& l, int o, int s) {
+    return reinterpret_cast<float*>(static_cast<char*>(ws) + l.off_lev[o]) + (size_t)s * l.plane(o);
+}
+static float2* map_at(void* ws, const LevelsLayout& l, int o, int s) {
+    return reinterpret_cast<float2*>(static_cast<char*>(ws) + l.off_map[o]) + (size_t)s * l.plane(o);
+}
+
+// Gaussian levels of the non-doubled image (pysift/core.py:1288-1343)
+static int build_levels(const pysift_detect_config* cfg, const float* img, int pitch, void* ws, const LevelsLayout& l,
+                        cudaStream_t st) {
+    for (int o = 0; o < l.n_oct; ++o) {
+        const int H = l.H[o], W = l.W[o], P = l.P[o];
+        if (o == 0) {
+            const int rc = blur_level(img, pitch, 1, lev_at(ws, l, 0, 0), P, nullptr, H, W, cfg->blur_weights[1],
+                                      cfg->blur_radius[1], st);
+            if (rc) return rc;
+        }
+        for (int s = 0; s < l.top; ++s) {
+            const bool first = o > 0 && s == 0;  // reads level S of the octave before at every second pixel
+            const float* in = first ? lev_at(ws, l, o - 1, cfg->n_scales) : lev_at(ws, l, o, s);
+            const int rc = blur_level(in, first ? l.P[o - 1] : P, first ? 2 : 1, lev_at(ws, l, o, s + 1), P,
+                                      first ? lev_at(ws, l, o, 0) : nullptr, H, W, cfg->blur_weights[2 + s],
+                                      cfg->blur_radius[2 + s], st);
+            if (rc) return rc;
+        }
+    }
+    return PYSIFT_OK;
+}
+
+static void levels_table(const pysift_detect_config* cfg, void* ws, const LevelsLayout& l, bool backward,
+                         DescTable& tab) {
+    memset(&tab, 0, sizeof(tab));
+    for (int o = 0; o < l.n_oct; ++o)
+        for (int s = 0; s <= l.top; ++s) {
+            const int ph = (int)cfg->desc_ph[s];
+            if (ph < 1 || ph > 200) continue;
+            DescLevel& v = tab.lv[o * PYSIFT_MAX_LEVELS + s];
+            v.G = lev_at(ws, l, o, s);
+            v.map = backward ? map_at(ws, l, o, s) : nullptr;
+            v.H = l.H[o];
+            v.W = l.W[o];
+            v.P = l.P[o];
+            v.ph = ph;
+        }
 }
 
 struct WarpF32Args {
@@ -397,15 +763,19 @@ using namespace pysift;
 
 extern "C" {
 
+static void one_level(const float* level, int H, int W, int pitch, int ph, DescTable& tab) {
+    memset(&tab, 0, sizeof(tab));
+    tab.lv[0] = DescLevel{level, nullptr, H, W, pitch, ph};
+}
+
 int pysift_desc_f32_forward(const float* level, int32_t H, int32_t W, int32_t pitch, const float* kp, int32_t n,
                             int32_t ph, float* hist, float* desc, pysift_stream_t stream) {
     PYSIFT_CHECK_ARG(level && kp && hist && desc && H > 2 && W > 2 && pitch >= W && n >= 0 && ph >= 1 && ph <= 200,
                      "bad arguments");
     if (n == 0) return PYSIFT_OK;
-    k_desc_f32_fwd<<<std::min(n, 148 * 8), GD_T, 0, reinterpret_cast<cudaStream_t>(stream)>>>(level, H, W, pitch, kp,
-                                                                                             n, ph, hist, desc);
-    PYSIFT_LAUNCH_CHECK("k_desc_f32_fwd");
-    return PYSIFT_OK;
+    DescTable tab;
+    one_level(level, H, W, pitch, ph, tab);
+    return launch_desc_fwd(tab, kp, n, false, hist, desc, reinterpret_cast<cudaStream_t>(stream));
 }
 
 int pysift_desc_f32_backward(const float* level, int32_t H, int32_t W, int32_t pitch, const float* kp, int32_t n,
@@ -415,10 +785,9 @@ int pysift_desc_f32_backward(const float* level, int32_t H, int32_t W, int32_t p
                          ph <= 200,
                      "bad arguments");
     if (n == 0) return PYSIFT_OK;
-    k_desc_f32_bwd<<<std::min(n, 148 * 8), GD_T, 0, reinterpret_cast<cudaStream_t>(stream)>>>(
-        level, H, W, pitch, kp, n, ph, hist, gdesc, glevel);
-    PYSIFT_LAUNCH_CHECK("k_desc_f32_bwd");
-    return PYSIFT_OK;
+    DescTable tab;
+    one_level(level, H, W, pitch, ph, tab);
+    return launch_desc_bwd(tab, kp, n, false, hist, gdesc, glevel, reinterpret_cast<cudaStream_t>(stream));
 }
 
 int pysift_blur_adjoint(const float* gout, int32_t gout_pitch, float* gin, int32_t gin_pitch, float* tmp,
@@ -427,13 +796,115 @@ int pysift_blur_adjoint(const float* gout, int32_t gout_pitch, float* gin, int32
     PYSIFT_CHECK_ARG(gout && gin && tmp && weights_dev && H > 0 && W > 0, "bad arguments");
     PYSIFT_CHECK_ARG(radius >= 0 && radius < H && radius < W && radius <= PYSIFT_MAX_RADIUS,
                      "radius %d must be below both image sides", radius);
+    AdjArgs a = {};
+    a.in = gout;
+    a.in_pitch = gout_pitch;
+    a.out = gin;
+    a.out_pitch = gin_pitch;
+    a.H = H;
+    a.W = W;
+    a.wdev = weights_dev;
+    a.accumulate = accumulate != 0;
+    return launch_adjoint_axes(a, radius, tmp, tmp_pitch, reinterpret_cast<cudaStream_t>(stream));
+}
+
+int pysift_desc_levels_workspace_size(const pysift_detect_config* cfg, int32_t H, int32_t W, int32_t n_octaves,
+                                      int32_t top, int32_t backward, size_t* bytes) {
+    PYSIFT_CHECK_ARG(bytes != nullptr, "bytes is NULL");
+    LevelsLayout l = {};
+    const int rc = levels_layout(cfg, H, W, n_octaves, top, backward != 0, l);
+    if (rc) return rc;
+    *bytes = l.total;
+    return PYSIFT_OK;
+}
+
+int pysift_desc_levels_forward(const pysift_detect_config* cfg, const float* img, int32_t H, int32_t W, int32_t pitch,
+                               const float* kp, int32_t n, int32_t n_octaves, int32_t top, void* workspace,
+                               size_t workspace_bytes, float* hist, float* desc, pysift_stream_t stream) {
+    LevelsLayout l = {};
+    int rc = levels_layout(cfg, H, W, n_octaves, top, false, l);
+    if (rc) return rc;
+    PYSIFT_CHECK_ARG(img && workspace && pitch >= W && n >= 0 && (n == 0 || (kp && hist && desc)), "bad arguments");
+    PYSIFT_CHECK_ARG((reinterpret_cast<uintptr_t>(workspace) & 255) == 0, "workspace must be 256-byte aligned");
+    if (workspace_bytes < l.total) {
+        set_error("workspace %zu bytes < required %zu", workspace_bytes, l.total);
+        return PYSIFT_ERR_WORKSPACE;
+    }
+    if (n == 0) return PYSIFT_OK;
     cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
-    dim3 grid(ceil_div(W, 128), H);
-    // forward = horizontal then vertical; adjoint = vertical^T then horizontal^T
-    k_blur_adjoint_axis<<<grid, 128, 0, st>>>(gout, gout_pitch, tmp, tmp_pitch, H, W, weights_dev, radius, 1, 0);
-    PYSIFT_LAUNCH_CHECK("k_blur_adjoint_axis");
-    k_blur_adjoint_axis<<<grid, 128, 0, st>>>(tmp, tmp_pitch, gin, gin_pitch, H, W, weights_dev, radius, 0, accumulate);
-    PYSIFT_LAUNCH_CHECK("k_blur_adjoint_axis");
+    rc = build_levels(cfg, img, pitch, workspace, l, st);
+    if (rc) return rc;
+    DescTable tab;
+    levels_table(cfg, workspace, l, false, tab);
+    return launch_desc_fwd(tab, kp, n, true, hist, desc, st);
+}
+
+int pysift_desc_levels_backward(const pysift_detect_config* cfg, const float* img, int32_t H, int32_t W, int32_t pitch,
+                                const float* kp, int32_t n, int32_t n_octaves, int32_t top, void* workspace,
+                                size_t workspace_bytes, const float* hist, const float* gdesc, float* gimg,
+                                int32_t gimg_pitch, pysift_stream_t stream) {
+    LevelsLayout l = {};
+    int rc = levels_layout(cfg, H, W, n_octaves, top, true, l);
+    if (rc) return rc;
+    PYSIFT_CHECK_ARG(img && workspace && gimg && pitch >= W && gimg_pitch >= W && n >= 0 &&
+                         (n == 0 || (kp && hist && gdesc)),
+                     "bad arguments");
+    PYSIFT_CHECK_ARG((reinterpret_cast<uintptr_t>(workspace) & 255) == 0, "workspace must be 256-byte aligned");
+    for (int o = 0; o < n_octaves; ++o)
+        for (int s = o ? 0 : -1; s < top; ++s) {
+            const int R = cfg->blur_radius[2 + s];
+            PYSIFT_CHECK_ARG(R < l.H[o] && R < l.W[o], "radius %d must be below both image sides", R);
+        }
+    if (workspace_bytes < l.total) {
+        set_error("workspace %zu bytes < required %zu", workspace_bytes, l.total);
+        return PYSIFT_ERR_WORKSPACE;
+    }
+    cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
+    char* ws = static_cast<char*>(workspace);
+    rc = build_levels(cfg, img, pitch, ws, l, st);
+    if (rc) return rc;
+    PYSIFT_CUDA_TRY(cudaMemsetAsync(ws + l.map_begin, 0, l.map_end - l.map_begin, st));
+    if (n > 0) {
+        DescTable tab;
+        levels_table(cfg, ws, l, true, tab);
+        rc = launch_desc_bwd(tab, kp, n, true, hist, gdesc, nullptr, st);
+        if (rc) return rc;
+    }
+    // the adjoint of the level chain, highest octave first
+    for (int o = n_octaves - 1; o >= 0; --o) {
+        const int Ho = l.H[o], Wo = l.W[o], P = l.P[o];
+        auto tail = [&](int s) {
+            AdjTail t = {};
+            t.map = map_at(ws, l, o, s);
+            t.map_pitch = P;
+            if (s == cfg->n_scales && o + 1 < n_octaves) {
+                t.sub = reinterpret_cast<float*>(ws + l.off_g0[o + 1]);
+                t.sub_pitch = l.P[o + 1];
+            }
+            return t;
+        };
+        float* const chain[2] = {reinterpret_cast<float*>(ws + l.off_chain[0]),
+                                 reinterpret_cast<float*>(ws + l.off_chain[1])};
+        float* cur = chain[0];
+        k_adjoint_tail<<<dim3(ceil_div(Wo, 256), Ho), 256, 0, st>>>(cur, P, Ho, Wo, tail(top));
+        PYSIFT_LAUNCH_CHECK("k_adjoint_tail");
+        for (int s = top; s >= (o ? 1 : 0); --s) {
+            // level s -> level s - 1 (s = 0: the base blur, into the image's gradient)
+            AdjArgs a = {};
+            a.in = cur;
+            a.in_pitch = P;
+            a.out = s == 0 ? gimg : (s == 1 ? reinterpret_cast<float*>(ws + l.off_g0[o]) : chain[(top - s + 1) & 1]);
+            a.out_pitch = s == 0 ? gimg_pitch : P;
+            a.H = Ho;
+            a.W = Wo;
+            const int R = cfg->blur_radius[1 + s];
+            for (int k = 0; k <= 2 * R; ++k) a.w[k] = cfg->blur_weights[1 + s][k];
+            if (s > 0) a.tail = tail(s - 1);
+            rc = launch_adjoint(a, R, reinterpret_cast<float*>(ws + l.off_chain[2]), P, st);
+            if (rc) return rc;
+            cur = a.out;
+        }
+    }
     return PYSIFT_OK;
 }
 

@@ -1,7 +1,7 @@
 """Differentiable SIFT descriptors and warp + feather blend (autograd).
 
 Two torch.autograd.Functions with hand-written CUDA forward and backward
-kernels (csrc/grad.cu, C ABI pysift_desc_f32_* / pysift_blur_adjoint /
+kernels (csrc/grad.cu, C ABI pysift_desc_levels_* / pysift_blur_adjoint /
 pysift_warp_f32_*):
 
 * ``descriptors(img, keypoints, sift)``: float descriptors (L2 -> clip 0.2
@@ -67,21 +67,40 @@ def _blur_adjoint(g, w, r, accumulate_into=None):
     return out
 
 
-def _levels(x, n_oct, S, base, incs, top):
-    """Gaussian levels 0..top of every octave (list of lists of tensors)."""
-    levels = []
-    cur = _blur(x, *base) if base[1] > 0 else x.clone()
-    for o in range(n_oct):
-        lv = [cur]
-        for s in range(top):
-            w, r = incs[s]
-            lv.append(_blur(lv[-1], w, r) if r > 0 else lv[-1].clone())
-        levels.append(lv)
-        if o + 1 < n_oct:
-            cur = lv[S][::2, ::2].contiguous()
-            if min(cur.shape) < 8:
-                break
-    return levels
+def _levels_plan(kps, sift, shape):
+    """What the library needs to know of a keypoint table: its rows [octave *
+    MAX_LEVELS + scale index, row, column, angle] (float32, host), the octaves
+    and the top level in use, and the (rows, columns) of every octave the
+    image has (the pyramid ends before a side falls below 8)."""
+    n_oct, S = sift._cfg.n_octaves, sift._cfg.n_scales
+    sizes = [tuple(shape)]
+    while len(sizes) < n_oct:
+        nxt = tuple((d + 1) // 2 for d in sizes[-1])
+        if min(nxt) < 8:
+            break
+        sizes.append(nxt)
+    if kps.shape[0] == 0:
+        return torch.empty((0, 4)), 1, S, sizes
+    k = kps.detach().cpu().numpy()
+    o, si = k[:, 0].astype(np.int64), k[:, 1].astype(np.int64)
+    o = np.where(o < 0, o + len(sizes), o)
+    if o.min() < 0 or o.max() >= len(sizes) or si.min() < 0 or si.max() > S + 2:
+        raise IndexError("keypoint on an octave or level the pyramid does not have")
+    for s in np.unique(si).tolist():
+        if not 1 <= int(sift._cfg.desc_ph[s]) <= 200:
+            raise ValueError(f"patch half-width {sift._cfg.desc_ph[s]} of scale index {s} is outside 1..200")
+    rows = np.empty((k.shape[0], 4), np.float32)
+    rows[:, 0] = o * _lib.MAX_LEVELS + si
+    rows[:, 1:] = k[:, 2:5]
+    return torch.from_numpy(rows), int(o.max()) + 1, max(int(si.max()), S), sizes
+
+
+def _levels_workspace(lib, sift, shape, n_oct, top, backward, device):
+    size = ctypes.c_size_t()
+    _lib.check(lib.pysift_desc_levels_workspace_size(ctypes.byref(sift._cfg), shape[0], shape[1], n_oct, top, backward,
+                                                     ctypes.byref(size)), "pysift_desc_levels_workspace_size")
+    # torch's blocks are 512-byte aligned
+    return torch.empty(int(size.value), dtype=torch.uint8, device=device)
 
 
 def keypoints_for_grad(sift, kpts, octave):
@@ -106,73 +125,43 @@ def keypoints_for_grad(sift, kpts, octave):
 class _Descriptors(torch.autograd.Function):
     @staticmethod
     def forward(ctx, img, kps, sift):
-        n_oct, S, base, incs = pyramid_params(sift)
         x = img.detach().contiguous().float()
-        top = int(kps[:, 1].max().item()) if kps.shape[0] else 1
-        top = max(top, S)
-        levels = _levels(x, n_oct, S, base, incs, top)
-        lib = _lib.load()
-        n = kps.shape[0]
-        desc = torch.zeros((n, 128), dtype=torch.float32, device=img.device)
-        hist = torch.zeros((n, 128), dtype=torch.float32, device=img.device)
-        groups = {}
-        for i, (o, si) in enumerate(kps[:, :2].long().tolist()):
-            groups.setdefault((o, si), []).append(i)
-        for (o, si), idx in groups.items():
-            G = levels[o][si]
-            sel = torch.tensor(idx, dtype=torch.long)
-            kp = kps[sel][:, 2:5].float().contiguous().to(img.device)
-            ph = int(sift._cfg.desc_ph[si])
-            d = torch.empty((len(idx), 128), dtype=torch.float32, device=img.device)
-            h = torch.empty_like(d)
-            _lib.check(lib.pysift_desc_f32_forward(G.data_ptr(), G.shape[0], G.shape[1], G.stride(0), kp.data_ptr(),
-                                                   len(idx), ph, h.data_ptr(), d.data_ptr(), _st()),
-                       "pysift_desc_f32_forward")
-            dev_idx = sel.to(img.device)
-            desc[dev_idx] = d
-            hist[dev_idx] = h
-        ctx.save_for_backward(img, hist)
-        ctx.kps = kps
+        H, W = x.shape
+        rows, n_oct, top, sizes = _levels_plan(kps, sift, (H, W))
+        n = rows.shape[0]
+        rows = rows.pin_memory().to(img.device, non_blocking=True) if n else rows.to(img.device)
+        desc = torch.empty((n, 128), dtype=torch.float32, device=img.device)
+        hist = torch.empty_like(desc)
+        if n:
+            lib = _lib.load()
+            ws = _levels_workspace(lib, sift, (H, W), n_oct, top, 0, img.device)
+            _lib.check(lib.pysift_desc_levels_forward(ctypes.byref(sift._cfg), x.data_ptr(), H, W, W, rows.data_ptr(),
+                                                      n, n_oct, top, ws.data_ptr(), ws.numel(), hist.data_ptr(),
+                                                      desc.data_ptr(), _st()), "pysift_desc_levels_forward")
+        ctx.save_for_backward(img, hist, rows)
         ctx.sift = sift
-        ctx.groups = groups
+        ctx.plan = (n_oct, top, sizes)
         return desc
 
     @staticmethod
     def backward(ctx, gdesc):
-        img, hist = ctx.saved_tensors
-        sift, kps, groups = ctx.sift, ctx.kps, ctx.groups
-        n_oct, S, base, incs = pyramid_params(sift)
+        img, hist, rows = ctx.saved_tensors
+        sift = ctx.sift
+        n_oct, top, sizes = ctx.plan
         x = img.detach().contiguous().float()
-        top = max(int(kps[:, 1].max().item()) if kps.shape[0] else 1, S)
-        levels = _levels(x, n_oct, S, base, incs, top)       # recomputed, not stored
+        H, W = x.shape
+        for o, size in enumerate(sizes):
+            for r in list(sift._cfg.blur_radius[1 if o == 0 else 2:2 + top]):
+                if r >= min(size):
+                    raise ValueError(f"pysift_desc_levels_backward: radius {r} must be below both image sides")
         lib = _lib.load()
-        grads = [[torch.zeros_like(G) for G in lv] for lv in levels]
         gdesc = gdesc.contiguous().float()
-        for (o, si), idx in groups.items():
-            G = levels[o][si]
-            sel = torch.tensor(idx, dtype=torch.long)
-            kp = kps[sel][:, 2:5].float().contiguous().to(img.device)
-            ph = int(sift._cfg.desc_ph[si])
-            dev_idx = sel.to(img.device)
-            h = hist[dev_idx].contiguous()
-            gd = gdesc[dev_idx].contiguous()
-            gG = grads[o][si]
-            _lib.check(lib.pysift_desc_f32_backward(G.data_ptr(), G.shape[0], G.shape[1], G.stride(0), kp.data_ptr(),
-                                                    len(idx), ph, h.data_ptr(), gd.data_ptr(), gG.data_ptr(), _st()),
-                       "pysift_desc_f32_backward")
-        # adjoint of the level chain, highest octave first
-        for o in range(len(levels) - 1, -1, -1):
-            g = grads[o]
-            for s in range(len(g) - 1, 0, -1):
-                w, r = incs[s - 1]
-                if r > 0:
-                    _blur_adjoint(g[s], w, r, accumulate_into=g[s - 1])
-                else:
-                    g[s - 1] += g[s]
-            if o > 0:
-                grads[o - 1][S][::2, ::2] += g[0]
-        g0 = grads[0][0]
-        gx = _blur_adjoint(g0, *base) if base[1] > 0 else g0
+        ws = _levels_workspace(lib, sift, (H, W), n_oct, top, 1, img.device)   # levels recomputed, not stored
+        gx = torch.empty_like(x)
+        _lib.check(lib.pysift_desc_levels_backward(ctypes.byref(sift._cfg), x.data_ptr(), H, W, W, rows.data_ptr(),
+                                                   rows.shape[0], n_oct, top, ws.data_ptr(), ws.numel(),
+                                                   hist.data_ptr(), gdesc.data_ptr(), gx.data_ptr(), W, _st()),
+                   "pysift_desc_levels_backward")
         return gx.to(img.dtype), None, None
 
 

@@ -60,6 +60,50 @@ def test_blur_adjoint_is_the_transpose():
         assert abs(lhs - rhs) <= 1e-5 * max(abs(lhs), 1.0)
 
 
+@pytest.mark.parametrize("H,W,n_oct,sigma0,n", [
+    (97, 131, 3, 1.6, 40), (64, 64, 3, 1.6, 1), (65, 33, 2, 1.6, 9), (150, 101, 2, 4.0, 24), (31, 127, 1, 1.6, 3),
+])
+def test_descriptor_levels_match_torch_autograd(H, W, n_oct, sigma0, n):
+    """Keypoints of every octave and scale index 0 .. S + 2, some on the
+    image's rim, in one call; sides at the edges of the blur adjoint's 64 x 32
+    tiles, radii past its 16 at sigma0 = 4."""
+    import torch
+    from pysift_b200 import PySIFT, grad
+    rng = np.random.default_rng(n)
+    sift = PySIFT(double_image=False, n_octaves=n_oct, sigma0=sigma0)
+    img = torch.from_numpy(_img(H, W, 5)).cuda()
+    rows = []
+    for i in range(n):
+        o = i % min(n_oct, 2)
+        h, w = -(-H >> o), -(-W >> o)
+        rim = [(0, 0), (h - 1, w - 1), (0, w // 2)][i % 3] if i % 4 == 3 else (rng.integers(1, h - 1), rng.integers(1, w - 1))
+        rows.append([o, i % (4 if sigma0 > 2 else 6), rim[0], rim[1], rng.uniform(0, 360)])
+    kps = torch.tensor(np.array(rows, np.float64))
+    x = img.clone().requires_grad_(True)
+    d = grad.descriptors(x, kps, sift)
+    r = torch.from_numpy(rng.standard_normal(d.shape).astype(np.float32)).cuda()
+    (d * r).sum().backward()
+    x64 = img.double().clone().requires_grad_(True)
+    d64 = grad.descriptors_torch(x64, kps, sift)
+    (d64 * r.double()).sum().backward()
+    assert _rel(d.detach().cpu(), d64.detach().cpu()) < 1e-4
+    assert _rel(x.grad.cpu(), x64.grad.cpu()) < 1e-4
+
+
+def test_descriptor_levels_refuse_what_the_pyramid_lacks():
+    import torch
+    from pysift_b200 import grad
+    img = torch.from_numpy(_img(40, 40, 5)).cuda()
+    for row in ([3, 1, 2, 2, 0.0], [0, 6, 2, 2, 0.0], [0, -1, 2, 2, 0.0]):
+        with pytest.raises(IndexError):
+            grad.descriptors(img, torch.tensor([row], dtype=torch.float64), _sift(3))
+    small = torch.from_numpy(_img(64, 64, 5)).cuda().requires_grad_(True)  # octave 3 is 8x8, the blurs reach radius 8
+    d = grad.descriptors(small, torch.tensor([[0, 1, 30, 30, 0.0]], dtype=torch.float64), _sift(5))
+    with pytest.raises(ValueError):
+        d.sum().backward()
+    assert grad.descriptors(img, torch.empty((0, 5), dtype=torch.float64), _sift(3)).shape == (0, 128)
+
+
 def test_descriptor_forward_and_grad_match_torch_autograd():
     import torch
     from pysift_b200 import grad
