@@ -429,8 +429,7 @@ def run_match(args, wl, world, rank, local):
         "config": {"workload": args.workload, "N": N, "M": M, "D": D, "seed": wl["seed"], "ratio": 0.75,
                    "mutual_matches": n_pairs, "l2": "flushed (256 MiB write) before every step",
                    "parallelism": f"replicas{world}"},
-        "roofline": {"bound": "tensor", "kernel": "whole match call (k_row_norms_u8 x2, "
-                     + ("k_split_nibbles_u8 x2, " if split else "k_tile_rows x2, ") + "k_match_rows x2, k_match_merge_u8 x2, "
+        "roofline": {"bound": "tensor", "kernel": "whole match call (k_match_prep, k_match_rows, k_match_merge_u8, "
                      "k_match_mutual); flops 2*N*M*D counted once" + (" (the e4m3 GEMM does 4x that)" if split else ""),
                      "achieved": achieved, "peak": peak, "unit": "TFLOP/s", "frac": achieved / peak,
                      "peak_source": peak_kind, "alg_flops_per_step": flops,

@@ -1,8 +1,14 @@
 // match.cu -- brute-force ratio-test matching on the 5th-generation tensor cores.
 //
-// Matching runs as two row scans: queries against the train set (forward
-// top-2) and the train set against the queries (backward top-2).  Both sets
-// are first written in a tiled operand layout (128-row tiles of 16 KB slabs
+// Matching runs as two row scans in one grid: queries against the train set
+// (forward top-2) and the train set against the queries (backward top-2);
+// the preparation of the two sets and the merges of the two directions are
+// one launch each as well.  The launches of one direction leave the chip
+// partly idle (a small pair's scan is a few CTAs, any scan ends in a ragged
+// wave, a merge waits on memory), so the two overlap: 104 -> 75 us of
+// kernels for an 8192 x 8192 x 128 uint8 match, 85 -> 63 for 7919 x 5003 x 64
+// fp16, 44 -> 25 for 997 x 613 x 64 int8.
+// Both sets are first written in a tiled operand layout (128-row tiles of 16 KB slabs
 // in the no-swizzle K-major core-matrix layout).  Each CTA of k_match_rows
 // keeps a 128-row query tile resident in shared memory; a loader thread
 // streams the train slabs into a ring with one bulk copy each, an MMA thread
@@ -186,18 +192,6 @@ __host__ __device__ __forceinline__ size_t tiled_off(int r, int c, int RB) {
     return (size_t)(r / MT) * MT * RB + (size_t)slab * MT * SW * 16 + (size_t)(((rr >> 3) * SW + cs) * 128 + (rr & 7) * 16);
 }
 
-// Row-major rows of RB bytes (16-byte aligned) into the tiled layout, rows
-// n .. n_pad-1 zero.  One thread per 16-byte chunk.
-__global__ void k_tile_rows(const uint8_t* __restrict__ src, int n, int n_pad, int RB, uint8_t* __restrict__ dst) {
-    const int KC = RB / 16;
-    const long long q = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (q >= (long long)n_pad * KC) return;
-    const int r = (int)(q / KC), c = (int)(q - (long long)r * KC);
-    uint4 v = make_uint4(0u, 0u, 0u, 0u);
-    if (r < n) v = *reinterpret_cast<const uint4*>(src + (size_t)r * RB + (size_t)c * 16);
-    *reinterpret_cast<uint4*>(dst + tiled_off(r, c, RB)) = v;
-}
-
 // Bounded mbarrier wait that also gives up once another role of the CTA has
 // raised the abort flag.
 __device__ __forceinline__ bool mbar_wait_bounded(uint64_t* bar, uint32_t parity, const volatile int* abort_flag) {
@@ -239,7 +233,8 @@ __device__ __forceinline__ void umma_commit(uint64_t* bar) {
                  : "memory");
 }
 
-struct RowScanArgs {
+// One direction of a match: the queries q against the train rows t.
+struct ScanSide {
     const uint8_t* q;    // n_q rows of RB bytes (fp16 / uint8 / int8 / e4m3 codes), tiled
     const uint8_t* t;    // n_t rows of RB bytes
     int n_q, n_t;
@@ -247,8 +242,13 @@ struct RowScanArgs {
     const int* norm_ti;    // DIST_U8: |t|^2 per train row as int32, padded to whole tiles
     const float* scale_q;  // SIM_I8: quantisation scale per query row
     const float* scale_t;  //         and per train row
-    int seg_tiles;       // train tiles per segment (blockIdx.y)
-    void* part;          // [n_q][gridDim.y] Top3 (chunk level; SIM_I8: Top2 of columns)
+    int nseg, seg_tiles;   // segments of the train side and their tiles
+    void* part;            // [n_q][nseg] Top3 (chunk level; SIM_I8: Top2 of columns)
+};
+
+struct RowScanArgs {
+    ScanSide side[2];
+    int blocks0;         // CTAs of side 0
     int* error;          // set when an MMA wait gives up
 };
 
@@ -360,7 +360,7 @@ constexpr int EPI_WARPS = MATCH_THREADS / 32;
 constexpr int SCAN_THREADS = MATCH_THREADS + 64;
 
 template <int MODE, int RB>
-__global__ void __launch_bounds__(SCAN_THREADS, 2) k_match_rows(const RowScanArgs args) {
+__global__ void __launch_bounds__(SCAN_THREADS, 2) k_match_rows(const __grid_constant__ RowScanArgs all) {
     using G = TileGeom<RB>;
     constexpr int NS = G::NS;
     // SIM_F16, DIST_U8, SPLIT_FP8: chunk-level state (the key of each
@@ -375,8 +375,14 @@ __global__ void __launch_bounds__(SCAN_THREADS, 2) k_match_rows(const RowScanArg
     __shared__ Top3 s_half[MT];  // Top2 in the first 16 bytes for SIM_I8
 
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    // both directions in one grid: CTA -> (side, query tile, segment)
+    const int sd = (int)blockIdx.x >= all.blocks0 ? 1 : 0;
+    const ScanSide& args = all.side[sd];
+    const int bl = (int)blockIdx.x - (sd ? all.blocks0 : 0);
+    const int n_qb = (args.n_q + MT - 1) / MT;
+    const int seg = bl / n_qb, qb = bl - seg * n_qb;
     const int n_tt = (args.n_t + NT - 1) / NT;
-    const int t_begin = blockIdx.y * args.seg_tiles;
+    const int t_begin = seg * args.seg_tiles;
     const int nt = min(n_tt, t_begin + args.seg_tiles) - t_begin;  // >= 1 by construction
 
     if (warp == 0) {
@@ -404,14 +410,14 @@ __global__ void __launch_bounds__(SCAN_THREADS, 2) k_match_rows(const RowScanArg
     const uint32_t tmem = tmem_base;
     auto give_up = [&]() {
         s_abort = 1;
-        atomicExch(args.error, 1);
+        atomicExch(all.error, 1);
     };
 
     if (warp == EPI_WARPS) {
         // ---- loader ----
         if (lane == 0) {
             mbar_expect_tx(&bar_q, G::TILE);
-            bulk_load(sQ, args.q + (size_t)blockIdx.x * G::TILE, G::TILE, &bar_q);
+            bulk_load(sQ, args.q + (size_t)qb * G::TILE, G::TILE, &bar_q);
             int issued = 0;  // slabs
             const int total = nt * G::NSL;
             for (int k = 0; k < total; ++k) {
@@ -494,7 +500,7 @@ __global__ void __launch_bounds__(SCAN_THREADS, 2) k_match_rows(const RowScanArg
         // ---- reducers ----
         const int quad = warp & 3, half = warp >> 2;  // TMEM lane quadrant, column half of each tile
         const int rloc = quad * 32 + lane;            // this thread's query row in the block
-        const int q0 = blockIdx.x * MT;
+        const int q0 = qb * MT;
         const float sq = (MODE == SIM_I8 && q0 + rloc < args.n_q) ? args.scale_q[q0 + rloc] : 1.0f;
         float k1 = -INFINITY, k2 = -INFINITY, m1 = -INFINITY, m2 = -INFINITY;
         int i1 = 0x7fffffff, j1 = 0x7fffffff;
@@ -556,7 +562,7 @@ __global__ void __launch_bounds__(SCAN_THREADS, 2) k_match_rows(const RowScanArg
             if (half == 0 && !s_abort && row < args.n_q) {
                 top3_merge(tc, s_half[rloc]);
                 tc.pad[0] = tc.pad[1] = tc.pad[2] = 0;
-                static_cast<Top3*>(args.part)[(size_t)row * gridDim.y + blockIdx.y] = tc;
+                static_cast<Top3*>(args.part)[(size_t)row * args.nseg + seg] = tc;
             }
         } else {
             top2_merge(k1, k2, i1, m1, m2, j1);
@@ -578,7 +584,7 @@ __global__ void __launch_bounds__(SCAN_THREADS, 2) k_match_rows(const RowScanArg
                 r.k2 = k2;
                 r.i1 = i1;
                 r.pad = 0;
-                static_cast<Top2*>(args.part)[(size_t)row * gridDim.y + blockIdx.y] = r;
+                static_cast<Top2*>(args.part)[(size_t)row * args.nseg + seg] = r;
             }
         }
     }
@@ -587,11 +593,45 @@ __global__ void __launch_bounds__(SCAN_THREADS, 2) k_match_rows(const RowScanArg
     if (warp == 0) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(2 * NT));
 }
 
+// The merge of both directions in one launch: blocks 0 .. blocks0 - 1 take
+// side 0's rows, the others side 1's.
+struct MergeSide {
+    const void* part;     // the scan's segments
+    int n, nseg;
+    const uint8_t* q;     // row-major rows as the caller passed them
+    const uint8_t* t;
+    int n_t;
+    const int* norm_q;    // uint8 modes: |row|^2
+    const int* norm_t;
+    const float* fnorm_q;         // SIM_F16: row norms rounded up
+    const unsigned* maxnorm_t;    //          and the train side's largest
+    int* best;
+    int* pass;
+    float* dist;
+    int* recheck;         // SIM_F16: rows left to the full recomputation
+    int* n_recheck;
+};
+
+struct MergeArgs {
+    MergeSide side[2];
+    int blocks0;
+    float ratio_sq;
+    int D;
+    const int* error;
+};
+
 // SIM_I8: merge the column-level segments of one scan (in index order),
 // ratio test on the similarities (pysift/core.py:2676-2680, float32).
-__global__ void k_match_merge_i8(const Top2* __restrict__ part, int n, int nseg, float ratio_sq,
-                                 int* __restrict__ best, int* __restrict__ pass, float* __restrict__ dist) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+__global__ void k_match_merge_i8(const __grid_constant__ MergeArgs m) {
+    const int sd = (int)blockIdx.x >= m.blocks0 ? 1 : 0;
+    const MergeSide& z = m.side[sd];
+    const Top2* __restrict__ part = static_cast<const Top2*>(z.part);
+    const int n = z.n, nseg = z.nseg;
+    const float ratio_sq = m.ratio_sq;
+    int* __restrict__ best = z.best;
+    int* __restrict__ pass = z.pass;
+    float* __restrict__ dist = z.dist;
+    const int i = ((int)blockIdx.x - (sd ? m.blocks0 : 0)) * blockDim.x + threadIdx.x;
     if (i >= n) return;
     float k1 = -INFINITY, k2 = -INFINITY;
     int i1 = 0x7fffffff;
@@ -659,15 +699,23 @@ __device__ __forceinline__ Top3 merge_parts(const Top3* __restrict__ part, int i
 // and the other chunks' largest (a.k2).  Keys 2 a.b - |b|^2 are exact
 // integers on both sides, so the recomputed maximum equals a.k1; a mismatch
 // (or a scan that gave up) leaves the row without a match.
-__global__ void k_match_merge_u8(const Top3* __restrict__ part, int n, int nseg, float ratio_sq,
-                                 const uint8_t* __restrict__ q, const uint8_t* __restrict__ t, int n_t, int D,
-                                 const int* __restrict__ norm_q, const int* __restrict__ norm_t,
-                                 const int* __restrict__ error, int* __restrict__ best, int* __restrict__ pass,
-                                 float* __restrict__ dist) {
-    const int i = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5), lane = threadIdx.x & 31;
-    if (i >= n) return;
-    const Top3 a = merge_parts(part, i, nseg);
-    const bool bad = *error || !(a.k1 > -INFINITY) || a.i1 < 0 || a.i1 >= n_t;
+__global__ void k_match_merge_u8(const __grid_constant__ MergeArgs m) {
+    const int sd = (int)blockIdx.x >= m.blocks0 ? 1 : 0;
+    const MergeSide& z = m.side[sd];
+    const uint8_t* __restrict__ q = z.q;
+    const uint8_t* __restrict__ t = z.t;
+    const int* __restrict__ norm_q = z.norm_q;
+    const int* __restrict__ norm_t = z.norm_t;
+    const int n_t = z.n_t, D = m.D;
+    const float ratio_sq = m.ratio_sq;
+    int* __restrict__ best = z.best;
+    int* __restrict__ pass = z.pass;
+    float* __restrict__ dist = z.dist;
+    const int i = ((int)blockIdx.x - (sd ? m.blocks0 : 0)) * (blockDim.x >> 5) + (threadIdx.x >> 5);
+    const int lane = threadIdx.x & 31;
+    if (i >= z.n) return;
+    const Top3 a = merge_parts(static_cast<const Top3*>(z.part), i, z.nseg);
+    const bool bad = *m.error || !(a.k1 > -INFINITY) || a.i1 < 0 || a.i1 >= n_t;
     unsigned long long kb = 0, ks = 0;
     if (!bad) {
         const int c = a.i1 + lane;
@@ -752,36 +800,6 @@ __device__ __forceinline__ double dot_f16_exact(const __half* a, const __half* b
     return (acc[0] + acc[1]) + (acc[2] + acc[3]);
 }
 
-// Row L2 norms of the two fp16 sets (set 1's rows, then set 2's) and the
-// largest of each set, rounded up with a relative margin of 2^-20, the
-// largest as float bits (non-negative floats order as their bits, so the
-// integer maximum is the float maximum and the result does not depend on the
-// order of the updates).  One warp per row; the block's largest per set
-// goes to one atomicMax each.
-__global__ void k_f16_max_norms(const __half* __restrict__ a, int n1, const __half* __restrict__ b, int n2, int D,
-                                unsigned* __restrict__ out, float* __restrict__ row_norm) {
-    __shared__ unsigned s_max[2];
-    if (threadIdx.x < 2) s_max[threadIdx.x] = 0u;
-    __syncthreads();
-    const int w = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5), lane = threadIdx.x & 31;
-    if (w < n1 + n2) {
-        const __half* row = w < n1 ? a + (size_t)w * D : b + (size_t)(w - n1) * D;
-        double s = 0.0;
-        for (int k = lane; k < D; k += 32) {
-            const float f = __half2float(row[k]);
-            s += (double)__fmul_rn(f, f);
-        }
-        for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(FULL_MASK, s, o);
-        if (lane == 0) {
-            const float nrm = __double2float_ru(sqrt(s) * (1.0 + 0x1p-20));
-            row_norm[w] = nrm;
-            atomicMax(&s_max[w < n1 ? 0 : 1], __float_as_uint(nrm));
-        }
-    }
-    __syncthreads();
-    if (threadIdx.x < 2 && s_max[threadIdx.x]) atomicMax(&out[threadIdx.x], s_max[threadIdx.x]);
-}
-
 __device__ __forceinline__ void finish_f16_row(int i, float f1, float f2, int c1, float ratio_sq, int* best, int* pass,
                                                float* dist) {
     // pysift/core.py:2676-2680 (float32); no second column: no pass
@@ -825,19 +843,24 @@ __device__ __forceinline__ int sim_key_column(unsigned long long k) {
 // tying F1 could have a lower index).  Unsettled rows are appended to
 // `recheck` (their order there does not matter: each row's result is
 // computed on its own).
-__global__ void k_match_merge_f16(const Top3* __restrict__ part, int n, int nseg, float ratio_sq,
-                                  const __half* __restrict__ q, const __half* __restrict__ t, int n_t, int D,
-                                  const float* __restrict__ norm_q, const unsigned* __restrict__ maxnorm_t,
-                                  const int* __restrict__ error,
-                                  int* __restrict__ best, int* __restrict__ pass, float* __restrict__ dist,
-                                  int* __restrict__ recheck, int* __restrict__ n_recheck) {
-    const int i = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5), lane = threadIdx.x & 31;
-    if (i >= n) return;
-    const Top3 a = merge_parts(part, i, nseg);
+__global__ void k_match_merge_f16(const __grid_constant__ MergeArgs m) {
+    const int sd = (int)blockIdx.x >= m.blocks0 ? 1 : 0;
+    const MergeSide& z = m.side[sd];
+    const __half* __restrict__ q = reinterpret_cast<const __half*>(z.q);
+    const __half* __restrict__ t = reinterpret_cast<const __half*>(z.t);
+    const int n_t = z.n_t, D = m.D;
+    const float ratio_sq = m.ratio_sq;
+    int* __restrict__ best = z.best;
+    int* __restrict__ pass = z.pass;
+    float* __restrict__ dist = z.dist;
+    const int i = ((int)blockIdx.x - (sd ? m.blocks0 : 0)) * (blockDim.x >> 5) + (threadIdx.x >> 5);
+    const int lane = threadIdx.x & 31;
+    if (i >= z.n) return;
+    const Top3 a = merge_parts(static_cast<const Top3*>(z.part), i, z.nseg);
     // a scan that gave up on its MMA barrier left its parts unwritten: no
     // result, and no candidate chunk is trusted
     const bool c2 = a.k2 > -INFINITY;
-    if (*error || !(a.k1 > -INFINITY) || a.i1 < 0 || a.i1 >= n_t || (c2 && (a.i2 < 0 || a.i2 >= n_t))) {
+    if (*m.error || !(a.k1 > -INFINITY) || a.i1 < 0 || a.i1 >= n_t || (c2 && (a.i2 < 0 || a.i2 >= n_t))) {
         if (lane == 0) {
             best[i] = -1;
             pass[i] = 0;
@@ -859,10 +882,10 @@ __global__ void k_match_merge_f16(const Top3* __restrict__ part, int n, int nseg
     const float f1 = sim_key_value(kb);
     const float f2 = ks ? sim_key_value(ks) : -INFINITY;
     if (a.k3 > -INFINITY) {
-        const double e = (double)D * 0x1p-21 * (double)norm_q[i] * (double)__uint_as_float(*maxnorm_t);
+        const double e = (double)D * 0x1p-21 * (double)z.fnorm_q[i] * (double)__uint_as_float(*z.maxnorm_t);
         const float u = f16_round_f64((double)a.k3 + e);
         if (!(u <= f2 && u < f1)) {
-            recheck[atomicAdd(n_recheck, 1)] = i;
+            z.recheck[atomicAdd(z.n_recheck, 1)] = i;
             return;
         }
     }
@@ -923,96 +946,169 @@ __global__ void __launch_bounds__(RECHECK_T) k_match_recheck_f16(const int* __re
     }
 }
 
-// Mutual matches in query order: fwd[i] = j passes, bwd[j] = i passes.
-// One CTA; each thread owns a run of up to 32 consecutive rows (so the pairs
-// of a thread are consecutive in the output), tests them with its loads
-// issued eight rows at a time, and one block scan of the per-thread counts
-// places them; more than 32 x blockDim rows take several rounds.
+// Mutual matches in query order: fwd[i] = j passes, bwd[j] = i passes.  One
+// CTA: a warp covers 256 consecutive rows a round (coalesced loads, 8 rows a
+// lane with both gathers of all of them in flight), ballots place the pairs.
 __global__ void __launch_bounds__(1024) k_match_mutual(const int* __restrict__ fbest, const int* __restrict__ fpass,
                                                        const float* __restrict__ fdist, const int* __restrict__ bbest,
                                                        const int* __restrict__ bpass, int n1, int2* __restrict__ pairs,
                                                        float* __restrict__ pdist, int* __restrict__ count) {
     __shared__ int sh[33];
-    const int span = (int)blockDim.x * 32;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const unsigned below = (1u << lane) - 1u;
+    constexpr int K = 8;
     int base = 0;
-    for (int c0 = 0; c0 < n1; c0 += span) {
-        const int per = min(32, ceil_div(min(span, n1 - c0), (int)blockDim.x));
-        const int r0 = c0 + (int)threadIdx.x * per;
-        unsigned mask = 0;
-        for (int k0 = 0; k0 < per; k0 += 8) {
-            int j[8];
+    for (int c0 = 0; c0 < n1; c0 += 1024 * K) {
+        const int w0 = c0 + warp * 32 * K;
+        int j[K], p[K], b[K];
+        float d[K];
 #pragma unroll
-            for (int u = 0; u < 8; ++u) {
-                const int i = r0 + k0 + u;
-                j[u] = (k0 + u < per && i < n1 && fpass[i]) ? fbest[i] : -1;
-            }
+        for (int k = 0; k < K; ++k) {
+            const int i = w0 + k * 32 + lane;
+            const bool in = i < n1;
+            p[k] = in ? fpass[i] : 0;
+            j[k] = in ? fbest[i] : -1;
+            d[k] = in ? fdist[i] : 0.0f;
+        }
 #pragma unroll
-            for (int u = 0; u < 8; ++u) {
-                const int i = r0 + k0 + u;
-                if (j[u] >= 0 && bpass[j[u]] && bbest[j[u]] == i) mask |= 1u << (k0 + u);
-            }
+        for (int k = 0; k < K; ++k) {
+            const bool ok = p[k] && j[k] >= 0;
+            p[k] = ok ? bpass[j[k]] : 0;
+            b[k] = ok ? bbest[j[k]] : -1;
+        }
+        unsigned bal[K];
+        int cnt = 0;
+#pragma unroll
+        for (int k = 0; k < K; ++k) {
+            bal[k] = __ballot_sync(FULL_MASK, p[k] && b[k] == w0 + k * 32 + lane);
+            cnt += __popc(bal[k]);
         }
         int tot;
-        int pos = base + block_excl_scan(__popc(mask), &tot, sh);
-        while (mask) {
-            const int k = __ffs(mask) - 1;
-            mask &= mask - 1;
-            const int i = r0 + k;
-            pairs[pos] = make_int2(i, fbest[i]);
-            pdist[pos] = fdist[i];
-            ++pos;
+        int pos = base + block_warp_excl_scan(cnt, &tot, sh);
+#pragma unroll
+        for (int k = 0; k < K; ++k) {
+            if ((bal[k] >> lane) & 1u) {
+                const int at = pos + __popc(bal[k] & below);
+                pairs[at] = make_int2(w0 + k * 32 + lane, j[k]);
+                pdist[at] = d[k];
+            }
+            pos += __popc(bal[k]);
         }
         base += tot;
     }
     if (threadIdx.x == 0) *count = base;
 }
 
-// |row|^2 of uint8 rows as int32 and float32 (exact: below 2^24).  Rows
-// n .. n_pad-1 get zero norms.
-__global__ void k_row_norms_u8(const uint8_t* __restrict__ d, int n, int n_pad, int D, int* __restrict__ norms,
-                               float* __restrict__ fnorms) {
-    const int i = blockIdx.x * blockDim.y + threadIdx.y;
-    if (i >= n_pad) return;
-    int s = 0;
-    for (int k = threadIdx.x; k < D; k += 32) {
-        const int v = i < n ? d[(size_t)i * D + k] : 0;
-        s += v * v;
+// The scan operands of both sets in one launch: the rows (16-byte aligned)
+// into the tiled layout with zero rows up to whole tiles, and what the mode
+// needs of each row.  A 16-byte chunk a thread, a row's chunks in adjacent
+// lanes.
+//   SIM_F16    row L2 norms and the largest of each set, rounded up with a
+//              relative margin of 2^-20, the largest as float bits
+//              (non-negative floats order as their bits); maxnorm is zeroed
+//              beforehand
+//   SIM_I8     the rows alone
+//   DIST_U8    |row|^2 as int32
+//   SPLIT_FP8  |row|^2 as int32 and float32 (exact: below 2^24), and
+//              split-nibble e4m3 planes: v = 16 h + l with h, l in 0..15 (e4m3
+//              holds 0..15 and 16 * (0..15) exactly); the query-side row is
+//              [16h | h | 16l | l], the train-side row [16h | 16l | h | l], each
+//              plane D bytes, so that the 4D-long dot product of the two is
+//              256 h.h' + 16 h.l' + 16 l.h' + l.l' = v.v', the four nibble GEMMs in one
+struct PrepSide {
+    const uint8_t* rows;
+    int n, n_pad;
+    uint8_t* q;   // tiled; the query side for SPLIT_FP8
+    uint8_t* t;   // SPLIT_FP8: the train side
+    int* norm;
+    float* fnorm;
+    unsigned* maxnorm;
+};
+struct PrepArgs {
+    PrepSide side[2];
+    int blocks0;
+    int RB;       // bytes of a row
+    int* ctl;     // zeroed by the first block except for SIM_F16
+};
+constexpr int PREP_T = 256, CTL_INTS = 8;
+
+__device__ __forceinline__ uint4 e4m3x16(const uint4& v, int shift, float scale) {
+    const uint32_t w[4] = {v.x, v.y, v.z, v.w};
+    uint32_t o[4];
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+        o[q] = 0u;
+#pragma unroll
+        for (int b = 0; b < 4; ++b) {
+            const float x = scale * (float)((w[q] >> (8 * b + shift)) & 15u);
+            o[q] |= (uint32_t)__nv_cvt_float_to_fp8(x, __NV_SATFINITE, __NV_E4M3) << (8 * b);
+        }
     }
-    for (int o = 16; o > 0; o >>= 1) s += __shfl_down_sync(FULL_MASK, s, o);
-    if (threadIdx.x == 0) {
-        norms[i] = s;
-        fnorms[i] = (float)s;
-    }
+    return make_uint4(o[0], o[1], o[2], o[3]);
 }
 
-// Split-nibble e4m3 planes of uint8-valued rows, v = 16 h + l with h, l in
-// 0..15 (e4m3 holds 0..15 and 16 * (0..15) exactly).  The query-side row is
-// [16h | h | 16l | l], the train-side row [16h | 16l | h | l], each plane D
-// bytes, so that the 4D-long dot product of the two is
-// 256 h.h' + 16 h.l' + 16 l.h' + l.l' = v.v', the four nibble GEMMs in one.
-// Both sides are written in the tiled layout of 4D-byte rows; rows
-// n .. n_pad-1 are zero.
-__global__ void k_split_nibbles_u8(const uint8_t* __restrict__ d, int n, int n_pad, int D,
-                                   uint8_t* __restrict__ qside, uint8_t* __restrict__ tside) {
-    const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= (size_t)n_pad * D) return;
-    const int r = (int)(i / D), k = (int)(i - (size_t)r * D);
-    const int v = r < n ? d[i] : 0;
-    const float h = (float)(v >> 4), l = (float)(v & 15);
-    const uint8_t e16h = __nv_cvt_float_to_fp8(16.0f * h, __NV_SATFINITE, __NV_E4M3);
-    const uint8_t eh = __nv_cvt_float_to_fp8(h, __NV_SATFINITE, __NV_E4M3);
-    const uint8_t e16l = __nv_cvt_float_to_fp8(16.0f * l, __NV_SATFINITE, __NV_E4M3);
-    const uint8_t el = __nv_cvt_float_to_fp8(l, __NV_SATFINITE, __NV_E4M3);
-    const int RB = 4 * D;
-    auto at = [&](int byte) { return tiled_off(r, byte >> 4, RB) + (byte & 15); };
-    qside[at(k)] = e16h;
-    qside[at(D + k)] = eh;
-    qside[at(2 * D + k)] = e16l;
-    qside[at(3 * D + k)] = el;
-    tside[at(k)] = e16h;
-    tside[at(D + k)] = e16l;
-    tside[at(2 * D + k)] = eh;
-    tside[at(3 * D + k)] = el;
+template <int MODE>
+__global__ void __launch_bounds__(PREP_T) k_match_prep(const __grid_constant__ PrepArgs a) {
+    __shared__ unsigned s_max;
+    const int sd = (int)blockIdx.x >= a.blocks0 ? 1 : 0;
+    const PrepSide& z = a.side[sd];
+    const int KC = a.RB / 16;  // 4, 8 or 16
+    const long long g = (long long)((int)blockIdx.x - (sd ? a.blocks0 : 0)) * PREP_T + threadIdx.x;
+    const int r = (int)(g / KC), c = (int)(g - (long long)r * KC);
+    if (MODE == SIM_F16) {
+        if (threadIdx.x == 0) s_max = 0u;
+        __syncthreads();
+    } else if (blockIdx.x == 0 && threadIdx.x < CTL_INTS) {
+        a.ctl[threadIdx.x] = 0;
+    }
+    uint4 v = make_uint4(0u, 0u, 0u, 0u);
+    if (r < z.n) v = reinterpret_cast<const uint4*>(z.rows)[g];
+    const bool in = r < z.n_pad;
+    if (MODE == SPLIT_FP8) {
+        if (in) {
+            const uint4 hh = e4m3x16(v, 4, 16.0f), h = e4m3x16(v, 4, 1.0f), ll = e4m3x16(v, 0, 16.0f),
+                        l = e4m3x16(v, 0, 1.0f);
+            const int RS = 4 * a.RB;
+            const uint4 q[4] = {hh, h, ll, l}, t[4] = {hh, ll, h, l};
+#pragma unroll
+            for (int k = 0; k < 4; ++k) {
+                *reinterpret_cast<uint4*>(z.q + tiled_off(r, c + k * KC, RS)) = q[k];
+                *reinterpret_cast<uint4*>(z.t + tiled_off(r, c + k * KC, RS)) = t[k];
+            }
+        }
+    } else if (in) {
+        *reinterpret_cast<uint4*>(z.q + tiled_off(r, c, a.RB)) = v;
+    }
+    if (MODE == DIST_U8 || MODE == SPLIT_FP8) {
+        unsigned s = 0u;
+        s = __dp4a(v.x, v.x, s);
+        s = __dp4a(v.y, v.y, s);
+        s = __dp4a(v.z, v.z, s);
+        s = __dp4a(v.w, v.w, s);
+        for (int o = KC / 2; o > 0; o >>= 1) s += __shfl_xor_sync(FULL_MASK, s, o);
+        if (in && c == 0) {
+            z.norm[r] = (int)s;
+            if (MODE == SPLIT_FP8) z.fnorm[r] = (float)s;
+        }
+    }
+    if (MODE == SIM_F16) {
+        double s = 0.0;
+        const __half2* h = reinterpret_cast<const __half2*>(&v);
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+            const float2 f = __half22float2(h[k]);
+            s += (double)__fmul_rn(f.x, f.x);
+            s += (double)__fmul_rn(f.y, f.y);
+        }
+        for (int o = KC / 2; o > 0; o >>= 1) s += __shfl_xor_sync(FULL_MASK, s, o);
+        if (r < z.n && c == 0) {
+            const float nrm = __double2float_ru(sqrt(s) * (1.0 + 0x1p-20));
+            z.fnorm[r] = nrm;
+            atomicMax(&s_max, __float_as_uint(nrm));
+        }
+        __syncthreads();
+        if (threadIdx.x == 0 && s_max) atomicMax(z.maxnorm, s_max);
+    }
 }
 
 static int sm_count() {
@@ -1022,50 +1118,65 @@ static int sm_count() {
     return n > 0 ? n : 148;
 }
 
-// Segments of the train side.  Two CTAs fit on an SM (tensor memory), so a
-// grid of n_qb x nseg CTAs runs in ceil(n_qb nseg / (2 SMs)) waves of
-// ceil(n_tt / nseg) tiles each (+1 for a CTA's prologue): the segment count
-// with the fewest tile-steps is taken (the smaller one on ties), so that a
-// few CTAs past a full wave do not double the scan.
-static void scan_split(int n_q, int n_t, int& nseg, int& seg_tiles) {
-    const int n_qb = ceil_div(n_q, MT), n_tt = ceil_div(n_t, NT);
+// Segments of the two directions' train sides, of st tiles at most.  Two CTAs
+// fit on an SM (tensor memory), so the common grid of n_qb1 nseg1 + n_qb2
+// nseg2 CTAs runs in whole waves of 2 CTAs per SM, each about st tiles long
+// (+3 for a CTA's start: allocation, the query tile and the first slabs take
+// as long as three tiles): the st with the fewest tile-steps is taken (the
+// larger one on ties), so that a few CTAs past a full wave do not double the
+// scan.
+static void scan_split(ScanSide side[2]) {
     const long long slots = 2LL * sm_count();
+    int n_qb[2], n_tt[2];
+    for (int d = 0; d < 2; ++d) {
+        n_qb[d] = ceil_div(side[d].n_q, MT);
+        n_tt[d] = ceil_div(side[d].n_t, NT);
+    }
+    const int top = std::max(n_tt[0], n_tt[1]);
     long long best = -1;
-    nseg = 1;
-    for (int s_ = 1; s_ <= n_tt; ++s_) {
-        const int st_ = ceil_div(n_tt, s_);
-        if (ceil_div(n_tt, st_) != s_) continue;  // a segment count that leaves none empty
-        const long long waves = (n_qb * (long long)s_ + slots - 1) / slots;
-        const long long cost = waves * (st_ + 1);
+    int best_st = top;
+    for (int st = top; st >= 1; --st) {
+        long long ctas = 0;
+        int longest = 0;
+        for (int d = 0; d < 2; ++d) {
+            const int nseg = ceil_div(n_tt[d], st);
+            ctas += (long long)n_qb[d] * nseg;
+            longest = std::max(longest, ceil_div(n_tt[d], nseg));
+        }
+        const long long cost = (ctas + slots - 1) / slots * (longest + 3);
         if (best < 0 || cost < best) {
             best = cost;
-            nseg = s_;
+            best_st = st;
         }
     }
-    seg_tiles = ceil_div(n_tt, nseg);
-    nseg = ceil_div(n_tt, seg_tiles);
+    for (int d = 0; d < 2; ++d) {
+        side[d].seg_tiles = ceil_div(n_tt[d], ceil_div(n_tt[d], best_st));
+        side[d].nseg = ceil_div(n_tt[d], side[d].seg_tiles);
+    }
 }
 
 template <int MODE, int RB>
-static int launch_scan(const RowScanArgs& a, int nseg, cudaStream_t st) {
+static int launch_scan(const RowScanArgs& a, int blocks, cudaStream_t st) {
     // query tile + the slab ring: about 96 KB, so that no more than two CTAs
     // (2 x 256 tensor-memory columns) share an SM
     using G = TileGeom<RB>;
     const size_t smem_launch = std::max((size_t)G::TILE + (size_t)G::NS * G::SLAB, (size_t)80 * 1024);
     PYSIFT_CUDA_TRY(cudaFuncSetAttribute(k_match_rows<MODE, RB>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                          (int)smem_launch));
-    dim3 grid(ceil_div(a.n_q, MT), nseg);
-    k_match_rows<MODE, RB><<<grid, SCAN_THREADS, smem_launch, st>>>(a);
+    k_match_rows<MODE, RB><<<blocks, SCAN_THREADS, smem_launch, st>>>(a);
     PYSIFT_LAUNCH_CHECK("k_match_rows");
     return PYSIFT_OK;
 }
 
 // row bytes: 2 D for fp16 rows, 4 D for the split e4m3 planes, D for uint8 / int8
-static int launch_scan_mode(int mode, const RowScanArgs& a, int D, int nseg, cudaStream_t st) {
-    if (mode == SIM_I8) return D == 64 ? launch_scan<SIM_I8, 64>(a, nseg, st) : launch_scan<SIM_I8, 128>(a, nseg, st);
-    if (mode == SIM_F16) return D == 64 ? launch_scan<SIM_F16, 128>(a, nseg, st) : launch_scan<SIM_F16, 256>(a, nseg, st);
-    if (mode == DIST_U8) return D == 64 ? launch_scan<DIST_U8, 64>(a, nseg, st) : launch_scan<DIST_U8, 128>(a, nseg, st);
-    return D == 64 ? launch_scan<SPLIT_FP8, 256>(a, nseg, st) : launch_scan<SPLIT_FP8, 512>(a, nseg, st);
+static int launch_scan_mode(int mode, const RowScanArgs& a, int D, int blocks, cudaStream_t st) {
+    if (mode == SIM_I8)
+        return D == 64 ? launch_scan<SIM_I8, 64>(a, blocks, st) : launch_scan<SIM_I8, 128>(a, blocks, st);
+    if (mode == SIM_F16)
+        return D == 64 ? launch_scan<SIM_F16, 128>(a, blocks, st) : launch_scan<SIM_F16, 256>(a, blocks, st);
+    if (mode == DIST_U8)
+        return D == 64 ? launch_scan<DIST_U8, 64>(a, blocks, st) : launch_scan<DIST_U8, 128>(a, blocks, st);
+    return D == 64 ? launch_scan<SPLIT_FP8, 256>(a, blocks, st) : launch_scan<SPLIT_FP8, 512>(a, blocks, st);
 }
 
 struct MatchLayout {
@@ -1104,7 +1215,7 @@ static MatchLayout match_layout(int n1, int n2, int D, int exact) {
     l.off_bbest = take((size_t)n2 * 4);
     l.off_bpass = take((size_t)n2 * 4);
     l.off_bdist = take((size_t)n2 * 4);
-    l.off_ctl = take(8 * sizeof(int));
+    l.off_ctl = take(CTL_INTS * sizeof(int));
     l.off_rl0 = l.off_rl1 = l.off_nrm = 0;
     if (exact == 0) {
         l.off_rl0 = take((size_t)n1 * 4);
@@ -1147,7 +1258,6 @@ static int run_match(int mode, const uint8_t* rows_a, int n1, const uint8_t* row
                      const float* sb = nullptr) {
     int* ctl = wsp<int>(ws, l.off_ctl);
     int* err = ctl;
-    PYSIFT_CUDA_TRY(cudaMemsetAsync(ctl, 0, 8 * sizeof(int), st));
     const __half* ha = reinterpret_cast<const __half*>(rows_a);
     const __half* hb = reinterpret_cast<const __half*>(rows_b);
     unsigned* maxnorm = reinterpret_cast<unsigned*>(ctl + 3);
@@ -1161,33 +1271,27 @@ static int run_match(int mode, const uint8_t* rows_a, int n1, const uint8_t* row
     int* nb = !sim ? wsp<int>(ws, l.off_nb) : nullptr;
     float* fna = !sim ? wsp<float>(ws, l.off_fna) : nullptr;
     float* fnb = !sim ? wsp<float>(ws, l.off_fnb) : nullptr;
-    if (sim) {
-        const int rb = mode == SIM_F16 ? 2 * D : D;
-        k_tile_rows<<<(unsigned)ceil_div_ll((long long)p1 * (rb / 16), 256), 256, 0, st>>>(rows_a, n1, p1, rb, qa);
-        PYSIFT_LAUNCH_CHECK("k_tile_rows");
-        k_tile_rows<<<(unsigned)ceil_div_ll((long long)p2 * (rb / 16), 256), 256, 0, st>>>(rows_b, n2, p2, rb, qb);
-        PYSIFT_LAUNCH_CHECK("k_tile_rows");
-    } else {
-        k_row_norms_u8<<<ceil_div(p1, 8), dim3(32, 8), 0, st>>>(rows_a, n1, p1, D, na, fna);
-        PYSIFT_LAUNCH_CHECK("k_row_norms_u8");
-        k_row_norms_u8<<<ceil_div(p2, 8), dim3(32, 8), 0, st>>>(rows_b, n2, p2, D, nb, fnb);
-        PYSIFT_LAUNCH_CHECK("k_row_norms_u8");
-        if (mode == DIST_U8) {
-            k_tile_rows<<<(unsigned)ceil_div_ll((long long)p1 * (D / 16), 256), 256, 0, st>>>(rows_a, n1, p1, D, qa);
-            PYSIFT_LAUNCH_CHECK("k_tile_rows");
-            k_tile_rows<<<(unsigned)ceil_div_ll((long long)p2 * (D / 16), 256), 256, 0, st>>>(rows_b, n2, p2, D, qb);
-            PYSIFT_LAUNCH_CHECK("k_tile_rows");
+    float* hna = mode == SIM_F16 ? wsp<float>(ws, l.off_nrm) : nullptr;
+    {
+        PrepArgs pa;
+        pa.RB = mode == SIM_F16 ? 2 * D : D;
+        pa.ctl = ctl;
+        pa.side[0] = PrepSide{rows_a, n1, p1, qa, ta, na, mode == SIM_F16 ? hna : fna, maxnorm};
+        pa.side[1] = PrepSide{rows_b, n2, p2, qb, tb, nb, mode == SIM_F16 ? hna + n1 : fnb, maxnorm + 1};
+        const int KC = pa.RB / 16;
+        pa.blocks0 = (int)ceil_div_ll((long long)p1 * KC, PREP_T);
+        const int blocks = pa.blocks0 + (int)ceil_div_ll((long long)p2 * KC, PREP_T);
+        if (mode == SIM_F16) {
+            PYSIFT_CUDA_TRY(cudaMemsetAsync(ctl, 0, CTL_INTS * sizeof(int), st));
+            k_match_prep<SIM_F16><<<blocks, PREP_T, 0, st>>>(pa);
+        } else if (mode == SIM_I8) {
+            k_match_prep<SIM_I8><<<blocks, PREP_T, 0, st>>>(pa);
+        } else if (mode == DIST_U8) {
+            k_match_prep<DIST_U8><<<blocks, PREP_T, 0, st>>>(pa);
+        } else {
+            k_match_prep<SPLIT_FP8><<<blocks, PREP_T, 0, st>>>(pa);
         }
-        if (mode == SPLIT_FP8) {
-            k_split_nibbles_u8<<<(unsigned)ceil_div_ll((long long)p1 * D, 256), 256, 0, st>>>(rows_a, n1, p1, D, qa, ta);
-            PYSIFT_LAUNCH_CHECK("k_split_nibbles_u8");
-            k_split_nibbles_u8<<<(unsigned)ceil_div_ll((long long)p2 * D, 256), 256, 0, st>>>(rows_b, n2, p2, D, qb, tb);
-            PYSIFT_LAUNCH_CHECK("k_split_nibbles_u8");
-        }
-    }
-    if (mode == SIM_F16) {
-        k_f16_max_norms<<<ceil_div(n1 + n2, 8), 256, 0, st>>>(ha, n1, hb, n2, D, maxnorm, wsp<float>(ws, l.off_nrm));
-        PYSIFT_LAUNCH_CHECK("k_f16_max_norms");
+        PYSIFT_LAUNCH_CHECK("k_match_prep");
     }
     int* fbest = fbest_out ? fbest_out : wsp<int>(ws, l.off_fbest);
     int* fpass = fpass_out ? fpass_out : wsp<int>(ws, l.off_fpass);
@@ -1195,43 +1299,29 @@ static int run_match(int mode, const uint8_t* rows_a, int n1, const uint8_t* row
     int* bpass = bpass_out ? bpass_out : wsp<int>(ws, l.off_bpass);
     float* fdist = wsp<float>(ws, l.off_fdist);
     float* bdist = wsp<float>(ws, l.off_bdist);
-    for (int dir = 0; dir < 2; ++dir) {
-        RowScanArgs s;
-        s.q = dir == 0 ? qa : qb;
-        s.t = dir == 0 ? tb : ta;
-        s.n_q = dir == 0 ? n1 : n2;
-        s.n_t = dir == 0 ? n2 : n1;
-        s.norm_t = dir == 0 ? fnb : fna;
-        s.norm_ti = dir == 0 ? nb : na;
-        s.scale_q = dir == 0 ? sa : sb;
-        s.scale_t = dir == 0 ? sb : sa;
-        s.part = wsp<void>(ws, dir == 0 ? l.off_fpart : l.off_bpart);
-        s.error = err;
-        int nseg;
-        scan_split(s.n_q, s.n_t, nseg, s.seg_tiles);
-        const int rc = launch_scan_mode(mode, s, D, nseg, st);
-        if (rc) return rc;
-        int* best = dir == 0 ? fbest : bbest;
-        int* pass = dir == 0 ? fpass : bpass;
-        float* dist = dir == 0 ? fdist : bdist;
-        if (mode == SIM_F16) {
-            k_match_merge_f16<<<ceil_div(s.n_q, 8), 256, 0, st>>>(
-                static_cast<const Top3*>(s.part), s.n_q, nseg, ratio_sq, dir == 0 ? ha : hb, dir == 0 ? hb : ha,
-                s.n_t, D, wsp<float>(ws, l.off_nrm) + (dir == 0 ? 0 : n1), maxnorm + (dir == 0 ? 1 : 0), err, best,
-                pass, dist,
-                wsp<int>(ws, dir == 0 ? l.off_rl0 : l.off_rl1), ctl + 1 + dir);
-            PYSIFT_LAUNCH_CHECK("k_match_merge_f16");
-        } else if (mode == SIM_I8) {
-            k_match_merge_i8<<<ceil_div(s.n_q, 256), 256, 0, st>>>(static_cast<const Top2*>(s.part), s.n_q, nseg,
-                                                                   ratio_sq, best, pass, dist);
-            PYSIFT_LAUNCH_CHECK("k_match_merge_i8");
-        } else {
-            k_match_merge_u8<<<ceil_div(s.n_q, 8), 256, 0, st>>>(
-                static_cast<const Top3*>(s.part), s.n_q, nseg, ratio_sq, dir == 0 ? rows_a : rows_b,
-                dir == 0 ? rows_b : rows_a, s.n_t, D, dir == 0 ? na : nb, dir == 0 ? nb : na, err, best, pass, dist);
-            PYSIFT_LAUNCH_CHECK("k_match_merge_u8");
-        }
-    }
+    RowScanArgs s;
+    s.side[0] = ScanSide{qa, tb, n1, n2, fnb, nb, sa, sb, 1, 1, wsp<void>(ws, l.off_fpart)};
+    s.side[1] = ScanSide{qb, ta, n2, n1, fna, na, sb, sa, 1, 1, wsp<void>(ws, l.off_bpart)};
+    s.error = err;
+    scan_split(s.side);
+    s.blocks0 = ceil_div(n1, MT) * s.side[0].nseg;
+    const int rc = launch_scan_mode(mode, s, D, s.blocks0 + ceil_div(n2, MT) * s.side[1].nseg, st);
+    if (rc) return rc;
+    MergeArgs m;
+    m.side[0] = MergeSide{s.side[0].part, n1, s.side[0].nseg, rows_a, rows_b, n2, na, nb, hna, maxnorm + 1, fbest, fpass,
+                          fdist, wsp<int>(ws, l.off_rl0), ctl + 1};
+    m.side[1] = MergeSide{s.side[1].part, n2, s.side[1].nseg, rows_b, rows_a, n1, nb, na, hna ? hna + n1 : nullptr,
+                          maxnorm, bbest, bpass, bdist, wsp<int>(ws, l.off_rl1), ctl + 2};
+    m.ratio_sq = ratio_sq;
+    m.D = D;
+    m.error = err;
+    const int per = mode == SIM_I8 ? 256 : 8;  // rows of a block: one a thread, or one a warp
+    m.blocks0 = ceil_div(n1, per);
+    const int blocks = m.blocks0 + ceil_div(n2, per);
+    if (mode == SIM_F16) k_match_merge_f16<<<blocks, 256, 0, st>>>(m);
+    else if (mode == SIM_I8) k_match_merge_i8<<<blocks, 256, 0, st>>>(m);
+    else k_match_merge_u8<<<blocks, 256, 0, st>>>(m);
+    PYSIFT_LAUNCH_CHECK("k_match_merge");
     if (mode == SIM_F16) {
         k_match_recheck_f16<<<sm_count(), RECHECK_T, 0, st>>>(wsp<int>(ws, l.off_rl0), wsp<int>(ws, l.off_rl1), ctl + 1,
                                                              ha, n1, hb, n2, D, ratio_sq, fbest, fpass, fdist, bbest,

@@ -44,7 +44,7 @@ def _run(fn, name, d1, d2, ratio, exact, stream=None):
            (("fwd_best", n1), ("fwd_pass", n1), ("bwd_best", n2), ("bwd_pass", n2))}
     pairs = torch.empty((n1, 2), dtype=torch.int32, device=dev)
     dist = torch.empty(n1, dtype=torch.float32, device=dev)
-    count = torch.zeros(1, dtype=torch.int32, device=dev)
+    count = torch.empty(1, dtype=torch.int32, device=dev)
     st = (stream or torch.cuda.current_stream(dev)).cuda_stream
     rc = fn(d1.data_ptr(), n1, d2.data_ptr(), n2, D, float(ratio), wp, wn, out["fwd_best"].data_ptr(),
             out["fwd_pass"].data_ptr(), out["bwd_best"].data_ptr(), out["bwd_pass"].data_ptr(), pairs.data_ptr(),
@@ -109,7 +109,7 @@ def match_i8(q1, s1, q2, s2, ratio=0.75, stream=None):
            (("fwd_best", n1), ("fwd_pass", n1), ("bwd_best", n2), ("bwd_pass", n2))}
     pairs = torch.empty((n1, 2), dtype=torch.int32, device=dev)
     dist = torch.empty(n1, dtype=torch.float32, device=dev)
-    count = torch.zeros(1, dtype=torch.int32, device=dev)
+    count = torch.empty(1, dtype=torch.int32, device=dev)
     st = (stream or torch.cuda.current_stream(dev)).cuda_stream
     rc = lib.pysift_match_i8(q1.data_ptr(), s1.data_ptr(), n1, q2.data_ptr(), s2.data_ptr(), n2, D, float(ratio),
                              wp, wn, out["fwd_best"].data_ptr(), out["fwd_pass"].data_ptr(),
