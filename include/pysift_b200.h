@@ -360,6 +360,10 @@ int pysift_warp_f32_backward(const float* img1, int32_t hs, int32_t ws, int32_t 
                              int32_t iox, int32_t ioy, const float* gout, float* gimg1, float* gimg2, double* ghinv,
                              pysift_stream_t stream);
 
+/* gh8 (8 doubles, device): the gradient of H's first 8 entries, -(Hinv^T G
+ * Hinv^T), from G = dL/dHinv (9 doubles, device) and Hinv (host). */
+int pysift_homography_adjoint(const double* hinv_host, const double* ghinv, double* gh8, pysift_stream_t stream);
+
 /* Reference composition (pysift/core.py:3386-3553, 3686-3714, 3794-3814):
  * gain compensation, seam cost (colour difference + 0.05 |Sobel| of the
  * average gray), dynamic-programming seam along the longer overlap axis,

@@ -297,9 +297,10 @@ class _WarpBlend(torch.autograd.Function):
     @staticmethod
     def forward(ctx, img1, img2, h8, geometry):
         cw, ch, ox, oy, iox, ioy = geometry
-        Hm = _h_from8(h8.detach())
-        Hinv = torch.linalg.inv(Hm)
-        hinv = np.ascontiguousarray(Hinv.cpu().numpy().ravel().astype(np.float64))
+        # a 3x3 inverse on the host: the kernels take it by value, and a
+        # singular homography is refused here
+        Hinv = torch.linalg.inv(_h_from8(h8.detach().cpu()))
+        hinv = np.ascontiguousarray(Hinv.numpy().ravel())
         a = img1.detach().contiguous().float()
         b = img2.detach().contiguous().float()
         C = a.shape[2]
@@ -308,14 +309,14 @@ class _WarpBlend(torch.autograd.Function):
                                                        b.shape[0], b.shape[1], cw, ch,
                                                        hinv.ctypes.data_as(ctypes.c_void_p), ox, oy, iox, ioy,
                                                        out.data_ptr(), _st()), "pysift_warp_f32_forward")
-        ctx.save_for_backward(a, b, Hinv)
+        ctx.save_for_backward(a, b)
         ctx.geometry = geometry
         ctx.hinv = hinv
         return out
 
     @staticmethod
     def backward(ctx, gout):
-        a, b, Hinv = ctx.saved_tensors
+        a, b = ctx.saved_tensors
         cw, ch, ox, oy, iox, ioy = ctx.geometry
         C = a.shape[2]
         g = gout.contiguous().float()
@@ -327,9 +328,9 @@ class _WarpBlend(torch.autograd.Function):
                                                         ctx.hinv.ctypes.data_as(ctypes.c_void_p), ox, oy, iox, ioy,
                                                         g.data_ptr(), ga.data_ptr(), gb.data_ptr(), gh.data_ptr(),
                                                         _st()), "pysift_warp_f32_backward")
-        G = gh.reshape(3, 3)
-        gH = -(Hinv.t() @ G @ Hinv.t())          # d(inv H) adjoint
-        g8 = gH.reshape(-1)[:8]
+        g8 = torch.empty(8, dtype=torch.float64, device=a.device)
+        _lib.check(_lib.load().pysift_homography_adjoint(ctx.hinv.ctypes.data_as(ctypes.c_void_p), gh.data_ptr(),
+                                                         g8.data_ptr(), _st()), "pysift_homography_adjoint")
         return ga, gb, g8, None
 
 
