@@ -52,16 +52,34 @@ __device__ __forceinline__ float expf_(float x) {
     return scale2(p, (int)n);
 }
 
+// expf_ for x in [-87, 0]: the same operations without the range checks, the
+// scale a normal power of two.
+__device__ __forceinline__ float expf_neg_(float x) {
+    const float LOG2E = 1.44269504088896341f;
+    const float LN2_HI = 0.693145751953125f;
+    const float LN2_LO = 1.42860682030941723212e-06f;
+    float n = rintf(x * LOG2E);
+    float r = fmaf(-n, LN2_HI, x);
+    r = fmaf(-n, LN2_LO, r);
+    float p = 2.48015873015873015873e-05f;
+    p = fmaf(p, r, 1.98412698412698412698e-04f);
+    p = fmaf(p, r, 1.38888888888888888889e-03f);
+    p = fmaf(p, r, 8.33333333333333333333e-03f);
+    p = fmaf(p, r, 4.16666666666666666667e-02f);
+    p = fmaf(p, r, 1.66666666666666666667e-01f);
+    p = fmaf(p, r, 0.5f);
+    p = fmaf(p, r, 1.0f);
+    p = fmaf(p, r, 1.0f);
+    return p * __uint_as_float((uint32_t)((int)n + 127) << 23);
+}
+
 constexpr float PI_F = 3.14159265358979323846f;
 constexpr float PIO2_F = 1.57079632679489661923f;
 constexpr float PIO4_F = 0.78539816339744830962f;
 
-__device__ __forceinline__ float atan2f_(float y, float x) {
-    float ax = fabsf(x), ay = fabsf(y);
-    if (ax == 0.0f && ay == 0.0f) {
-        float a = signbit(x) ? PI_F : 0.0f;
-        return signbit(y) ? -a : a;
-    }
+// atan2f_ except at (0, 0), where this is NaN
+__device__ __forceinline__ float atan2f_nonzero_(float y, float x) {
+    const float ax = fabsf(x), ay = fabsf(y);
     const bool swap = ay > ax;
     const float mn = swap ? ax : ay;
     const float mx = swap ? ay : ax;
@@ -82,6 +100,14 @@ __device__ __forceinline__ float atan2f_(float y, float x) {
     if (signbit(x)) a = PI_F - a;
     if (signbit(y)) a = -a;
     return a;
+}
+
+__device__ __forceinline__ float atan2f_(float y, float x) {
+    if (x == 0.0f && y == 0.0f) {
+        const float a = signbit(x) ? PI_F : 0.0f;
+        return signbit(y) ? -a : a;
+    }
+    return atan2f_nonzero_(y, x);
 }
 
 __device__ __forceinline__ void sincosf_(float x, float* s, float* c) {

@@ -91,6 +91,15 @@ def test_wide_image_bit_exact(oracle_lib):
     _compare(out, ref)
 
 
+@pytest.mark.parametrize("H,W,n_scales", [(31, 62, 3), (33, 63, 3), (34, 124, 1), (64, 126, 2), (65, 61, 5), (70, 187, 4)])
+def test_extrema_strip_edges(H, W, n_scales, oracle_lib):
+    """Sides at the edges of the extrema strips (62 columns, 4 to 32 rows) and
+    every level count."""
+    img = synthetic.dense_texture(H, W, seed=H + W, sigma=1.0)
+    sift, out, ref = _run_both(img, oracle_lib, double_image=False, n_scales=n_scales, n_octaves=2)
+    _compare(out, ref)
+
+
 def test_no_doubling(oracle_lib):
     img = synthetic.scene(480, 640, seed=3)
     sift, out, ref = _run_both(img, oracle_lib, double_image=False)
