@@ -5,6 +5,7 @@
 #include <cstdint>
 #include <cstdio>
 #include <string>
+#include <utility>
 
 #include "../../include/pysift_b200.h"
 
@@ -47,10 +48,40 @@ void count_launch();
         }                                                                                  \
     } while (0)
 
+// Programmatic dependent launch: a kernel that begins with chain_begin() may be
+// launched with launch_chained() right after another kernel of its stream;
+// its launch then overlaps the end of the one before, and chain_begin() waits
+// for that one's completion and for its writes.  It also lets the kernel
+// after it be launched.  A no-op in a kernel launched the ordinary way.
+__device__ __forceinline__ void chain_begin() {
+    asm volatile("griddepcontrol.wait;\n\tgriddepcontrol.launch_dependents;" ::: "memory");
+}
+
+// The overlap is worth a launch's latency (about a microsecond); a large
+// grid's waiting blocks would only keep other streams' blocks off the SMs, so
+// it is taken for grids that leave most of the chip free.
+constexpr long long CHAIN_MAX_THREADS = 148 * 1024;
+
+template <typename... P, typename... A>
+inline void launch_chained(void (*kernel)(P...), dim3 grid, int threads, size_t smem, cudaStream_t st, A&&... args) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = grid;
+    cfg.blockDim = dim3(threads);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = st;
+    cudaLaunchAttribute at = {};
+    at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at.val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = &at;
+    cfg.numAttrs = (long long)grid.x * grid.y * grid.z * threads <= CHAIN_MAX_THREADS ? 1 : 0;
+    cudaLaunchKernelEx(&cfg, kernel, std::forward<A>(args)...);  // errors are left to PYSIFT_LAUNCH_CHECK
+}
+
 // One blurred level (detect.cu): in at `step` (1, or 2 to read every second
-// pixel, which copy0, if not null, receives), pitches in floats.
+// pixel, which copy0, if not null, receives), pitches in floats; chained: the
+// stream's last operation is a kernel launch.
 int blur_level(const float* in, long long in_pitch, int step, float* out, int out_pitch, float* copy0, int H, int W,
-               const float* w, int R, cudaStream_t st);
+               const float* w, int R, bool chained, cudaStream_t st);
 
 inline size_t align_up(size_t x, size_t a) { return (x + a - 1) / a * a; }
 __host__ __device__ inline int ceil_div(int a, int b) { return (a + b - 1) / b; }

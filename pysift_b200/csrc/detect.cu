@@ -14,8 +14,8 @@
 //                        integer counts
 //   k_rowscan, k_scatter deterministic compaction in (s, r, c) order, cap per octave
 //   k_refine             Taylor refinement + contrast + edge (pysift/core.py:343-463)
-//   k_refine_compact     valid keypoints in candidate order
-//   k_retry_decide       starvation retry at half threshold (pysift/core.py:2066-2071)
+//   k_refine_compact     valid keypoints in candidate order; decides on the starvation
+//                        retry at half threshold (pysift/core.py:2066-2071)
 //   k_cap                top-cap by response, stable (pysift/core.py:2078-2080)
 //   k_orientation        36-bin histogram, peaks (pysift/core.py:228-333)
 //   k_expand             orientation expansion + (x, y) sort keys (pysift/core.py:1592-1598)
@@ -60,6 +60,7 @@ struct Ctrl {
     int found[PYSIFT_MAX_OCTAVES];
     int ncand[PYSIFT_MAX_OCTAVES];
     int nref[PYSIFT_MAX_OCTAVES];
+    int compact_done;  // octaves of the first pass compacted
     int retried;
     int n_total_ref;
     int n_kept;
@@ -96,7 +97,7 @@ struct Layout {
     size_t off_bkt, off_members;  // bucket ranks: [2 orders][cnt | off | cursor][BR_NB], [2][4 kc] members
     size_t off_xblk;              // k_expand block counts
     size_t off_split;             // k_descriptor: totals and counts of the entries cut into parts
-    size_t zero_bytes;  // row counts and masks, cleared before each pass
+    size_t zero_bytes;  // row counts and masks of a pass; the retry's follow the first pass's
     size_t off_rowcnt_base;
     size_t total;
 };
@@ -154,7 +155,8 @@ static Layout make_layout(const pysift_detect_config* c, int H, int W) {
     const size_t cap = (size_t)c->max_cands_per_octave;
     const size_t kc = (size_t)c->keypoint_cap;
     l.off_ctrl = take(sizeof(Ctrl));
-    // row counts and masks of all octaves are contiguous so one memset clears them
+    // row counts and masks of all octaves, and a second set for the retry, are
+    // contiguous so one memset clears them
     l.off_rowcnt_base = off;
     size_t rc = 0;
     for (int o = 0; o < l.n_oct; ++o) rc += (size_t)l.S * l.H[o];
@@ -166,6 +168,7 @@ static Layout make_layout(const pysift_detect_config* c, int H, int W) {
     }
     for (int o = 0; o < l.n_oct; ++o) l.off_mask[o] = take((size_t)l.S * l.H[o] * l.wpr[o] * sizeof(uint32_t));
     l.zero_bytes = off - l.off_rowcnt_base;
+    take(l.zero_bytes);
     for (int o = 0; o < l.n_oct; ++o) l.off_rowoff[o] = take((size_t)l.S * l.H[o] * sizeof(int));
     l.off_cand = take(cap * l.n_oct * sizeof(int4));
     l.off_rv_valid = take(cap * l.n_oct * sizeof(int));
@@ -306,6 +309,7 @@ __device__ __forceinline__ float u8_to_unit(uint8_t u, int fp16) {
 
 __global__ void k_u8_to_f32(const uint8_t* __restrict__ img, int H, int W, long long pitch, int fp16,
                             float* __restrict__ out, int out_pitch) {
+    chain_begin();
     int c = blockIdx.x * blockDim.x + threadIdx.x;
     int r = blockIdx.y;
     if (c < W) out[(long long)r * out_pitch + c] = u8_to_unit(img[(long long)r * pitch + c], fp16);
@@ -364,6 +368,7 @@ constexpr int PC_TW = 32, PC_RB = 8, PC_TH = 8 * PC_RB;
 __global__ void __launch_bounds__(256) k_prefilter_cols(const uint8_t* __restrict__ img, int H, int W,
                                                         long long pitch, int fp16, double* __restrict__ coef,
                                                         const SplTaps taps) {
+    chain_begin();
     __shared__ double tile[(PC_TH + 2 * SPL_K) * PC_TW];
     const int x0 = blockIdx.x * PC_TW, r0 = blockIdx.y * PC_TH;
     const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
@@ -440,6 +445,7 @@ constexpr int PR_EXT = PR_CW + 2 * SPL_K;
 __device__ __forceinline__ int pr_phys(int e) { return e + (e >> 3); }
 
 __global__ void __launch_bounds__(PR_NT) k_prefilter_rows(double* __restrict__ coef, int W, const SplTaps taps) {
+    chain_begin();
     // a strip that ends past the chunk reads up to 7 positions beyond the
     // window (values that feed no stored output), so the array covers them
     __shared__ double ext[PR_EXT + 7 + (PR_EXT + 7) / 8 + 1];
@@ -513,6 +519,7 @@ __device__ __forceinline__ double zoom_term_sum(const double (*win)[ZI_CC], cons
 
 __global__ void __launch_bounds__(256) k_zoom_interp(const double* __restrict__ coef, int H, int W, int fp16,
                                                      float* __restrict__ out, int out_pitch) {
+    chain_begin();
     __shared__ int rvalid[ZI_TH], ridx[4][ZI_TH];
     __shared__ double rw[4][ZI_TH];
     __shared__ int cvalid[ZI_TW], cidx[4][ZI_TW];
@@ -663,10 +670,10 @@ static int launch_zoom2x(const uint8_t* gray, int H, int W, long long pitch, int
     k_prefilter_cols<<<dim3(ceil_div(W, PC_TW), ceil_div(H, PC_TH)), 256, 0, st>>>(gray, H, W, pitch, fp16, coef,
                                                                                   taps);
     PYSIFT_LAUNCH_CHECK("k_prefilter_cols");
-    k_prefilter_rows<<<H, PR_NT, 0, st>>>(coef, W, taps);
+    launch_chained(k_prefilter_rows, dim3(H), PR_NT, 0, st, coef, W, taps);
     PYSIFT_LAUNCH_CHECK("k_prefilter_rows");
-    k_zoom_interp<<<dim3(ceil_div(2 * W + 1, ZI_TW), ceil_div(2 * H + 1, ZI_TH)), 256, 0, st>>>(coef, H, W, fp16,
-                                                                                               out, out_pitch);
+    launch_chained(k_zoom_interp, dim3(ceil_div(2 * W + 1, ZI_TW), ceil_div(2 * H + 1, ZI_TH)), 256, 0, st,
+                   (const double*)coef, H, W, fp16, out, out_pitch);
     PYSIFT_LAUNCH_CHECK("k_zoom_interp");
     return PYSIFT_OK;
 }
@@ -1036,6 +1043,7 @@ __host__ __device__ constexpr size_t blur_smem_bytes_rt() {
 
 template <int R, int TH>
 __global__ void __launch_bounds__(BLUR_NT, TH == 40 ? 7 : 1) k_blur(const BlurArgs a) {
+    chain_begin();
     extern __shared__ __align__(16) float smem[];
     const TileIO io{a.in, a.in_pitch, a.step, a.out, a.out_r, a.copy0, a.copy0_r, a.out_pitch, a.H, a.W};
     auto w = [&](int k) { return a.w2[k]; };
@@ -1047,6 +1055,7 @@ __global__ void __launch_bounds__(BLUR_NT, TH == 40 ? 7 : 1) k_blur(const BlurAr
 
 // Any radius up to PYSIFT_MAX_RADIUS (no register blocking); radius 0 copies.
 __global__ void __launch_bounds__(BLUR_NT) k_blur_generic(const BlurArgs a, int R) {
+    chain_begin();
     const int RA = (R + 3) / 4 * 4;
     const int TWP = BLUR_TW + 2 * RA, ROWS = BLUR_TH + 2 * R;
     extern __shared__ float smem[];
@@ -1210,7 +1219,7 @@ static int ensure_blur_attrs() {
     return PYSIFT_OK;
 }
 
-static int launch_blur(BlurArgs& a, int R, const float* w, cudaStream_t st) {
+static int launch_blur(BlurArgs& a, int R, const float* w, bool chained, cudaStream_t st) {
     for (int k = 0; k <= 2 * R; ++k) a.w[k] = w[k];
     for (int k = 0; k <= 2 * R && k <= 2 * BLUR_PAIR_MAX_R; ++k) {
         unsigned u = 0;
@@ -1221,7 +1230,8 @@ static int launch_blur(BlurArgs& a, int R, const float* w, cudaStream_t st) {
         const int v = blur_pick(R, a.H, a.W);
         const BlurVariant bv = blur_variant(R, v);
         dim3 grid(ceil_div(a.W, BLUR_TW), ceil_div(a.H, BLUR_THS[v]));
-        bv.fn<<<grid, BLUR_NT, bv.smem, st>>>(a);
+        if (chained) launch_chained(bv.fn, grid, BLUR_NT, bv.smem, st, a);
+        else bv.fn<<<grid, BLUR_NT, bv.smem, st>>>(a);
         PYSIFT_LAUNCH_CHECK("k_blur");
     } else {
         dim3 grid(ceil_div(a.W, BLUR_TW), ceil_div(a.H, BLUR_TH));
@@ -1234,7 +1244,7 @@ static int launch_blur(BlurArgs& a, int R, const float* w, cudaStream_t st) {
 }
 
 int blur_level(const float* in, long long in_pitch, int step, float* out, int out_pitch, float* copy0, int H, int W,
-               const float* w, int R, cudaStream_t st) {
+               const float* w, int R, bool chained, cudaStream_t st) {
     static thread_local BlurArgs a;  // large (weights by value); not on the stack
     memset(&a, 0, sizeof(a));
     a.in = in;
@@ -1245,7 +1255,7 @@ int blur_level(const float* in, long long in_pitch, int step, float* out, int ou
     a.copy0 = copy0;
     a.H = H;
     a.W = W;
-    return launch_blur(a, R, w, st);
+    return launch_blur(a, R, w, chained, st);
 }
 
 // ---------------------------------------------------------------------------
@@ -1305,15 +1315,13 @@ __device__ __forceinline__ float min3(float a, float b, float c) {
 constexpr int EX_T = 128, EX_COLS = 62;
 
 template <int NL>
-__global__ void __launch_bounds__(EX_T, 8) k_extrema_mask(const __grid_constant__ ExtArgs a, Ctrl* ctrl) {
+__device__ __forceinline__ void extrema_strips(const ExtArgs& a, int block, float thr) {
     constexpr int S = NL - 3, ND = NL - 1;
-    if (a.retry_mode && !ctrl->retried) return;
-    const float thr = ctrl->thr[a.thr_idx];
-    const int o = find_octave(a.blk_off, a.n_oct, blockIdx.x);
+    const int o = find_octave(a.blk_off, a.n_oct, block);
     const OctView& v = a.oct[o];
     const int H = v.H, W = v.W, B = a.border, wpr = a.wpr[o];
     const int lane = threadIdx.x & 31;
-    const int unit = (blockIdx.x - a.blk_off[o]) * (EX_T / 32) + (threadIdx.x >> 5);
+    const int unit = (block - a.blk_off[o]) * (EX_T / 32) + (threadIdx.x >> 5);
     const int ncx = ceil_div(W, EX_COLS);
     const int ry = unit / ncx, r0 = ry * a.rows;
     if (r0 >= H) return;
@@ -1386,6 +1394,14 @@ __global__ void __launch_bounds__(EX_T, 8) k_extrema_mask(const __grid_constant_
     }
 }
 
+template <int NL>
+__global__ void __launch_bounds__(EX_T, 8) k_extrema_mask(const __grid_constant__ ExtArgs a, Ctrl* ctrl) {
+    chain_begin();
+    if (a.retry_mode && !ctrl->retried) return;
+    const float thr = ctrl->thr[a.thr_idx];
+    for (int b = blockIdx.x; b < a.blk_off[a.n_oct]; b += gridDim.x) extrema_strips<NL>(a, b, thr);
+}
+
 typedef void (*ExtremaKernel)(const ExtArgs, Ctrl*);
 
 static ExtremaKernel extrema_kernel(int S) {
@@ -1401,6 +1417,7 @@ static ExtremaKernel extrema_kernel(int S) {
 static_assert(PYSIFT_MAX_LEVELS == 8, "extrema_kernel covers n_scales 1..5");
 
 __global__ void __launch_bounds__(1024) k_rowscan(const ExtArgs a, Ctrl* ctrl) {
+    chain_begin();
     if (a.retry_mode && !ctrl->retried) return;
     __shared__ int sh[33];
     const int o = blockIdx.x;
@@ -1424,29 +1441,31 @@ __global__ void __launch_bounds__(1024) k_rowscan(const ExtArgs a, Ctrl* ctrl) {
 }
 
 __global__ void __launch_bounds__(256) k_scatter(const ExtArgs a, Ctrl* ctrl) {
+    chain_begin();
     if (a.retry_mode && !ctrl->retried) return;
-    const int o = find_octave(a.blk_off, a.n_oct, blockIdx.x);
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int H = a.oct[o].H;
-    const int unit = (blockIdx.x - a.blk_off[o]) * 8 + warp;  // (s-1)*H + r
-    if (unit >= a.S * H) return;
-    if (a.rowcnt[o][unit] == 0) return;
-    const int s = unit / H + 1, r = unit - (s - 1) * H;
-    const int wpr = a.wpr[o];
-    int base = a.rowoff[o][unit];
-    const uint32_t* mrow = a.mask[o] + (long long)unit * wpr;
-    int4* out = a.cand + (long long)o * a.cap;
-    for (int w0 = 0; w0 < wpr; w0 += 32) {
-        uint32_t word = (w0 + lane < wpr) ? mrow[w0 + lane] : 0u;
-        int tot;
-        int pos = base + warp_excl_scan(__popc(word), &tot);
-        while (word) {
-            int b = __ffs(word) - 1;
-            word &= word - 1;
-            if (pos < a.cap) out[pos] = make_int4(s, r, (w0 + lane) * 32 + b, 0);
-            ++pos;
+    for (int b = blockIdx.x; b < a.blk_off[a.n_oct]; b += gridDim.x) {
+        const int o = find_octave(a.blk_off, a.n_oct, b);
+        const int H = a.oct[o].H;
+        const int unit = (b - a.blk_off[o]) * 8 + warp;  // (s-1)*H + r
+        if (unit >= a.S * H || a.rowcnt[o][unit] == 0) continue;
+        const int s = unit / H + 1, r = unit - (s - 1) * H;
+        const int wpr = a.wpr[o];
+        int base = a.rowoff[o][unit];
+        const uint32_t* mrow = a.mask[o] + (long long)unit * wpr;
+        int4* out = a.cand + (long long)o * a.cap;
+        for (int w0 = 0; w0 < wpr; w0 += 32) {
+            uint32_t word = (w0 + lane < wpr) ? mrow[w0 + lane] : 0u;
+            int tot;
+            int pos = base + warp_excl_scan(__popc(word), &tot);
+            while (word) {
+                int bit = __ffs(word) - 1;
+                word &= word - 1;
+                if (pos < a.cap) out[pos] = make_int4(s, r, (w0 + lane) * 32 + bit, 0);
+                ++pos;
+            }
+            base += tot;
         }
-        base += tot;
     }
 }
 
@@ -1455,7 +1474,7 @@ __global__ void __launch_bounds__(256) k_scatter(const ExtArgs a, Ctrl* ctrl) {
 // ---------------------------------------------------------------------------
 struct RefArgs {
     OctView oct[PYSIFT_MAX_OCTAVES];
-    int n_oct, S, border, cap, thr_idx, retry_mode;
+    int n_oct, S, border, cap, thr_idx, retry_mode, starvation_min;
     float edge_score;
     const int4* cand;
     int* rv_valid;
@@ -1470,6 +1489,7 @@ struct RefArgs {
 };
 
 __global__ void __launch_bounds__(256) k_refine(const RefArgs a, Ctrl* ctrl) {
+    chain_begin();
     if (a.retry_mode && !ctrl->retried) return;
     const float cthr = ctrl->thr[a.thr_idx];
     const long long nslots = (long long)a.n_oct * a.cap;
@@ -1557,6 +1577,7 @@ struct RefinedRow {
     int si, valid;
 };
 __global__ void __launch_bounds__(1024) k_refine_compact(const RefArgs a, Ctrl* ctrl) {
+    chain_begin();
     if (a.retry_mode && !ctrl->retried) return;
     __shared__ int sh[33];
     const int o = blockIdx.x;
@@ -1581,13 +1602,19 @@ __global__ void __launch_bounds__(1024) k_refine_compact(const RefArgs a, Ctrl* 
             a.rf_resp[base + pos] = r.resp;
         },
         sh);
-    if (threadIdx.x == 0) ctrl->nref[o] = total;
-}
-
-__global__ void k_retry_decide(Ctrl* ctrl, int n_oct, int starvation_min) {
-    int t = 0;
-    for (int o = 0; o < n_oct; ++o) t += ctrl->nref[o];
-    ctrl->retried = (t < starvation_min) ? 1 : 0;
+    if (threadIdx.x == 0) {
+        ctrl->nref[o] = total;
+        if (a.retry_mode) return;
+        // the last octave of the first pass decides on the starvation retry
+        // (pysift/core.py:2066-2071)
+        __threadfence();
+        if (atomicAdd(&ctrl->compact_done, 1) == a.n_oct - 1) {
+            __threadfence();
+            int t = 0;
+            for (int k = 0; k < a.n_oct; ++k) t += __ldcg(&ctrl->nref[k]);
+            ctrl->retried = t < a.starvation_min ? 1 : 0;
+        }
+    }
 }
 
 // ---------------------------------------------------------------------------
@@ -1621,6 +1648,7 @@ constexpr int CAP_T = 1024;
 constexpr size_t CAP_SMEM_BYTES = (size_t)(32 * 256 + CAP_SMEM_KEYS) * sizeof(unsigned int);
 
 __global__ void __launch_bounds__(CAP_T) k_cap(const CapArgs a, Ctrl* ctrl) {
+    chain_begin();
     extern __shared__ unsigned int cap_smem[];
     unsigned int* whist = cap_smem;              // [32 warps][256] private digit histograms
     unsigned int* s_keys = cap_smem + 32 * 256;  // staged keys
@@ -2020,6 +2048,7 @@ __device__ __forceinline__ void orientation_groups(const OriArgs& a, Ctrl* ctrl,
 }
 
 __global__ void __launch_bounds__(ORI_T) k_orientation(const __grid_constant__ OriArgs a, Ctrl* ctrl) {
+    chain_begin();
     __shared__ OriShared sh;
     const int n = ctrl->n_kept;
     if (n <= (int)gridDim.x * 2) orientation_groups<256>(a, ctrl, n, sh);
@@ -2072,6 +2101,7 @@ constexpr int EXP_T = 256;
 constexpr int EXP_PER_BLOCK = EXP_T * EXP_K;
 
 __global__ void __launch_bounds__(EXP_T) k_expand_count(const ExpArgs a, const Ctrl* ctrl) {
+    chain_begin();
     __shared__ int sh[33];
     const int n = ctrl->n_kept;
     const int i0 = blockIdx.x * EXP_PER_BLOCK + (int)threadIdx.x * EXP_K;
@@ -2085,6 +2115,7 @@ __global__ void __launch_bounds__(EXP_T) k_expand_count(const ExpArgs a, const C
 }
 
 __global__ void __launch_bounds__(EXP_T) k_expand(const ExpArgs a, Ctrl* ctrl) {
+    chain_begin();
     __shared__ int sh[33];
     __shared__ int s_base;
     const int n = ctrl->n_kept;
@@ -2172,6 +2203,7 @@ __device__ __forceinline__ int br_bucket(const BRArgs& a, int i) {
 
 template <int ORD>
 __global__ void __launch_bounds__(1024) k_br_scan(const BRArgs a, const Ctrl* ctrl) {
+    chain_begin();
     __shared__ int sh[33];
     if (br_skip<ORD>(a, ctrl->n_oriented)) return;
     constexpr int PER = BR_NB / 1024;
@@ -2193,6 +2225,7 @@ __global__ void __launch_bounds__(1024) k_br_scan(const BRArgs a, const Ctrl* ct
 
 template <int ORD>
 __global__ void k_br_scatter(const BRArgs a, const Ctrl* ctrl) {
+    chain_begin();
     const int n = ctrl->n_oriented;
     if (br_skip<ORD>(a, n)) return;
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x)
@@ -2201,6 +2234,7 @@ __global__ void k_br_scatter(const BRArgs a, const Ctrl* ctrl) {
 
 template <int ORD>
 __global__ void k_br_rank(const BRArgs a, const Ctrl* ctrl) {
+    chain_begin();
     const int n = ctrl->n_oriented;
     if (br_skip<ORD>(a, n)) return;
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
@@ -2250,6 +2284,8 @@ struct DescArgs {
     float* out_resp;
     int* out_oct;
     float* out_desc;
+    int n_oct, doubled;  // for the counters
+    int32_t* stats;
 };
 
 constexpr int DESC_T = 256;
@@ -2413,6 +2449,27 @@ __device__ __forceinline__ float bins_sum(float x, float* part) {
     return s;
 }
 
+// The run's counters (one thread).
+__device__ void write_stats(const Ctrl* ctrl, int32_t* stats, int n_oct, int doubled, int limit) {
+    for (int t = 0; t < PYSIFT_STAT_COUNT; ++t) stats[t] = 0;
+    {
+        int nref = 0;
+        for (int o = 0; o < n_oct; ++o) nref += ctrl->nref[o];
+        stats[PYSIFT_STAT_N_KEYPOINTS] = (limit > 0 && ctrl->n_oriented > limit) ? limit : ctrl->n_oriented;
+        stats[PYSIFT_STAT_N_REFINED] = nref;
+        stats[PYSIFT_STAT_N_KEPT] = ctrl->n_kept;
+        stats[PYSIFT_STAT_RETRIED] = ctrl->retried;
+        stats[PYSIFT_STAT_CAPPED] = ctrl->capped;
+        stats[PYSIFT_STAT_DOUBLED] = doubled;
+        stats[PYSIFT_STAT_CAND_OVERFLOW] = ctrl->overflow_octs;
+        for (int o = 0; o < n_oct; ++o) {
+            stats[PYSIFT_STAT_CANDS + o] = ctrl->found[o];
+            stats[PYSIFT_STAT_REFINED_OCT + o] = ctrl->nref[o];
+        }
+        stats[PYSIFT_STAT_THRESH_BITS] = (int32_t)__float_as_uint(ctrl->thr[ctrl->retried ? 1 : 0]);
+    }
+}
+
 // One DESC_T-thread block per oriented keypoint at a time; a block takes its
 // next entry from a counter (entries differ in patch size, so blocks stay
 // busy until the list is done; every entry writes its own output row).
@@ -2434,6 +2491,7 @@ constexpr int DESC_UNITS_DSP = 6, DESC_UNITS = 1;
 constexpr int DESC_SPLIT_MAX = 148 * DESC_OCC * DESC_UNITS_DSP / 2;  // entries that can be cut (two parts at least)
 
 __global__ void __launch_bounds__(DESC_T, DESC_OCC) k_descriptor(const DescArgs a, Ctrl* ctrl) {
+    chain_begin();
     __shared__ unsigned int wh32[DESC_W][128];
     __shared__ unsigned long long whist[DESC_W][128];
     __shared__ float part_sum[4];
@@ -2441,6 +2499,7 @@ __global__ void __launch_bounds__(DESC_T, DESC_OCC) k_descriptor(const DescArgs 
     __shared__ int s_last;
     const int tid = threadIdx.x, warp = tid >> 5;
     const int n = ctrl->n_oriented;
+    if (blockIdx.x == gridDim.x - 1 && tid == DESC_T - 1) write_stats(ctrl, a.stats, a.n_oct, a.doubled, a.limit);
     const int parts =
         n > DESC_SPLIT_MAX || n == 0
             ? 1
@@ -2534,33 +2593,12 @@ __global__ void __launch_bounds__(DESC_T, DESC_OCC) k_descriptor(const DescArgs 
 __global__ void k_row_resp(const int* __restrict__ ent_kp, const float* __restrict__ kp_resp,
                            const int* __restrict__ rank, float* __restrict__ row_resp, int* __restrict__ resp_cnt,
                            const Ctrl* ctrl) {
+    chain_begin();
     const int n = ctrl->n_oriented;
     for (int e = blockIdx.x * blockDim.x + threadIdx.x; e < n; e += gridDim.x * blockDim.x) {
         const float r = kp_resp[ent_kp[e]];
         row_resp[rank[e]] = r;
         atomicAdd(&resp_cnt[br_bucket_resp(r)], 1);
-    }
-}
-
-__global__ void k_finalize(const Ctrl* ctrl, int32_t* stats, int n_oct, int doubled, int limit) {
-    int t = threadIdx.x;
-    if (t < PYSIFT_STAT_COUNT) stats[t] = 0;
-    __syncthreads();
-    if (t == 0) {
-        int nref = 0;
-        for (int o = 0; o < n_oct; ++o) nref += ctrl->nref[o];
-        stats[PYSIFT_STAT_N_KEYPOINTS] = (limit > 0 && ctrl->n_oriented > limit) ? limit : ctrl->n_oriented;
-        stats[PYSIFT_STAT_N_REFINED] = nref;
-        stats[PYSIFT_STAT_N_KEPT] = ctrl->n_kept;
-        stats[PYSIFT_STAT_RETRIED] = ctrl->retried;
-        stats[PYSIFT_STAT_CAPPED] = ctrl->capped;
-        stats[PYSIFT_STAT_DOUBLED] = doubled;
-        stats[PYSIFT_STAT_CAND_OVERFLOW] = ctrl->overflow_octs;
-        for (int o = 0; o < n_oct; ++o) {
-            stats[PYSIFT_STAT_CANDS + o] = ctrl->found[o];
-            stats[PYSIFT_STAT_REFINED_OCT + o] = ctrl->nref[o];
-        }
-        stats[PYSIFT_STAT_THRESH_BITS] = (int32_t)__float_as_uint(ctrl->thr[ctrl->retried ? 1 : 0]);
     }
 }
 
@@ -2671,8 +2709,11 @@ static int run_detect(const pysift_detect_config* cfg, const uint8_t* gray, int 
         PYSIFT_CUDA_TRY(cudaEventRecord(sp->ev[0], st));
         PYSIFT_CUDA_TRY(cudaStreamWaitEvent(side, sp->ev[0], 0));
     }
-    // (side stream) the descriptor's split totals; A1, read by the extrema test after the join
+    // (side stream, read after the join) what later kernels count in; A1, the threshold of the extrema test
     PYSIFT_CUDA_TRY(cudaMemsetAsync(at<char>(ws, l.off_split), 0, split_bytes(kcap), side));
+    int* bkt = at<int>(ws, l.off_bkt);  // [order][cnt | off | cursor][BR_NB]
+    PYSIFT_CUDA_TRY(cudaMemsetAsync(bkt, 0, sizeof(int) * 2 * 3 * BR_NB, side));
+    PYSIFT_CUDA_TRY(cudaMemsetAsync(at<char>(ws, l.off_rowcnt_base), 0, 2 * l.zero_bytes, side));
     {
         const int blocks = std::max(1, std::min(ceil_div(H, 8), num_sms() * 2));
         k_histogram<<<blocks, 256, 0, side>>>(gray, H, W, pitch, ctrl, cfg->contrast_thresh, S);
@@ -2709,7 +2750,7 @@ static int run_detect(const pysift_detect_config* cfg, const uint8_t* gray, int 
                 a.step = 1;
                 a.out = pyr;
                 a.out_r = pyr_r;
-                int rc = launch_blur(a, cfg->blur_radius[k], cfg->blur_weights[k], st);
+                int rc = launch_blur(a, cfg->blur_radius[k], cfg->blur_weights[k], true, st);
                 if (rc) return rc;
             }
             for (int s = 0; s < S + 2; ++s) {
@@ -2740,7 +2781,7 @@ static int run_detect(const pysift_detect_config* cfg, const uint8_t* gray, int 
                 }
                 a.out = pyr + (size_t)(s + 1) * lev;
                 a.out_r = pyr_r ? pyr_r + (size_t)(s + 1) * lev : nullptr;
-                int rc = launch_blur(a, cfg->blur_radius[2 + s], cfg->blur_weights[2 + s], ls);
+                int rc = launch_blur(a, cfg->blur_radius[2 + s], cfg->blur_weights[2 + s], s != S || !sp, ls);
                 if (rc) return rc;
             }
         }
@@ -2773,6 +2814,7 @@ static int run_detect(const pysift_detect_config* cfg, const uint8_t* gray, int 
         for (int o = 0; o < n_oct; ++o) n += (long long)ceil_div(l.H[o], rows) * ceil_div(l.W[o], EX_COLS);
         return n;
     };
+    const int retry_blocks = num_sms() * 8;
     ea.rows = 32;
     while (ea.rows > 4 && strips(ea.rows) < 40LL * num_sms()) ea.rows /= 2;
     for (int o = 0; o < n_oct; ++o) {
@@ -2780,14 +2822,13 @@ static int run_detect(const pysift_detect_config* cfg, const uint8_t* gray, int 
         mask_blocks += ceil_div(ceil_div(l.H[o], ea.rows) * ceil_div(l.W[o], EX_COLS), EX_T / 32);
         row_off[o] = row_blocks;
         row_blocks += ceil_div(S * l.H[o], 8);
-        ea.mask[o] = at<uint32_t>(ws, l.off_mask[o]);
-        ea.rowcnt[o] = at<int>(ws, l.off_rowcnt[o]);
         ea.rowoff[o] = at<int>(ws, l.off_rowoff[o]);
         ea.wpr[o] = l.wpr[o];
     }
     ea.blk_off[n_oct] = mask_blocks;
     row_off[n_oct] = row_blocks;
     ra.edge_score = cfg->edge_score;
+    ra.starvation_min = cfg->starvation_min;
     ra.rv_valid = at<int>(ws, l.off_rv_valid);
     ra.rv_ri = at<float>(ws, l.off_rv_ri);
     ra.rv_ci = at<float>(ws, l.off_rv_ci);
@@ -2801,29 +2842,30 @@ static int run_detect(const pysift_detect_config* cfg, const uint8_t* gray, int 
     for (int pass = 0; pass < 2; ++pass) {
         ea.thr_idx = ra.thr_idx = pass;
         ea.retry_mode = ra.retry_mode = pass;
-        // row counts and masks
-        PYSIFT_CUDA_TRY(cudaMemsetAsync(at<char>(ws, l.off_rowcnt_base), 0, l.zero_bytes, st));
-        extrema_kernel(S)<<<mask_blocks, EX_T, 0, st>>>(ea, ctrl);
+        for (int o = 0; o < n_oct; ++o) {
+            ea.mask[o] = at<uint32_t>(ws, l.off_mask[o] + pass * l.zero_bytes);
+            ea.rowcnt[o] = at<int>(ws, l.off_rowcnt[o] + pass * l.zero_bytes);
+        }
+        // the retry's grid is small (its kernels loop), so that finding nothing
+        // to do is cheap
+        if (pass == 0) extrema_kernel(S)<<<mask_blocks, EX_T, 0, st>>>(ea, ctrl);
+        else launch_chained(extrema_kernel(S), dim3(std::min(mask_blocks, retry_blocks)), EX_T, 0, st, ea, ctrl);
         PYSIFT_LAUNCH_CHECK("k_extrema_mask");
         if (pass == 0) PYSIFT_STAGE(3);
-        k_rowscan<<<n_oct, 1024, 0, st>>>(ea, ctrl);
+        launch_chained(k_rowscan, dim3(n_oct), 1024, 0, st, ea, ctrl);
         PYSIFT_LAUNCH_CHECK("k_rowscan");
         // k_scatter indexes blocks by (s, r) rows: reuse blk_off for its own table
         ExtArgs& sa = ea;
         int saved[PYSIFT_MAX_OCTAVES + 1];
         memcpy(saved, sa.blk_off, sizeof(saved));
         memcpy(sa.blk_off, row_off, sizeof(row_off));
-        k_scatter<<<row_blocks, 256, 0, st>>>(sa, ctrl);
+        launch_chained(k_scatter, dim3(pass == 0 ? row_blocks : std::min(row_blocks, retry_blocks)), 256, 0, st, sa, ctrl);
         PYSIFT_LAUNCH_CHECK("k_scatter");
         memcpy(sa.blk_off, saved, sizeof(saved));
-        k_refine<<<refine_blocks, 256, 0, st>>>(ra, ctrl);
+        launch_chained(k_refine, dim3(refine_blocks), 256, 0, st, ra, ctrl);
         PYSIFT_LAUNCH_CHECK("k_refine");
-        k_refine_compact<<<n_oct, 1024, 0, st>>>(ra, ctrl);
+        launch_chained(k_refine_compact, dim3(n_oct), 1024, 0, st, ra, ctrl);
         PYSIFT_LAUNCH_CHECK("k_refine_compact");
-        if (pass == 0) {
-            k_retry_decide<<<1, 1, 0, st>>>(ctrl, n_oct, cfg->starvation_min);
-            PYSIFT_LAUNCH_CHECK("k_retry_decide");
-        }
     }
     // A9
     CapArgs ca;
@@ -2843,7 +2885,7 @@ static int run_detect(const pysift_detect_config* cfg, const uint8_t* gray, int 
     {
         PYSIFT_CUDA_TRY(
             cudaFuncSetAttribute(k_cap, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)CAP_SMEM_BYTES));
-        k_cap<<<1, CAP_T, CAP_SMEM_BYTES, st>>>(ca, ctrl);
+        launch_chained(k_cap, dim3(1), CAP_T, CAP_SMEM_BYTES, st, ca, ctrl);
     }
     PYSIFT_LAUNCH_CHECK("k_cap");
     PYSIFT_STAGE(4);
@@ -2858,7 +2900,7 @@ static int run_detect(const pysift_detect_config* cfg, const uint8_t* gray, int 
     oa.kp_ci = ca.kp_ci;
     oa.ang = at<float>(ws, l.off_ang);
     oa.angcnt = at<int>(ws, l.off_angcnt);
-    k_orientation<<<std::min(kcap, num_sms() * 5), ORI_T, 0, st>>>(oa, ctrl);
+    launch_chained(k_orientation, dim3(std::min(kcap, num_sms() * 5)), ORI_T, 0, st, oa, ctrl);
     PYSIFT_LAUNCH_CHECK("k_orientation");
     // expansion + keys + rank
     ExpArgs xa;
@@ -2873,17 +2915,16 @@ static int run_detect(const pysift_detect_config* cfg, const uint8_t* gray, int 
     xa.ent_slot = at<int>(ws, l.off_ent_slot);
     xa.keys = at<uint4>(ws, l.off_keys);
     for (int o = 0; o < n_oct; ++o) xa.coord_scale[o] = (float)((double)(1 << o) * (l.doubled ? 0.5 : 1.0));
-    int* bkt = at<int>(ws, l.off_bkt);  // [order][cnt | off | cursor][BR_NB]
-    PYSIFT_CUDA_TRY(cudaMemsetAsync(bkt, 0, sizeof(int) * 2 * 3 * BR_NB, st));
     xa.xy_cnt = bkt;
     xa.xy_bscale = (float)BR_NB / (float)W;
     xa.blk_cnt = at<int>(ws, l.off_xblk);
     const int exp_blocks = ceil_div(kcap, EXP_PER_BLOCK);
-    k_expand_count<<<exp_blocks, EXP_T, 0, st>>>(xa, ctrl);
-    k_expand<<<exp_blocks, EXP_T, 0, st>>>(xa, ctrl);
+    launch_chained(k_expand_count, dim3(exp_blocks), EXP_T, 0, st, xa, ctrl);
+    PYSIFT_LAUNCH_CHECK("k_expand_count");
+    launch_chained(k_expand, dim3(exp_blocks), EXP_T, 0, st, xa, ctrl);
     PYSIFT_LAUNCH_CHECK("k_expand");
     int* rank = at<int>(ws, l.off_rank);
-    const int br_blocks = std::max(1, std::min(ceil_div(4 * kcap, 256), num_sms() * 4));
+    const int br_blocks = std::max(1, std::min(ceil_div(4 * kcap, 128), num_sms() * 4));
     BRArgs bx{};
     bx.keys = xa.keys;
     bx.xy_bscale = xa.xy_bscale;
@@ -2892,10 +2933,13 @@ static int run_detect(const pysift_detect_config* cfg, const uint8_t* gray, int 
     bx.cursor = bkt + 2 * BR_NB;
     bx.members = at<int>(ws, l.off_members);
     bx.rank = rank;
-    k_br_scan<0><<<1, 1024, 0, st>>>(bx, ctrl);
-    k_br_scatter<0><<<br_blocks, 256, 0, st>>>(bx, ctrl);
-    k_br_rank<0><<<br_blocks, 256, 0, st>>>(bx, ctrl);
-    PYSIFT_LAUNCH_CHECK("k_br (x, y)");
+    const int br_threads = 128;
+    launch_chained(k_br_scan<0>, dim3(1), 1024, 0, st, bx, ctrl);
+    PYSIFT_LAUNCH_CHECK("k_br_scan");
+    launch_chained(k_br_scatter<0>, dim3(br_blocks), br_threads, 0, st, bx, ctrl);
+    PYSIFT_LAUNCH_CHECK("k_br_scatter");
+    launch_chained(k_br_rank<0>, dim3(br_blocks), br_threads, 0, st, bx, ctrl);
+    PYSIFT_LAUNCH_CHECK("k_br_rank");
     PYSIFT_STAGE(5);
     // A11
     static thread_local DescArgs da;
@@ -2932,21 +2976,25 @@ static int run_detect(const pysift_detect_config* cfg, const uint8_t* gray, int 
         br.cursor = bkt + 5 * BR_NB;
         br.members = at<int>(ws, l.off_members) + 4 * (size_t)kcap;
         br.rank = at<int>(ws, l.off_lrank);
-        k_row_resp<<<br_blocks, 256, 0, st>>>(xa.ent_kp, ca.kp_resp, rank, row_resp, br.cnt, ctrl);
+        launch_chained(k_row_resp, dim3(br_blocks), br_threads, 0, st, (const int*)xa.ent_kp, (const float*)ca.kp_resp,
+                       (const int*)rank, row_resp, br.cnt, ctrl);
         PYSIFT_LAUNCH_CHECK("k_row_resp");
-        k_br_scan<1><<<1, 1024, 0, st>>>(br, ctrl);
-        k_br_scatter<1><<<br_blocks, 256, 0, st>>>(br, ctrl);
-        k_br_rank<1><<<br_blocks, 256, 0, st>>>(br, ctrl);
-        PYSIFT_LAUNCH_CHECK("k_br (response)");
+        launch_chained(k_br_scan<1>, dim3(1), 1024, 0, st, br, ctrl);
+        PYSIFT_LAUNCH_CHECK("k_br_scan");
+        launch_chained(k_br_scatter<1>, dim3(br_blocks), br_threads, 0, st, br, ctrl);
+        PYSIFT_LAUNCH_CHECK("k_br_scatter");
+        launch_chained(k_br_rank<1>, dim3(br_blocks), br_threads, 0, st, br, ctrl);
+        PYSIFT_LAUNCH_CHECK("k_br_rank");
     }
     da.out_kpts = kpts;
     da.out_resp = resp;
     da.out_oct = octv;
     da.out_desc = desc;
-    k_descriptor<<<std::min(4 * kcap, num_sms() * DESC_OCC), DESC_T, 0, st>>>(da, ctrl);
+    da.n_oct = n_oct;
+    da.doubled = l.doubled ? 1 : 0;
+    da.stats = stats;
+    launch_chained(k_descriptor, dim3(std::min(4 * kcap, num_sms() * DESC_OCC)), DESC_T, 0, st, da, ctrl);
     PYSIFT_LAUNCH_CHECK("k_descriptor");
-    k_finalize<<<1, 32, 0, st>>>(ctrl, stats, n_oct, l.doubled ? 1 : 0, cfg->output_limit);
-    PYSIFT_LAUNCH_CHECK("k_finalize");
     PYSIFT_STAGE(6);
     return PYSIFT_OK;
 }
@@ -3039,7 +3087,7 @@ int pysift_gauss_blur(const float* in, int32_t in_pitch, float* out, int32_t out
     PYSIFT_CHECK_ARG(H > 0 && W > 0 && in_pitch >= W && out_pitch >= W, "bad sizes");
     PYSIFT_CHECK_ARG(radius >= 0 && radius <= PYSIFT_MAX_RADIUS, "radius %d outside 0..%d", radius,
                      PYSIFT_MAX_RADIUS);
-    return blur_level(in, in_pitch, 1, out, out_pitch, nullptr, H, W, weights, radius,
+    return blur_level(in, in_pitch, 1, out, out_pitch, nullptr, H, W, weights, radius, false,
                       reinterpret_cast<cudaStream_t>(stream));
 }
 

@@ -578,7 +578,7 @@ static int build_levels(const pysift_detect_config* cfg, const float* img, int p
         const int H = l.H[o], W = l.W[o], P = l.P[o];
         if (o == 0) {
             const int rc = blur_level(img, pitch, 1, lev_at(ws, l, 0, 0), P, nullptr, H, W, cfg->blur_weights[1],
-                                      cfg->blur_radius[1], st);
+                                      cfg->blur_radius[1], false, st);
             if (rc) return rc;
         }
         for (int s = 0; s < l.top; ++s) {
@@ -586,7 +586,7 @@ static int build_levels(const pysift_detect_config* cfg, const float* img, int p
             const float* in = first ? lev_at(ws, l, o - 1, cfg->n_scales) : lev_at(ws, l, o, s);
             const int rc = blur_level(in, first ? l.P[o - 1] : P, first ? 2 : 1, lev_at(ws, l, o, s + 1), P,
                                       first ? lev_at(ws, l, o, 0) : nullptr, H, W, cfg->blur_weights[2 + s],
-                                      cfg->blur_radius[2 + s], st);
+                                      cfg->blur_radius[2 + s], true, st);
             if (rc) return rc;
         }
     }
