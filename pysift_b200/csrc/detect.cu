@@ -365,27 +365,38 @@ constexpr int PC_TW = 32, PC_RB = 8, PC_TH = 8 * PC_RB;
 // Column FIR straight from the uint8 image: coef[r][x] = sum_k h[k] u[mirror(r+k)][x].
 // Each thread produces PC_RB consecutive rows of one column, streaming the
 // input window through registers (taps in ascending k for every output).
+// Bound by its float64 multiply-adds (61 a coefficient, 39 us for 12 Mpixel);
+// the window's bytes go through a table of the 256 widened values and skip
+// the mirroring away from the edges: 86 -> 72 us there.
 __global__ void __launch_bounds__(256) k_prefilter_cols(const uint8_t* __restrict__ img, int H, int W,
                                                         long long pitch, int fp16, double* __restrict__ coef,
                                                         const SplTaps taps) {
     chain_begin();
     __shared__ double tile[(PC_TH + 2 * SPL_K) * PC_TW];
+    // u / 255 as the base image holds it, widened: one conversion a value
+    __shared__ double unit[256];
     const int x0 = blockIdx.x * PC_TW, r0 = blockIdx.y * PC_TH;
     const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
     const int x = x0 + tx;
     {
-        // every load of the window issued before the first conversion
+        // every load of the window issued before the first look-up
         constexpr int NL = (PC_TH + 2 * SPL_K + 7) / 8;
         uint8_t u[NL];
+        const bool inside = r0 >= SPL_K && r0 + PC_TH + SPL_K <= H;
+        const uint8_t* src = img + (long long)(r0 - SPL_K + ty) * pitch + x;
 #pragma unroll
         for (int q = 0; q < NL; ++q) {
             const int rr = ty + 8 * q;
-            u[q] = (x < W && rr < PC_TH + 2 * SPL_K) ? img[mirror_index(r0 - SPL_K + rr, H) * pitch + x] : 0;
+            u[q] = 0;
+            if (x < W && rr < PC_TH + 2 * SPL_K)
+                u[q] = inside ? src[(long long)(8 * q) * pitch] : img[mirror_index(r0 - SPL_K + rr, H) * pitch + x];
         }
+        unit[threadIdx.x] = (double)u8_to_unit((uint8_t)threadIdx.x, fp16);
+        __syncthreads();
 #pragma unroll
         for (int q = 0; q < NL; ++q) {
             const int rr = ty + 8 * q;
-            if (rr < PC_TH + 2 * SPL_K) tile[rr * PC_TW + tx] = x < W ? (double)u8_to_unit(u[q], fp16) : 0.0;
+            if (rr < PC_TH + 2 * SPL_K) tile[rr * PC_TW + tx] = unit[u[q]];
         }
     }
     __syncthreads();
@@ -411,15 +422,14 @@ __global__ void __launch_bounds__(256) k_prefilter_cols(const uint8_t* __restric
 }
 
 // Output-coordinate setup for one axis of scipy's zoom (grid_mode=False,
-// mode='constant'): input coordinate k*(in-1)/(out-1), cubic B-spline
-// weights, mirror-mapped support; false outside [0, in-1] (cval 0).
-__device__ __forceinline__ bool zoom_axis(long long k, long long in_len, long long out_len, long long idx[4],
-                                          double w[4]) {
-    double zoom = (out_len > 1) ? (double)(in_len - 1) / (double)(out_len - 1) : 1.0;
+// mode='constant'): input coordinate k * zoom, zoom = (in-1)/(out-1), the first of the four
+// support positions (before mirroring) and cubic B-spline weights; false
+// outside [0, in-1] (cval 0).
+__device__ __forceinline__ bool zoom_axis(int k, int in_len, double zoom, int& start, double w[4]) {
     double cc = (double)k * zoom;
     if (cc < 0.0 || cc > (double)(in_len - 1)) return false;
     double fl = floor(cc);
-    long long start = (long long)fl - 1;
+    start = (int)fl - 1;
     double y = cc - fl;
     double z = 1.0 - y;
     w[0] = z * z * z / 6.0;
@@ -427,7 +437,6 @@ __device__ __forceinline__ bool zoom_axis(long long k, long long in_len, long lo
     double y1 = 1.0 - y;
     w[2] = (y1 * y1 * (y1 - 2.0) * 3.0 + 4.0) / 6.0;
     w[3] = 1.0 - w[0] - w[1] - w[2];
-    for (int h = 0; h < 4; ++h) idx[h] = mirror_index(start + h, in_len);
     return true;
 }
 
@@ -491,178 +500,164 @@ __global__ void __launch_bounds__(PR_NT) k_prefilter_rows(double* __restrict__ c
 // grid, t = sum_a sum_b (c[a][b] * wy_a) * wx_b in scipy's order, rounded to
 // float32.  On the 2x grid the output columns 2k-1 and 2k interpolate the
 // same 4 input columns (their input coordinates share the floor k-1), and
-// likewise the output rows 2k-1 and 2k.  A tile covers output rows
-// oy0-1 .. oy0+30 and columns ox0-1 .. ox0+62, so it splits into 16 x 32
-// such 2x2 quads; each thread takes 2 quads, loads the quad's 16
-// coefficients once and forms each c * wy_a once per row for both columns.
-// A quad whose rows or columns do not share their support (mirrored image
-// edges) reads each output's coefficients separately; either way each
-// output is the same sequence of products and sums.  The tile touches at
-// most 20 input rows and 36 input columns (zoom factor below 1/2).
-constexpr int ZI_TW = 64, ZI_TH = 32;
-constexpr int ZI_CR = 20, ZI_CC = 36;
+// likewise the output rows 2j-1 and 2j, so the grid splits into 2x2 quads of
+// common support.  A lane owns a column pair and its warp walks down the row
+// pairs of a tile: of the 16 coefficients 4 are new at each step (the window
+// in shared memory holds mirrored rows and columns past the image's edges, so
+// that every support is contiguous), the column weights stay in registers,
+// and each c * wy_a serves both columns.  What is left is the 160 float64
+// operations of a quad (108 us for the 48 Mpixel of a doubled 4000x3000 image
+// at 64 a cycle and SM); with all 16 coefficients and both axes' weights
+// fetched from shared memory per quad it was issue-bound: 283 -> 196 us there.
+// Three blocks an SM (80 registers) hide the chains' latency best.
+constexpr int ZI_T = 256, ZI_W = ZI_T / 32;
+constexpr int ZI_MAX_PAIRS = 16;                       // row pairs of a warp, at most
+constexpr int ZI_CC = 36;
 
-__device__ __forceinline__ double zoom_term_sum(const double (*win)[ZI_CC], const int* ry, const double* wy,
-                                                const int* cx, const double* wx) {
-    double t = 0.0;
-#pragma unroll
-    for (int a = 0; a < 4; ++a)
-#pragma unroll
-        for (int b = 0; b < 4; ++b) {
-            double coeff = win[ry[a]][cx[b]];
-            coeff *= wy[a];
-            coeff *= wx[b];
-            t += coeff;
-        }
-    return t;
-}
-
-__global__ void __launch_bounds__(256) k_zoom_interp(const double* __restrict__ coef, int H, int W, int fp16,
-                                                     float* __restrict__ out, int out_pitch) {
+__global__ void __launch_bounds__(ZI_T, 3) k_zoom_interp(const double* __restrict__ coef, int H, int W, double zy,
+                                                      double zx, int fp16, int pairs, float* __restrict__ out, int out_pitch) {
     chain_begin();
-    __shared__ int rvalid[ZI_TH], ridx[4][ZI_TH];
-    __shared__ double rw[4][ZI_TH];
-    __shared__ int cvalid[ZI_TW], cidx[4][ZI_TW];
-    __shared__ double cw[4][ZI_TW];
-    __shared__ int s_lo[2], s_hi[2];
-    __shared__ double win[ZI_CR][ZI_CC];
+    __shared__ __align__(16) double rw[2 * ZI_W * ZI_MAX_PAIRS][4];  // weights of output rows 2 j0 - 1 + i
+    __shared__ int rstart[2 * ZI_W * ZI_MAX_PAIRS];                  // first window row of their support, -1: outside
+    extern __shared__ double zi_win[];
+    double (*const win)[ZI_CC] = reinterpret_cast<double (*)[ZI_CC]>(zi_win);  // ZI_W * pairs + 4 rows
     const int OH = 2 * H, OW = 2 * W;
-    const int ox0 = blockIdx.x * ZI_TW, oy0 = blockIdx.y * ZI_TH;
-    const int tid = threadIdx.x;
-    if (tid < 2) {
-        s_lo[tid] = 0x7fffffff;
-        s_hi[tid] = -1;
+    const int k0 = blockIdx.x * 32, j0 = blockIdx.y * ZI_W * pairs;
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int npairs = min(ZI_W * pairs, H + 1 - j0);  // row pairs j0 .. of this tile
+    const int ylo = j0 - 2, xlo = k0 - 2;
+    {
+        const int xm = (int)mirror_index(xlo + lane, W), xn = (int)mirror_index(xlo + 32 + (lane & 3), W);
+        for (int yy = warp; yy < npairs + 4; yy += ZI_W) {
+            const int y = ylo + yy;
+            const double* src = coef + (long long)(y >= 0 && y < H ? y : (int)mirror_index(y, H)) * W;
+            const unsigned d = (unsigned)__cvta_generic_to_shared(&win[yy][lane]);
+            asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(d), "l"(src + xm) : "memory");
+            if (lane < 4)
+                asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(d + 32 * 8), "l"(src + xn) : "memory");
+        }
     }
-    __syncthreads();
-    if (tid < ZI_TH) {
-        const int r = oy0 - 1 + tid;
-        long long idx[4];
+    for (int i = tid; i < 2 * npairs; i += ZI_T) {
+        const int r = 2 * j0 - 1 + i;
         double w[4];
-        bool v = (r >= 0 && r < OH) && zoom_axis(r, H, OH, idx, w);
-        rvalid[tid] = v;
-        if (v) {
-            int lo = 0x7fffffff, hi = -1;
-            for (int q = 0; q < 4; ++q) {
-                ridx[q][tid] = (int)idx[q];
-                rw[q][tid] = w[q];
-                lo = min(lo, (int)idx[q]);
-                hi = max(hi, (int)idx[q]);
-            }
-            atomicMin(&s_lo[0], lo);
-            atomicMax(&s_hi[0], hi);
-        }
-    } else if (tid >= 32 && tid < 32 + ZI_TW) {
-        const int t = tid - 32;
-        const int x = ox0 - 1 + t;
-        long long idx[4];
-        double w[4];
-        bool v = (x >= 0 && x < OW) && zoom_axis(x, W, OW, idx, w);
-        cvalid[t] = v;
-        if (v) {
-            int lo = 0x7fffffff, hi = -1;
-            for (int q = 0; q < 4; ++q) {
-                cidx[q][t] = (int)idx[q];
-                cw[q][t] = w[q];
-                lo = min(lo, (int)idx[q]);
-                hi = max(hi, (int)idx[q]);
-            }
-            atomicMin(&s_lo[1], lo);
-            atomicMax(&s_hi[1], hi);
-        }
+        int start = 0;
+        const bool v = r >= 0 && r < OH && zoom_axis(r, H, zy, start, w);
+        rstart[i] = v ? start - ylo : -1;
+#pragma unroll
+        for (int q = 0; q < 4; ++q) rw[i][q] = v ? w[q] : 0.0;
     }
+    // this lane's column pair 2 k - 1, 2 k
+    const int xa = 2 * (k0 + lane) - 1, xb = xa + 1;
+    double wxa[4] = {0.0, 0.0, 0.0, 0.0}, wxb[4] = {0.0, 0.0, 0.0, 0.0};
+    int sa = 0, sb = 0;
+    const bool cva = xa >= 0 && xa < OW && zoom_axis(xa, W, zx, sa, wxa);
+    const bool cvb = xb < OW && zoom_axis(xb, W, zx, sb, wxb);
+    const int col = cva ? sa - xlo : (cvb ? sb - xlo : 0);
+    // both columns of a pair share their support wherever both exist
+    const bool odd_pair = cva && cvb && sa != sb;
+    asm volatile("cp.async.wait_all;" ::: "memory");
     __syncthreads();
-    const int ylo = s_lo[0], yhi = s_hi[0], xlo = s_lo[1], xhi = s_hi[1];
-    const bool any = (yhi >= 0 && xhi >= 0);
-    const int ny = any ? yhi - ylo + 1 : 0, nx = any ? xhi - xlo + 1 : 0;
-    const bool fits = ny <= ZI_CR && nx <= ZI_CC;
-    const int warp = tid >> 5, lane = tid & 31;
-    if (any && fits) {
-        for (int yy = warp; yy < ny; yy += 8) {
-            const double* src = coef + (long long)(ylo + yy) * W + xlo;
-            for (int xx = lane; xx < nx; xx += 32) {
-                const unsigned d = (unsigned)__cvta_generic_to_shared(&win[yy][xx]);
-                asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(d), "l"(src + xx) : "memory");
-            }
-        }
-        asm volatile("cp.async.wait_all;" ::: "memory");
-    }
-    __syncthreads();
-    // this lane's column pair
-    const int ta = 2 * lane, tb = ta + 1;
-    const int xa = ox0 - 1 + ta, xb = xa + 1;
-    const bool cva = cvalid[ta], cvb = cvalid[tb];
-    int cxa[4], cxb[4];
-    double wxa[4], wxb[4];
-    bool csame = cva && cvb;
+    const bool pair_stores = (out_pitch & 1) == 0 && (reinterpret_cast<uintptr_t>(out) & 7) == 0;
+    double c[4][4];  // rows of the support, rotating
+    int have = -2;   // window row of the support's first row
+    auto step = [&](int q, auto phase) {
+        constexpr int ph = decltype(phase)::value;
+        const int pair = warp * pairs + q;
+        if (pair >= npairs) return;
+        const int i = 2 * pair, ra = 2 * j0 - 1 + i, rb = ra + 1;
+        const int ya = rstart[i], yb = rstart[i + 1], y = ya >= 0 ? ya : yb;
+        float v[2][2] = {{0.0f, 0.0f}, {0.0f, 0.0f}};
+        if (y >= 0) {
+            if (y == have + 1) {
 #pragma unroll
-    for (int q = 0; q < 4; ++q) {
-        cxa[q] = cva ? cidx[q][ta] - xlo : 0;
-        cxb[q] = cvb ? cidx[q][tb] - xlo : 0;
-        wxa[q] = cva ? cw[q][ta] : 0.0;
-        wxb[q] = cvb ? cw[q][tb] : 0.0;
-        csame = csame && cxa[q] == cxb[q];
-    }
-    const float nan = __int_as_float(0x7fc00000);  // unreachable by construction; visible in parity tests
-    for (int pr = warp; pr < ZI_TH / 2; pr += 8) {
-        const int ua = 2 * pr, ub = ua + 1;
-        const int ra = oy0 - 1 + ua, rb = ra + 1;
-        const bool rva = rvalid[ua], rvb = rvalid[ub];
-        int rya[4], ryb[4];
-        double wya[4], wyb[4];
-        bool rsame = rva && rvb;
-#pragma unroll
-        for (int q = 0; q < 4; ++q) {
-            rya[q] = rva ? ridx[q][ua] - ylo : 0;
-            ryb[q] = rvb ? ridx[q][ub] - ylo : 0;
-            wya[q] = rva ? rw[q][ua] : 0.0;
-            wyb[q] = rvb ? rw[q][ub] : 0.0;
-            rsame = rsame && rya[q] == ryb[q];
-        }
-        double t00 = 0.0, t01 = 0.0, t10 = 0.0, t11 = 0.0;
-        if (fits) {
-            if (rsame && csame) {
-                double c[4][4];
-#pragma unroll
-                for (int a = 0; a < 4; ++a)
-#pragma unroll
-                    for (int b = 0; b < 4; ++b) c[a][b] = win[rya[a]][cxa[b]];
-#pragma unroll
-                for (int a = 0; a < 4; ++a)
-#pragma unroll
-                    for (int b = 0; b < 4; ++b) {
-                        const double pa = c[a][b] * wya[a];
-                        const double pb = c[a][b] * wyb[a];
-                        t00 += pa * wxa[b];
-                        t01 += pa * wxb[b];
-                        t10 += pb * wxa[b];
-                        t11 += pb * wxb[b];
-                    }
+                for (int b = 0; b < 4; ++b) c[(ph + 3) & 3][b] = win[y + 3][col + b];
             } else {
-                if (rva && cva) t00 = zoom_term_sum(win, rya, wya, cxa, wxa);
-                if (rva && cvb) t01 = zoom_term_sum(win, rya, wya, cxb, wxb);
-                if (rvb && cva) t10 = zoom_term_sum(win, ryb, wyb, cxa, wxa);
-                if (rvb && cvb) t11 = zoom_term_sum(win, ryb, wyb, cxb, wxb);
+#pragma unroll
+                for (int a = 0; a < 4; ++a)
+#pragma unroll
+                    for (int b = 0; b < 4; ++b) c[(ph + a) & 3][b] = win[y + a][col + b];
             }
-        }
-        const double tq[2][2] = {{t00, t01}, {t10, t11}};
-        const bool rv[2] = {rva, rvb}, cv[2] = {cva, cvb};
-        const int rr[2] = {ra, rb}, xx[2] = {xa, xb};
+            have = y;
+            double wy[2][4];
 #pragma unroll
-        for (int i = 0; i < 2; ++i) {
-            if (rr[i] < 0 || rr[i] >= OH) continue;
+            for (int u = 0; u < 2; ++u)
 #pragma unroll
-            for (int j = 0; j < 2; ++j) {
-                if (xx[j] < 0 || xx[j] >= OW) continue;
-                float res = 0.0f;
-                if (rv[i] && cv[j]) {
-                    res = fits ? (float)tq[i][j] : nan;
-                    if (fits && fp16) res = round_half(res);
+                for (int h = 0; h < 2; ++h) {
+                    const double2 w2 = reinterpret_cast<const double2*>(rw[i + u])[h];
+                    wy[u][2 * h] = w2.x;
+                    wy[u][2 * h + 1] = w2.y;
                 }
-                out[(long long)rr[i] * out_pitch + xx[j]] = res;
+            double t[2][2] = {{0.0, 0.0}, {0.0, 0.0}};
+#pragma unroll
+            for (int a = 0; a < 4; ++a) {
+                const double w0 = wy[0][a], w1 = wy[1][a];
+#pragma unroll
+                for (int b = 0; b < 4; ++b) {
+                    const double p0 = c[(ph + a) & 3][b] * w0, p1 = c[(ph + a) & 3][b] * w1;
+                    t[0][0] += p0 * wxa[b];
+                    t[0][1] += p0 * wxb[b];
+                    t[1][0] += p1 * wxa[b];
+                    t[1][1] += p1 * wxb[b];
+                }
+            }
+            if (odd_pair || (ya >= 0 && yb >= 0 && ya != yb)) {
+                // supports that differ: each output from its own
+                for (int u = 0; u < 2; ++u)
+                    for (int w = 0; w < 2; ++w) {
+                        const int y0 = u ? yb : ya, x0 = (w ? sb : sa) - xlo;
+                        double s = 0.0;
+                        if (y0 >= 0 && (w ? cvb : cva))
+                            for (int a = 0; a < 4; ++a)
+                                for (int b = 0; b < 4; ++b) {
+                                    double coeff = win[y0 + a][x0 + b] * rw[i + u][a];
+                                    coeff *= w ? wxb[b] : wxa[b];
+                                    s += coeff;
+                                }
+                        if (u == 0 && w == 0) t[0][0] = s;
+                        if (u == 0 && w == 1) t[0][1] = s;
+                        if (u == 1 && w == 0) t[1][0] = s;
+                        if (u == 1 && w == 1) t[1][1] = s;
+                    }
+            }
+#pragma unroll
+            for (int u = 0; u < 2; ++u) {
+                const bool rv = (u ? yb : ya) >= 0;
+                v[u][0] = rv && cva ? (float)t[u][0] : 0.0f;
+                v[u][1] = rv && cvb ? (float)t[u][1] : 0.0f;
+                if (fp16) {
+                    v[u][0] = round_half(v[u][0]);
+                    v[u][1] = round_half(v[u][1]);
+                }
+            }
+        } else {
+            have = -2;
+        }
+        // columns 2 k (this lane's) and 2 k + 1 (the next lane's) as one word
+#pragma unroll
+        for (int u = 0; u < 2; ++u) {
+            const float right = __shfl_down_sync(FULL_MASK, v[u][0], 1);
+            const int r = u ? rb : ra;
+            if (r < 0 || r >= OH) continue;
+            float* row = out + (long long)r * out_pitch;
+            if (lane == 0 && xa >= 0 && xa < OW) row[xa] = v[u][0];
+            if (xb < OW) {
+                if (lane < 31 && pair_stores) *reinterpret_cast<float2*>(row + xb) = make_float2(v[u][1], right);
+                else {
+                    row[xb] = v[u][1];
+                    if (lane < 31) row[xb + 1] = right;
+                }
             }
         }
+    };
+    for (int q = 0; q < pairs; q += 4) {
+        step(q, std::integral_constant<int, 0>{});
+        if (q + 1 < pairs) step(q + 1, std::integral_constant<int, 1>{});
+        if (q + 2 < pairs) step(q + 2, std::integral_constant<int, 2>{});
+        if (q + 3 < pairs) step(q + 3, std::integral_constant<int, 3>{});
     }
 }
+
+static int num_sms();
 
 static int launch_zoom2x(const uint8_t* gray, int H, int W, long long pitch, int fp16, double* coef, float* out,
                          int out_pitch, cudaStream_t st) {
@@ -672,8 +667,15 @@ static int launch_zoom2x(const uint8_t* gray, int H, int W, long long pitch, int
     PYSIFT_LAUNCH_CHECK("k_prefilter_cols");
     launch_chained(k_prefilter_rows, dim3(H), PR_NT, 0, st, coef, W, taps);
     PYSIFT_LAUNCH_CHECK("k_prefilter_rows");
-    launch_chained(k_zoom_interp, dim3(ceil_div(2 * W + 1, ZI_TW), ceil_div(2 * H + 1, ZI_TH)), 256, 0, st,
-                   (const double*)coef, H, W, fp16, out, out_pitch);
+    // row pairs of a warp: long walks while they fill the SMs, shorter ones for
+    // small images
+    int pairs = ZI_MAX_PAIRS;
+    auto blocks = [&] { return (long long)ceil_div(W + 1, 32) * ceil_div(H + 1, ZI_W * pairs); };
+    while (pairs > 1 && blocks() < 3LL * num_sms()) pairs /= 2;
+    const double zy = (double)(H - 1) / (double)(2 * H - 1), zx = (double)(W - 1) / (double)(2 * W - 1);
+    const size_t window = (size_t)(ZI_W * pairs + 4) * ZI_CC * sizeof(double);
+    launch_chained(k_zoom_interp, dim3(ceil_div(W + 1, 32), ceil_div(H + 1, ZI_W * pairs)), ZI_T, window, st,
+                   (const double*)coef, H, W, zy, zx, fp16, pairs, out, out_pitch);
     PYSIFT_LAUNCH_CHECK("k_zoom_interp");
     return PYSIFT_OK;
 }
