@@ -47,6 +47,7 @@ struct BlendCtl {
     int have_ov, vertical, first_side;  // first_side: image 1 left of (vertical) / above the seam
     int n_lines, seam_end;              // overlap lines; seam position on the last one
     int band_lo, band_hi;               // union of the overlap lines' ranges
+    int ov_x0, ov_x1, ov_y0, ov_y1;     // bounding box of the overlap (x1 < x0 without one)
     int chunk;                          // backtrack chunk length
     int hist;                           // colour matching: 0 gain, 1 histograms (pysift/core.py:3694-3699)
     unsigned int hist1[3][256], hist2[3][256];  // overlap histograms of images 1 and 2
@@ -73,6 +74,22 @@ __device__ __forceinline__ float color_matched(const BlendCtl* ctl, float v, int
     const float x = v * ctl->gain[c];
     return x < 0.0f ? 0.0f : (x > 255.0f ? 255.0f : x);
 }
+
+// color_matched of one channel with its control words read once
+struct ChannelMatch {
+    const BlendCtl* ctl;
+    int c;
+    bool have, hist;
+    float gain;
+    __device__ __forceinline__ ChannelMatch(const BlendCtl* k, int ch)
+        : ctl(k), c(ch), have(k->have_ov != 0), hist(k->hist != 0), gain(k->gain[ch]) {}
+    __device__ __forceinline__ float operator()(float v) const {
+        if (!have) return v;
+        if (hist) return color_matched(ctl, v, c);
+        const float x = v * gain;
+        return x < 0.0f ? 0.0f : (x > 255.0f ? 255.0f : x);
+    }
+};
 
 template <typename T>
 __device__ __forceinline__ T warp_sum(T v) {
@@ -302,6 +319,11 @@ __global__ void __launch_bounds__(1024) k_blend_decide(BlendCtl* ctl, const int*
         ctl->n_lines = nL;
         ctl->band_lo = s_lo;
         ctl->band_hi = s_hi;
+        const int l0 = nL ? ovl[0] : 0x7fffffff, l1 = nL ? ovl[nL - 1] : -1;
+        ctl->ov_x0 = vert ? s_lo : l0;
+        ctl->ov_x1 = vert ? s_hi : l1;
+        ctl->ov_y0 = vert ? l0 : s_lo;
+        ctl->ov_y1 = vert ? l1 : s_hi;
         int R = 16;
         while (2 * R * R < nL) R *= 2;
         ctl->chunk = R;
@@ -754,7 +776,7 @@ __global__ void __launch_bounds__(1024) k_seam_walk(const uint8_t* __restrict__ 
 // filter taps passed by value (kernel parameters: no host copies, so the
 // composition can be captured in a CUDA graph)
 struct SeamTaps {
-    float k[25];
+    double k[25];
 };
 struct GaussTaps {
     double w[9];
@@ -785,11 +807,15 @@ __global__ void __launch_bounds__(SR_T) k_seam_rows(const uint8_t* __restrict__ 
                                                     const SeamTaps k25, float* __restrict__ out, int W) {
     __shared__ float sv[SR_N + SR_N / 8 + 1];
     const int y = blockIdx.y, x0 = blockIdx.x * SR_T * SR_R;
+    // only what the column pass reads: the overlap's box, 12 rows taller each
+    // side (88 -> 47 us on a 4783x2585 canvas)
+    const int ox0 = ctl->ov_x0, ox1 = ctl->ov_x1;
+    if (y < ctl->ov_y0 - 12 || y > ctl->ov_y1 + 12 || x0 > ox1 || x0 + SR_T * SR_R <= ox0) return;
     for (int i = threadIdx.x; i < SR_N; i += SR_T)
         sv[sr_phys(i)] = seam_value(m1, m2, seam, ctl, refl_101(x0 + i - 12, W), y, W);
     __syncthreads();
     const int b = threadIdx.x * SR_R;
-    if (x0 + b >= W) return;
+    if (x0 + b > ox1 || x0 + b + SR_R <= ox0) return;
     double v[SR_R + 24];
 #pragma unroll
     for (int m = 0; m < SR_R + 24; ++m) v[m] = (double)sv[sr_phys(b + m)];
@@ -799,26 +825,49 @@ __global__ void __launch_bounds__(SR_T) k_seam_rows(const uint8_t* __restrict__ 
         if (x >= W) break;
         double s = 0.0;
 #pragma unroll
-        for (int t = 0; t < 25; ++t) s = s + (double)k25.k[t] * v[j + t];
+        for (int t = 0; t < 25; ++t) s = s + k25.k[t] * v[j + t];
         out[(long long)y * W + x] = (float)s;
     }
 }
 
 // ... then the column pass; the blurred value replaces the mask where both
-// images cover the canvas (pysift/core.py:3469-3471)
-__global__ void k_seam_cols(const float* __restrict__ rows, const uint8_t* __restrict__ m1,
-                            const uint8_t* __restrict__ m2, const int* __restrict__ seam, const BlendCtl* ctl,
-                            const SeamTaps k25, float* __restrict__ gm0, int W, int H) {
-    const int x = blockIdx.x * blockDim.x + threadIdx.x, y = blockIdx.y;
+// images cover the canvas (pysift/core.py:3469-3471).  A thread owns SC_L rows
+// of one column and walks their SC_L + 24 inputs once: each is loaded and
+// widened once and added to the up to 25 sums that hold it, which live in
+// registers (the loop is unrolled over the strip) and each take their taps in
+// order.  One sum at a time over 25 loads was bound by the 25 conversions to
+// float64 an output: 50 us on a 2112x1213 canvas and 226 us at 4783x2585, now
+// 20 and 57.  Columns of a strip without overlap only take the mask.
+constexpr int SC_T = 128, SC_L = 32;
+__global__ void __launch_bounds__(SC_T) k_seam_cols(const float* __restrict__ rows, const uint8_t* __restrict__ m1,
+                                                    const uint8_t* __restrict__ m2, const SeamTaps k25,
+                                                    float* __restrict__ gm0, int W, int H) {
+    __shared__ long long s_row[SC_L + 24];
+    const int x = blockIdx.x * SC_T + threadIdx.x, y0 = blockIdx.y * SC_L;
+    if (threadIdx.x < SC_L + 24)
+        s_row[threadIdx.x] = (long long)refl_101(min(y0 + (int)threadIdx.x - 12, H + 11), H) * W;
+    __syncthreads();
     if (x >= W) return;
-    const long long p = (long long)y * W + x;
-    if (m1[p] && m2[p]) {
-        double s = 0.0;
-#pragma unroll 5
-        for (int t = 0; t < 25; ++t) s = s + (double)k25.k[t] * (double)rows[(long long)refl_101(y + t - 12, H) * W + x];
-        gm0[p] = (float)s;
-    } else {
-        gm0[p] = seam_value(m1, m2, seam, ctl, x, y, W);
+    const int n = min(SC_L, H - y0);
+    uint32_t need = 0;
+#pragma unroll 8
+    for (int r = 0; r < SC_L; ++r) {
+        if (r < n) {
+            const long long p = (long long)(y0 + r) * W + x;
+            const bool a = m1[p] != 0, b = m2[p] != 0;
+            if (a && b) need |= 1u << r;
+            else gm0[p] = a ? 1.0f : 0.0f;
+        }
+    }
+    if (!need) return;
+    double s[SC_L];
+#pragma unroll
+    for (int i = 0; i < SC_L + 24; ++i) {
+        const double v = (double)rows[s_row[i] + x];
+#pragma unroll
+        for (int o = i > 24 ? i - 24 : 0; o <= (i < SC_L ? i : SC_L - 1); ++o)
+            s[o] = (i == o ? 0.0 : s[o]) + k25.k[i - o] * v;
+        if (i >= 24 && (need >> (i - 24) & 1u)) gm0[(long long)(y0 + i - 24) * W + x] = (float)s[i - 24];
     }
 }
 
@@ -1014,47 +1063,145 @@ __global__ void k_blend_reconstruct(const float* __restrict__ res, int hn, int w
 // (result = up(res) + lb0) and the paste (pysift/core.py:3806-3809): uint8
 // truncation of the clipped value where either image covers the canvas.
 // With one level there is no pyramid: result = m * I1 + (1 - m) * I2.
-__global__ void k_blend_final(const Level0 src, const float* __restrict__ gm0, const float* __restrict__ g1n,
-                              const float* __restrict__ g2n, const float* __restrict__ res, int hn, int wn, int H,
-                              int W, ZoomF zf, uint8_t* __restrict__ pano, uint8_t* __restrict__ both,
-                              float* __restrict__ blended, double* __restrict__ seam_rmse) {
-    const int x = blockIdx.x * blockDim.x + threadIdx.x, y = blockIdx.y;
-    if (x == 0 && y == 0 && seam_rmse) {
-        const BlendCtl* ctl = src.ctl;
+// A thread owns one column and walks BF_R rows down.  The corners of the three
+// zooms stay in registers as float64: about every second row brings a new
+// source row, 9 conversions to float64 a pixel instead of 36.  What is left is
+// latency: the corners take 72 registers, so 16 warps run on an SM.  71 us on a
+// 2112x1213 canvas and 279 us at 4783x2585; one thread a pixel that loads and
+// widens every corner 82 and 397, one channel a thread (all accesses
+// contiguous, but the address work three times) 94 and 404.
+constexpr int BF_T = 128, BF_R = 16;
+template <bool U8, bool PYR>
+__global__ void __launch_bounds__(BF_T, 4) k_blend_final(const Level0 src, const float* __restrict__ gm0,
+                                                         const float* __restrict__ g1n, const float* __restrict__ g2n,
+                                                         const float* __restrict__ res, int hn, int wn, int H, int W,
+                                                         ZoomF zf, uint8_t* __restrict__ pano,
+                                                         uint8_t* __restrict__ both, float* __restrict__ blended,
+                                                         double* __restrict__ seam_rmse) {
+    __shared__ int s_y[BF_R][2];
+    __shared__ double s_w[BF_R][2];
+    const BlendCtl* ctl = src.ctl;
+    const int y0 = blockIdx.y * BF_R, x = blockIdx.x * BF_T + threadIdx.x;
+    if (x == 0 && y0 == 0 && seam_rmse)
         *seam_rmse = ctl->n_ov ? sqrt((double)ctl->sq / (3.0 * (double)ctl->n_ov))
                                : __longlong_as_double(0x7ff8000000000000ll);
+    if (PYR && threadIdx.x < BF_R) {
+        const Zoom1 z(hn, wn, zf, y0 + threadIdx.x, 0);
+        s_y[threadIdx.x][0] = (int)(z.o[0] / wn);
+        s_y[threadIdx.x][1] = (int)(z.o[2] / wn);
+        s_w[threadIdx.x][0] = z.wy[0];
+        s_w[threadIdx.x][1] = z.wy[1];
     }
+    __syncthreads();
     if (x >= W) return;
-    const long long p = (long long)y * W + x;
-    const bool any = src.m1[p] || src.m2[p];
-    if (both) both[p] = any;
-    float i1[3], i2[3];
-    src.px(p, i1, i2);
-    const float m = gm0[p];
-    const float mc = 1.0f - m;
-    float v[3];
-    if (res) {
-        const Zoom1 z(hn, wn, zf, y, x);
+    // without an overlap a gain of 1 leaves uint8 values as they are
+    const bool special = (U8 ? false : ctl->have_ov == 0) || (ctl->have_ov && ctl->hist);
+    const float gain[3] = {ctl->gain[0], ctl->gain[1], ctl->gain[2]};
+    // the corner columns and weights of x (row 0: offsets within a row)
+    int oa = 0, ob = 0;
+    double wx0 = 0.0, wx1 = 0.0;
+    if (PYR) {
+        const Zoom1 z(hn, wn, zf, 0, x);
+        oa = 3 * (int)z.o[0];
+        ob = 3 * (int)z.o[1];
+        wx0 = z.wx[0];
+        wx1 = z.wx[1];
+    }
+    const int n = min(BF_R, H - y0);
+    double top[9][2], bot[9][2];  // the source rows ya and yb
+    int ya = -1, yb = -1;
+    auto load = [&](double (*d)[2], int yy) {
+        const long long row = (long long)yy * wn * 3;
+        const float* const ga[3] = {g1n + row + oa, g2n + row + oa, res + row + oa};
+        const float* const gb[3] = {g1n + row + ob, g2n + row + ob, res + row + ob};
 #pragma unroll
-        for (int c = 0; c < 3; ++c) {
-            const float l1 = i1[c] - z.at(g1n, 3, c);
-            const float l2 = i2[c] - z.at(g2n, 3, c);
-            const float lb = m * l1 + mc * l2;
-            v[c] = z.at(res, 3, c) + lb;
+        for (int k = 0; k < 9; ++k) {
+            d[k][0] = (double)ga[k / 3][k % 3];
+            d[k][1] = (double)gb[k / 3][k % 3];
         }
-    } else {
-#pragma unroll
-        for (int c = 0; c < 3; ++c) v[c] = m * i1[c] + mc * i2[c];
-    }
-    if (blended) {
-#pragma unroll
-        for (int c = 0; c < 3; ++c) blended[p * 3 + c] = v[c];
-    }
-    if (pano) {
+    };
+    const long long p0 = (long long)y0 * W + x;
+    const uint8_t* pm1 = src.m1 + p0;
+    const uint8_t* pm2 = src.m2 + p0;
+    const uint8_t* pc2 = src.c2 + 3 * p0;
+    const uint8_t* pu = U8 ? src.w1.u8 + 3 * p0 : nullptr;
+    const float* pf = U8 ? nullptr : src.w1.f32 + 3 * p0;
+    const float* pg = gm0 + p0;
+    uint8_t* po = pano ? pano + 3 * p0 : nullptr;
+    for (int r = 0; r < n; ++r) {
+        const bool a = *pm1 != 0, b = *pm2 != 0;
+        float v[3], v2[3];
 #pragma unroll
         for (int c = 0; c < 3; ++c) {
-            const float t = v[c] < 0.0f ? 0.0f : (v[c] > 255.0f ? 255.0f : v[c]);
-            pano[p * 3 + c] = any ? (uint8_t)(int)t : (uint8_t)0;
+            v[c] = U8 ? (float)pu[c] : pf[c];
+            v2[c] = (float)pc2[c];
+        }
+        const float m = *pg, mc = 1.0f - m;
+        pm1 += W, pm2 += W, pg += W, pc2 += 3 * W;
+        if (U8) pu += 3 * W;
+        else pf += 3 * W;
+        if (special) {
+#pragma unroll
+            for (int c = 0; c < 3; ++c) v[c] = color_matched(ctl, v[c], c);
+        } else {
+#pragma unroll
+            for (int c = 0; c < 3; ++c) {
+                const float t = v[c] * gain[c];
+                v[c] = t < 0.0f ? 0.0f : (t > 255.0f ? 255.0f : t);
+            }
+        }
+        float o[3];
+        if (PYR) {
+            const int wa = s_y[r][0], wb = s_y[r][1];
+            if (wa != ya) {
+                if (wa == yb) {
+#pragma unroll
+                    for (int k = 0; k < 9; ++k) top[k][0] = bot[k][0], top[k][1] = bot[k][1];
+                } else {
+                    load(top, wa);
+                }
+                ya = wa;
+            }
+            if (wb != yb) {
+                load(bot, wb);
+                yb = wb;
+            }
+        }
+        const double wy0 = PYR ? s_w[r][0] : 0.0, wy1 = PYR ? s_w[r][1] : 0.0;
+#pragma unroll
+        for (int c = 0; c < 3; ++c) {
+            const float i1 = a ? v[c] : (b ? v2[c] : 0.0f), i2 = b ? v2[c] : (a ? v[c] : 0.0f);
+            if (PYR) {
+                float up[3];  // Zoom1::at's sums
+#pragma unroll
+                for (int k = 0; k < 3; ++k) {
+                    const int j = 3 * k + c;
+                    double t = 0.0 + (top[j][0] * wy0) * wx0;
+                    t = t + (top[j][1] * wy0) * wx1;
+                    t = t + (bot[j][0] * wy1) * wx0;
+                    t = t + (bot[j][1] * wy1) * wx1;
+                    up[k] = (float)t;
+                }
+                const float l1 = i1 - up[0], l2 = i2 - up[1];
+                o[c] = up[2] + (m * l1 + mc * l2);
+            } else {
+                o[c] = m * i1 + mc * i2;
+            }
+        }
+        if (po) {
+            const float lim = a || b ? 255.0f : 0.0f;  // 0 off the canvas' covered part
+#pragma unroll
+            for (int c = 0; c < 3; ++c) {
+                const float t = o[c] < 0.0f ? 0.0f : (o[c] > lim ? lim : o[c]);
+                po[c] = (uint8_t)(int)t;
+            }
+            po += 3 * W;
+        }
+        const long long p = p0 + (long long)r * W;
+        if (both) both[p] = a || b;
+        if (blended) {
+#pragma unroll
+            for (int c = 0; c < 3; ++c) blended[3 * p + c] = o[c];
         }
     }
 }
@@ -1330,10 +1477,12 @@ int pysift_blend_multiband(const void* image1, int32_t image1_f32, const uint8_t
     PYSIFT_CUDA_TRY(cudaMemsetAsync(colf, 0, (size_t)cw * 4, st));
     PYSIFT_CUDA_TRY(cudaMemsetAsync(clo, 0x7f, (size_t)cw * 4, st));
     PYSIFT_CUDA_TRY(cudaMemsetAsync(chi, 0xff, (size_t)cw * 4, st));
+    uint8_t* dir = bwp<uint8_t>(ws, l.off_dir);
+    PYSIFT_CUDA_TRY(cudaMemsetAsync(dir, 0, std::max(align_up(cw, 4) * ch, align_up(ch, 4) * cw), st));
     GaussTaps w9;
     SeamTaps k25;
     for (int i = 0; i < 9; ++i) w9.w[i] = gauss_w9[i];
-    for (int i = 0; i < 25; ++i) k25.k[i] = seam_k25[i];
+    for (int i = 0; i < 25; ++i) k25.k[i] = (double)seam_k25[i];
     const dim3 g2d(ceil_div(cw, 256), ch);
     // gain, overlap flags and ranges, seam orientation
     const int hist = color_match == 1;
@@ -1347,7 +1496,6 @@ int pysift_blend_multiband(const void* image1, int32_t image1_f32, const uint8_t
         k_blend_hist_lut<<<3, 256, 0, st>>>(ctl);
         PYSIFT_LAUNCH_CHECK("k_blend_hist_lut");
     }
-    // Gaussian pyramids of I1 and I2 on a side stream: they need only the gain
     Level0 src;
     src.w1 = w1;
     src.m1 = mask1;
@@ -1359,26 +1507,6 @@ int pysift_blend_multiband(const void* image1, int32_t image1_f32, const uint8_t
     cudaEvent_t fork_ev = nullptr, join_ev = nullptr;
     PYSIFT_CUDA_TRY(cudaEventCreateWithFlags(&fork_ev, cudaEventDisableTiming));
     PYSIFT_CUDA_TRY(cudaEventCreateWithFlags(&join_ev, cudaEventDisableTiming));
-    PYSIFT_CUDA_TRY(cudaEventRecord(fork_ev, st));
-    PYSIFT_CUDA_TRY(cudaStreamWaitEvent(side, fork_ev, 0));
-    {
-        float* t1 = bwp<float>(ws, l.off_t1);
-        float* t2 = bwp<float>(ws, l.off_t2);
-        for (int k = 0; k + 1 < n_levels; ++k) {
-            PyrLevel in;
-            in.g1 = k ? bwp<float>(ws, l.off_g1[k]) : nullptr;
-            in.g2 = k ? bwp<float>(ws, l.off_g2[k]) : nullptr;
-            in.gm = nullptr;
-            const int ho = l.h[k + 1], wo = l.w[k + 1];
-            const dim3 gr(ceil_div(l.w[k], 128), ho), gc(ceil_div(wo, 128), ho);
-            if (k == 0) k_pyr_rows<6, true><<<gr, 128, 0, side>>>(src, in, l.w[k], l.h[k], t1, t2, w9);
-            else k_pyr_rows<6, false><<<gr, 128, 0, side>>>(src, in, l.w[k], l.h[k], t1, t2, w9);
-            k_pyr_cols<6><<<gc, 128, 0, side>>>(t1, t2, l.w[k], wo, w9, bwp<float>(ws, l.off_g1[k + 1]),
-                                                bwp<float>(ws, l.off_g2[k + 1]));
-        }
-        PYSIFT_LAUNCH_CHECK("k_pyr images");
-    }
-    PYSIFT_CUDA_TRY(cudaEventRecord(join_ev, side));
     // seam cost
     float* color = bwp<float>(ws, l.off_color);
     float* avg = bwp<float>(ws, l.off_avg);
@@ -1387,16 +1515,36 @@ int pysift_blend_multiband(const void* image1, int32_t image1_f32, const uint8_t
     PYSIFT_LAUNCH_CHECK("k_blend_prepare");
     k_sobel_cost<<<g2d, 256, 0, st>>>(avg, color, mask1, mask2, ctl, dpc, cw, ch);
     PYSIFT_LAUNCH_CHECK("k_sobel_cost");
+    PYSIFT_CUDA_TRY(cudaEventRecord(fork_ev, st));
     // DP seam and backtrack
     int* seam = bwp<int>(ws, l.off_seam);
     {
-        uint8_t* dir = bwp<uint8_t>(ws, l.off_dir);
         const int M = cw > ch ? cw : ch;
-        const size_t dir_bytes = std::max(align_up(cw, 4) * ch, align_up(ch, 4) * cw);
-        PYSIFT_CUDA_TRY(cudaMemsetAsync(dir, 0, dir_bytes, st));
         k_blend_dp<<<DP_CTAS, DP_T, 0, st>>>(dpc, ovl, cw, ch, ctl, bwp<double>(ws, l.off_rowA),
                                              bwp<double>(ws, l.off_rowB), dir);
         PYSIFT_LAUNCH_CHECK("k_blend_dp");
+        // the Gaussian pyramids of I1 and I2, which need only the gain, on a
+        // side stream beside the 8 CTAs of the seam search (beside the seam
+        // cost, which fills the chip, they held it up by 60 us at 2112x1213)
+        PYSIFT_CUDA_TRY(cudaStreamWaitEvent(side, fork_ev, 0));
+        {
+            float* t1 = bwp<float>(ws, l.off_t1);
+            float* t2 = bwp<float>(ws, l.off_t2);
+            for (int k = 0; k + 1 < n_levels; ++k) {
+                PyrLevel in;
+                in.g1 = k ? bwp<float>(ws, l.off_g1[k]) : nullptr;
+                in.g2 = k ? bwp<float>(ws, l.off_g2[k]) : nullptr;
+                in.gm = nullptr;
+                const int ho = l.h[k + 1], wo = l.w[k + 1];
+                const dim3 gr(ceil_div(l.w[k], 128), ho), gc(ceil_div(wo, 128), ho);
+                if (k == 0) k_pyr_rows<6, true><<<gr, 128, 0, side>>>(src, in, l.w[k], l.h[k], t1, t2, w9);
+                else k_pyr_rows<6, false><<<gr, 128, 0, side>>>(src, in, l.w[k], l.h[k], t1, t2, w9);
+                k_pyr_cols<6><<<gc, 128, 0, side>>>(t1, t2, l.w[k], wo, w9, bwp<float>(ws, l.off_g1[k + 1]),
+                                                    bwp<float>(ws, l.off_g2[k + 1]));
+            }
+            PYSIFT_LAUNCH_CHECK("k_pyr images");
+        }
+        PYSIFT_CUDA_TRY(cudaEventRecord(join_ev, side));
         int* jump = bwp<int>(ws, l.off_jump);
         k_seam_jump<<<dim3(ceil_div(M, 256), l.nchunk), 256, 0, st>>>(dir, ovl, ctl, cw, ch, jump);
         PYSIFT_LAUNCH_CHECK("k_seam_jump");
@@ -1408,7 +1556,7 @@ int pysift_blend_multiband(const void* image1, int32_t image1_f32, const uint8_t
     float* srow = bwp<float>(ws, l.off_srow);
     k_seam_rows<<<dim3(ceil_div(cw, SR_T * SR_R), ch), SR_T, 0, st>>>(mask1, mask2, seam, ctl, k25, srow, cw);
     PYSIFT_LAUNCH_CHECK("k_seam_rows");
-    k_seam_cols<<<g2d, 256, 0, st>>>(srow, mask1, mask2, seam, ctl, k25, gm0, cw, ch);
+    k_seam_cols<<<dim3(ceil_div(cw, SC_T), ceil_div(ch, SC_L)), SC_T, 0, st>>>(srow, mask1, mask2, k25, gm0, cw, ch);
     PYSIFT_LAUNCH_CHECK("k_seam_cols");
     // Gaussian pyramid of the seam mask, then join the image pyramids
     {
@@ -1451,9 +1599,13 @@ int pysift_blend_multiband(const void* image1, int32_t image1_f32, const uint8_t
     }
     PYSIFT_LAUNCH_CHECK("k_blend_reconstruct");
     // level 0: Laplacian blend, last reconstruction step and paste
-    k_blend_final<<<g2d, 256, 0, st>>>(src, gm0, n_levels > 1 ? bwp<float>(ws, l.off_g1[1]) : nullptr,
-                                       n_levels > 1 ? bwp<float>(ws, l.off_g2[1]) : nullptr, res, rh, rw, ch, cw,
-                                       zoom_factors(rh, rw, ch, cw), pano, both, blended, seam_rmse);
+    const dim3 gf(ceil_div(cw, BF_T), ceil_div(ch, BF_R));
+    const float* g1n = n_levels > 1 ? bwp<float>(ws, l.off_g1[1]) : nullptr;
+    const float* g2n = n_levels > 1 ? bwp<float>(ws, l.off_g2[1]) : nullptr;
+    const ZoomF zf = zoom_factors(rh, rw, ch, cw);
+    auto final_kernel = n_levels > 1 ? (image1_f32 ? k_blend_final<false, true> : k_blend_final<true, true>)
+                                     : (image1_f32 ? k_blend_final<false, false> : k_blend_final<true, false>);
+    final_kernel<<<gf, BF_T, 0, st>>>(src, gm0, g1n, g2n, res, rh, rw, ch, cw, zf, pano, both, blended, seam_rmse);
     PYSIFT_LAUNCH_CHECK("k_blend_final");
     return PYSIFT_OK;
 }

@@ -176,6 +176,37 @@ def test_blend_seam_band_edges(rows, lo, na, gap, nb):
         assert np.array_equal(pano, ref)
 
 
+@pytest.mark.parametrize("ch,cw", [(12, 127), (13, 130), (16, 128), (17, 129), (31, 257), (32, 513), (33, 512),
+                                   (44, 520), (45, 60), (64, 90), (65, 385)])
+def test_blend_strip_edges(ch, cw):
+    """The seam-mask blur (32-row strips, 512-column row blocks, only the
+    overlap's box and 12 rows around it) and the level-0 blend (16-row strips
+    of 128 columns) at the ends of their tiles, with the overlap inside the
+    canvas, for uint8 and float32 images and for one level and several."""
+    import torch
+    from oracle import blend_oracle as bo
+    from pysift_b200 import blend
+    rng = np.random.default_rng(ch * 1000 + cw)
+    yy, xx = np.mgrid[0:ch, 0:cw]
+    m1 = (xx < cw * 0.6) & (yy < ch - 1)
+    m2 = (xx >= cw * 0.4) & (yy >= 1)
+    w1 = rng.integers(0, 256, (ch, cw, 3), dtype=np.uint8)
+    c2 = rng.integers(0, 256, (ch, cw, 3), dtype=np.uint8)
+    w1[~m1] = 0
+    c2[~m2] = 0
+    wf = (w1 + rng.uniform(-3, 3, w1.shape)).astype(np.float32)
+    t = lambda a: torch.from_numpy(np.ascontiguousarray(a)).cuda()
+    for img in (w1, wf):
+        for n_levels in (1, 2, 4):
+            out = torch.empty((ch, cw, 3), dtype=torch.float32, device="cuda")
+            pano, both, _, _ = blend.blend_multiband(t(img), t(m1.astype(np.uint8)), t(c2), t(m2.astype(np.uint8)),
+                                                     n_levels, blended=out)
+            ref, ref_both, _ = bo.blend_core(img.astype(np.float32), m1, c2.astype(np.float32), m2, n_levels)
+            assert np.array_equal(both.cpu().numpy().astype(bool), ref_both)
+            assert np.array_equal(pano.cpu().numpy(), bo.paste(ref, ref_both))
+            assert np.array_equal(pano.cpu().numpy(), bo.paste(out.cpu().numpy(), ref_both))
+
+
 def test_blend_no_overlap_and_edges():
     """No overlap (no gain, no seam), an overlap of one column and one of one row."""
     from oracle import blend_oracle as bo
