@@ -31,10 +31,10 @@
 //             The canonical similarity is the fp16 rounding (nearest, ties to
 //             even) of the EXACT dot product.  The tensor cores' fp32
 //             accumulation is within e = D 2^-21 |a| max|b| of it.  The merge
-//             recomputes every column of the two best chunks exactly (float64
-//             sums of the exact fp16 products: every partial sum is a multiple
-//             of 2^-48 below 2^5 in magnitude for rows of norm <= 1, hence
-//             exact in any order) and accepts the row when no column of the
+//             recomputes the largest columns of the two best chunks exactly
+//             (float64 sums of the exact fp16 products: every partial sum is a
+//             multiple of 2^-48 below 2^5 in magnitude for rows of norm <= 1,
+//             hence exact in any order) and accepts the row when no column of the
 //             other chunks can reach the exact second value
 //             (fp16(third chunk key + e) <= second, and < best); the other rows
 //             are recomputed over every column by k_match_recheck_f16.
@@ -58,6 +58,7 @@
 #include <cstdint>
 
 #include "common.cuh"
+#include <cooperative_groups.h>
 #include <cuda_fp8.h>
 
 namespace pysift {
@@ -616,7 +617,6 @@ struct MergeArgs {
     MergeSide side[2];
     int blocks0;
     float ratio_sq;
-    int D;
     const int* error;
 };
 
@@ -680,7 +680,8 @@ __device__ __forceinline__ Top3 shfl_xor_top3(const Top3& t, int o) {
 
 // The segments of one row merged by the whole warp: lane s loads parts s,
 // s + 32, ... (all loads in flight at once), then a butterfly of top3_merge
-// leaves the union in every lane.  The union's two first entries in
+// over the lanes that hold any (a scan usually has 1 to 4 segments) and a
+// broadcast leave the union in every lane.  The union's two first entries in
 // (key desc, first column asc) order and its third key do not depend on the
 // order of the merges.
 __device__ __forceinline__ Top3 merge_parts(const Top3* __restrict__ part, int i, int nseg) {
@@ -688,17 +689,53 @@ __device__ __forceinline__ Top3 merge_parts(const Top3* __restrict__ part, int i
     Top3 a;
     top3_init(a);
     for (int s_ = lane; s_ < nseg; s_ += 32) top3_merge(a, part[(size_t)i * nseg + s_]);
-    for (int o = 16; o > 0; o >>= 1) top3_merge(a, shfl_xor_top3(a, o));
+    int o = 1;
+    for (; o < min(nseg, 32); o <<= 1) top3_merge(a, shfl_xor_top3(a, o));
+    if (o < 32) {
+        a.k1 = __shfl_sync(FULL_MASK, a.k1, 0);
+        a.k2 = __shfl_sync(FULL_MASK, a.k2, 0);
+        a.k3 = __shfl_sync(FULL_MASK, a.k3, 0);
+        a.i1 = __shfl_sync(FULL_MASK, a.i1, 0);
+        a.i2 = __shfl_sync(FULL_MASK, a.i2, 0);
+    }
     return a;
+}
+
+// Rows of a 32-column chunk read by a warp with consecutive lanes on one row:
+// LPR lanes hold a row's 16-byte words, so a load instruction covers 32 / LPR
+// rows of a few cache lines.  A row a lane touches 32 lines each time, which
+// bound both merges: 24.8 -> 11.7 us for two 8192x128 uint8 sets.  get(j, row) is the lane's share of row j's sum;
+// the LPR shares of each row are then added by halves across the lanes, so
+// that lane l ends with the whole sum of row chunk_row<LPR>(l).
+template <int LPR>
+__device__ __forceinline__ int chunk_row(int lane) {
+    return (lane & (LPR - 1)) * (32 / LPR) + lane / LPR;
+}
+template <int LPR, typename T, typename F>
+__device__ __forceinline__ T chunk_sums(int lane, F&& get) {
+    T v[LPR];
+#pragma unroll
+    for (int k = 0; k < LPR; ++k) v[k] = get(k * (32 / LPR) + lane / LPR);
+#pragma unroll
+    for (int h = LPR / 2; h > 0; h >>= 1) {
+        const bool up = (lane & h) != 0;
+#pragma unroll
+        for (int j = 0; j < h; ++j) {
+            const T give = up ? v[j] : v[j + h], keep = up ? v[j + h] : v[j];
+            v[j] = keep + __shfl_xor_sync(FULL_MASK, give, h);
+        }
+    }
+    return v[0];
 }
 
 // DIST_U8 / SPLIT_FP8: the best chunk of row i (the first chunk holding
 // the row's largest key) recomputed exactly from the uint8 rows, one warp per
-// row and one column per lane: the best column is the first in that chunk
+// row: the best column is the first in that chunk
 // with the chunk's key, and the second key the larger of the chunk's second
 // and the other chunks' largest (a.k2).  Keys 2 a.b - |b|^2 are exact
 // integers on both sides, so the recomputed maximum equals a.k1; a mismatch
 // (or a scan that gave up) leaves the row without a match.
+template <int D>
 __global__ void k_match_merge_u8(const __grid_constant__ MergeArgs m) {
     const int sd = (int)blockIdx.x >= m.blocks0 ? 1 : 0;
     const MergeSide& z = m.side[sd];
@@ -706,7 +743,7 @@ __global__ void k_match_merge_u8(const __grid_constant__ MergeArgs m) {
     const uint8_t* __restrict__ t = z.t;
     const int* __restrict__ norm_q = z.norm_q;
     const int* __restrict__ norm_t = z.norm_t;
-    const int n_t = z.n_t, D = m.D;
+    const int n_t = z.n_t;
     const float ratio_sq = m.ratio_sq;
     int* __restrict__ best = z.best;
     int* __restrict__ pass = z.pass;
@@ -718,19 +755,19 @@ __global__ void k_match_merge_u8(const __grid_constant__ MergeArgs m) {
     const bool bad = *m.error || !(a.k1 > -INFINITY) || a.i1 < 0 || a.i1 >= n_t;
     unsigned long long kb = 0, ks = 0;
     if (!bad) {
-        const int c = a.i1 + lane;
+        constexpr int LPR = D / 16;
+        const uint4 x = *reinterpret_cast<const uint4*>(q + (size_t)i * D + (lane & (LPR - 1)) * 16);
+        const int dot = chunk_sums<LPR, int>(lane, [&](int j) {
+            const size_t r = (size_t)min(a.i1 + j, n_t - 1);
+            const uint4 y = *reinterpret_cast<const uint4*>(t + r * D + (lane & (LPR - 1)) * 16);
+            unsigned acc = __dp4a(x.x, y.x, 0u);
+            acc = __dp4a(x.y, y.y, acc);
+            acc = __dp4a(x.z, y.z, acc);
+            return (int)__dp4a(x.w, y.w, acc);
+        });
+        const int c = a.i1 + chunk_row<LPR>(lane);
         if (c < n_t) {
-            const uint4* pq = reinterpret_cast<const uint4*>(q + (size_t)i * D);
-            const uint4* pt = reinterpret_cast<const uint4*>(t + (size_t)c * D);
-            unsigned acc = 0;
-            for (int w = 0; w < D / 16; ++w) {
-                const uint4 x = pq[w], y = pt[w];
-                acc = __dp4a(x.x, y.x, acc);
-                acc = __dp4a(x.y, y.y, acc);
-                acc = __dp4a(x.z, y.z, acc);
-                acc = __dp4a(x.w, y.w, acc);
-            }
-            const int key = 2 * (int)acc - norm_t[c];  // > -2^24
+            const int key = 2 * dot - norm_t[c];  // > -2^24
             // order-preserving bits of the key above the complemented column
             kb = ((unsigned long long)((unsigned)key ^ 0x80000000u) << 32) | (0xFFFFFFFFu - (unsigned)c);
         }
@@ -833,22 +870,147 @@ __device__ __forceinline__ int sim_key_column(unsigned long long k) {
     return (int)(0xFFFFFFFFu - (unsigned)(k & 0xFFFFFFFFu));
 }
 
+// The two largest keys of some columns of a row, one warp.  The exact value
+// takes a conversion to float64 for every product, 16 a clock on an SM, and
+// only the two largest count: each chunk's columns are first formed in fp32
+// (coalesced, within e of the exact value, see the header), and only those
+// within `margin` of the second largest seen so far are formed exactly, by the
+// whole warp.  A column left out is below the second largest by more than the
+// width of its fp16 interval, so it changes neither the second value nor a tie
+// of the best (width: 2^-10 of the value, taken twice; and 2^-23 for
+// subnormals).  The sums are exact in any order while |a| max|b| <= 16 (every
+// partial sum a multiple of 2^-48 below 2^5); rows beyond that take the
+// one-column-a-lane sums of dot_f16_exact.  Merge of 7919 x 5003 rows of 64:
+// 45 -> 25 us, now bound by the chain of loads (parts, chunks, candidates) and
+// ~1000 instructions a row.
+template <int D>
+struct F16Row {
+    const __half* q;
+    const __half* t;
+    int n_t, lane;
+    bool fast;
+    float e2;       // twice the fp32 error bound
+    float x[8];     // the lane's 16 bytes of the query row
+    float m1 = -INFINITY, m2 = -INFINITY;
+    unsigned long long kb = 0, ks = 0;  // best and second keys; 0 = none
+    static constexpr int LPR = D / 8;
+
+    __device__ __forceinline__ F16Row(const MergeSide& z, int i)
+        : q(reinterpret_cast<const __half*>(z.q) + (size_t)i * D), t(reinterpret_cast<const __half*>(z.t)), n_t(z.n_t),
+          lane(threadIdx.x & 31) {
+        const float bound = z.fnorm_q[i] * __uint_as_float(*z.maxnorm_t);
+        fast = bound <= 16.0f;
+        e2 = (float)D * 0x1p-20f * bound;
+        const uint4 w = *reinterpret_cast<const uint4*>(q + (lane & (LPR - 1)) * 8);
+        unpack(w, x);
+    }
+    static __device__ __forceinline__ void unpack(const uint4& w, float (&f)[8]) {
+        const __half2* h = reinterpret_cast<const __half2*>(&w);
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+            const float2 v = __half22float2(h[k]);
+            f[2 * k] = v.x;
+            f[2 * k + 1] = v.y;
+        }
+    }
+    __device__ __forceinline__ void take(unsigned long long key) {
+        ks = max(ks, min(kb, key));
+        kb = max(kb, key);
+    }
+    // the fp32 value of column c0 + chunk_row<LPR>(lane)
+    __device__ __forceinline__ float rough(int c0) const {
+        return chunk_sums<LPR, float>(lane, [&](int j) {
+            const size_t r = (size_t)min(c0 + j, n_t - 1);
+            float y[8];
+            unpack(*reinterpret_cast<const uint4*>(t + r * D + (lane & (LPR - 1)) * 8), y);
+            float s = 0.0f;
+#pragma unroll
+            for (int k = 0; k < 8; ++k) s = __fmaf_rn(x[k], y[k], s);
+            return s;
+        });
+    }
+    __device__ __forceinline__ void exact(int c) {
+        double s = 0.0;
+        const __half2* a = reinterpret_cast<const __half2*>(q);
+        const __half2* b = reinterpret_cast<const __half2*>(t + (size_t)c * D);
+#pragma unroll
+        for (int k = 0; k < D / 64; ++k) {
+            const float2 u = __half22float2(a[k * 32 + lane]), v = __half22float2(b[k * 32 + lane]);
+            s += (double)__fmul_rn(u.x, v.x);
+            s += (double)__fmul_rn(u.y, v.y);
+        }
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(FULL_MASK, s, o);
+        take(sim_key(f16_round_f64(s), c));
+    }
+    // N chunks of 32 columns starting at c0[.] (>= n_t: none), N * 32 columns
+    // or fewer; the keys are warp-uniform when fast, a lane's own otherwise
+    template <int N>
+    __device__ __forceinline__ void chunks(const int (&c0)[N]) {
+        if (!fast) {
+#pragma unroll
+            for (int k = 0; k < N; ++k)
+                if (c0[k] < n_t && c0[k] + lane < n_t)
+                    take(sim_key(f16_round_f64(dot_f16_exact(q, t + (size_t)(c0[k] + lane) * D, D)), c0[k] + lane));
+            return;
+        }
+        float v[N];
+        bool in[N];
+#pragma unroll
+        for (int k = 0; k < N; ++k) {
+            in[k] = false;
+            v[k] = -INFINITY;
+            if (c0[k] < n_t) {
+                v[k] = rough(c0[k]);
+                in[k] = c0[k] + chunk_row<LPR>(lane) < n_t;
+            }
+        }
+        float b1 = -INFINITY, b2 = -INFINITY;
+#pragma unroll
+        for (int k = 0; k < N; ++k) {
+            const float w = in[k] ? v[k] : -INFINITY;
+            b2 = fmaxf(b2, fminf(b1, w));
+            b1 = fmaxf(b1, w);
+        }
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) {
+            const float o1 = __shfl_xor_sync(FULL_MASK, b1, o), o2 = __shfl_xor_sync(FULL_MASK, b2, o);
+            b2 = fmaxf(fmaxf(b2, o2), fminf(b1, o1));
+            b1 = fmaxf(b1, o1);
+        }
+        m2 = fmaxf(fmaxf(m2, b2), fminf(m1, b1));
+        m1 = fmaxf(m1, b1);
+        const float margin = e2 + (0x1p-9f * (fabsf(m1) + e2) + 0x1p-23f);
+#pragma unroll
+        for (int k = 0; k < N; ++k) {
+            unsigned todo = __ballot_sync(FULL_MASK, in[k] && !(v[k] < m2 - margin));
+            while (todo) {
+                const int l = __ffs(todo) - 1;
+                todo &= todo - 1;
+                exact(c0[k] + chunk_row<LPR>(l));
+            }
+        }
+    }
+    // the two largest over the warp
+    __device__ __forceinline__ void join() {
+        if (!fast) warp_top2_u64(kb, ks);
+    }
+};
+
 // Merge the chunk-level segments of one SIM_F16 scan (in segment order) and
-// settle the row from its two best chunks: every column of both is
-// recomputed exactly (one warp per row, a column of each chunk per lane),
-// giving the exact best F1 (lowest index on ties) and second F2 among them.
-// Every column of the other chunks has an fp32 value <= k3 (the third chunk's
-// largest), so its exact value is <= k3 + e and its fp16 similarity
-// <= U = fp16(k3 + e); the row is settled when U <= F2 and U < F1 (a column
-// tying F1 could have a lower index).  Unsettled rows are appended to
-// `recheck` (their order there does not matter: each row's result is
+// settle the row from its two best chunks (one warp per row): the two largest
+// of their columns give the exact best F1 (lowest index on ties) and second F2
+// among them.  Every column of the other chunks has an fp32 value <= k3 (the
+// third chunk's largest), so its exact value is <= k3 + e and its fp16
+// similarity <= U = fp16(k3 + e); the row is settled when U <= F2 and U < F1
+// (a column tying F1 could have a lower index).  Unsettled rows are appended
+// to `recheck` (their order there does not matter: each row's result is
 // computed on its own).
+template <int D>
 __global__ void k_match_merge_f16(const __grid_constant__ MergeArgs m) {
     const int sd = (int)blockIdx.x >= m.blocks0 ? 1 : 0;
     const MergeSide& z = m.side[sd];
-    const __half* __restrict__ q = reinterpret_cast<const __half*>(z.q);
-    const __half* __restrict__ t = reinterpret_cast<const __half*>(z.t);
-    const int n_t = z.n_t, D = m.D;
+    const int n_t = z.n_t;
     const float ratio_sq = m.ratio_sq;
     int* __restrict__ best = z.best;
     int* __restrict__ pass = z.pass;
@@ -868,19 +1030,12 @@ __global__ void k_match_merge_f16(const __grid_constant__ MergeArgs m) {
         }
         return;
     }
-    const __half* qi = q + (size_t)i * D;
-    unsigned long long kb = 0, ks = 0;
-    const int ca = a.i1 + lane, cb = a.i2 + lane;
-    if (ca < n_t) kb = sim_key(f16_round_f64(dot_f16_exact(qi, t + (size_t)ca * D, D)), ca);
-    if (c2 && cb < n_t) {
-        const unsigned long long k = sim_key(f16_round_f64(dot_f16_exact(qi, t + (size_t)cb * D, D)), cb);
-        ks = min(kb, k);
-        kb = max(kb, k);
-    }
-    warp_top2_u64(kb, ks);
+    F16Row<D> row(z, i);
+    row.chunks({a.i1, c2 ? a.i2 : n_t});
+    row.join();
     if (lane != 0) return;
-    const float f1 = sim_key_value(kb);
-    const float f2 = ks ? sim_key_value(ks) : -INFINITY;
+    const float f1 = sim_key_value(row.kb);
+    const float f2 = row.ks ? sim_key_value(row.ks) : -INFINITY;
     if (a.k3 > -INFINITY) {
         const double e = (double)D * 0x1p-21 * (double)z.fnorm_q[i] * (double)__uint_as_float(*z.maxnorm_t);
         const float u = f16_round_f64((double)a.k3 + e);
@@ -889,60 +1044,66 @@ __global__ void k_match_merge_f16(const __grid_constant__ MergeArgs m) {
             return;
         }
     }
-    finish_f16_row(i, f1, f2, sim_key_column(kb), ratio_sq, best, pass, dist);
+    finish_f16_row(i, f1, f2, sim_key_column(row.kb), ratio_sq, best, pass, dist);
 }
 
 // Rows the merge could not settle: the exact fp16 similarity against every
-// column, top-2 by (similarity desc, index asc).  One CTA per row (grid
-// stride over both directions' lists); keys pack the order-preserving bits
-// of the similarity above the complemented column index, so the integer
-// maximum is the best with the lowest index.
-constexpr int RECHECK_T = 1024;
+// column, top-2 by (similarity desc, index asc).  One cluster of RECHECK_C
+// CTAs per row (stride over both directions' lists): there are usually few
+// rows, so what counts is the chain of one row.  Its warps take chunks in
+// turn, two at a time; keys pack the order-preserving bits of the similarity
+// above the complemented column index, so the integer maximum is the best with
+// the lowest index.  Sets of 8000 x 64 with a few such rows: 40 -> 7 us
+// against one CTA a row that formed every column in float64.
+constexpr int RECHECK_T = 512, RECHECK_C = 8;
 
-__global__ void __launch_bounds__(RECHECK_T) k_match_recheck_f16(const int* __restrict__ list0, const int* __restrict__ list1,
-                                                           const int* __restrict__ counts, const __half* __restrict__ a,
-                                                           int n1, const __half* __restrict__ b, int n2, int D,
-                                                           float ratio_sq, int* __restrict__ fbest,
-                                                           int* __restrict__ fpass, float* __restrict__ fdist,
-                                                           int* __restrict__ bbest, int* __restrict__ bpass,
-                                                           float* __restrict__ bdist) {
-    __shared__ __align__(16) __half qrow[128];
+template <int D>
+__global__ void __cluster_dims__(RECHECK_C, 1, 1) __launch_bounds__(RECHECK_T)
+    k_match_recheck_f16(const __grid_constant__ MergeArgs m) {
     __shared__ unsigned long long s_b[RECHECK_T / 32], s_s[RECHECK_T / 32];
-    const int c0 = counts[0], call = c0 + counts[1];
+    __shared__ unsigned long long s_cta[2];
+    namespace cg = cooperative_groups;
+    cg::cluster_group cluster = cg::this_cluster();
+    const int rank = (int)cluster.block_rank();
+    const int c0 = *m.side[0].n_recheck, call = c0 + *m.side[1].n_recheck;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    for (int v = blockIdx.x; v < call; v += gridDim.x) {
-        const bool fwd = v < c0;
-        const int i = fwd ? list0[v] : list1[v - c0];
-        const __half* t = fwd ? b : a;
-        const int nt = fwd ? n2 : n1;
-        if ((int)threadIdx.x < D) qrow[threadIdx.x] = (fwd ? a : b)[(size_t)i * D + threadIdx.x];
-        __syncthreads();
-        unsigned long long kb = 0, ks = 0;  // best and second keys; 0 = none
-        for (int j = threadIdx.x; j < nt; j += blockDim.x) {
-            const unsigned long long key = sim_key(f16_round_f64(dot_f16_exact(qrow, t + (size_t)j * D, D)), j);
-            ks = max(ks, min(kb, key));
-            kb = max(kb, key);
-        }
-        warp_top2_u64(kb, ks);
+    for (int v = blockIdx.x / RECHECK_C; v < call; v += gridDim.x / RECHECK_C) {
+        const MergeSide& z = m.side[v < c0 ? 0 : 1];
+        const int i = v < c0 ? z.recheck[v] : z.recheck[v - c0];
+        F16Row<D> row(z, i);
+        constexpr int STEP = RECHECK_C * RECHECK_T;
+        for (int c = rank * RECHECK_T + warp * 32; c < z.n_t; c += 2 * STEP) row.chunks({c, c + STEP});
+        row.join();
         if (lane == 0) {
-            s_b[warp] = kb;
-            s_s[warp] = ks;
+            s_b[warp] = row.kb;
+            s_s[warp] = row.ks;
         }
         __syncthreads();
-        if (threadIdx.x == 0) {
-            for (int w = 1; w < (int)(blockDim.x >> 5); ++w) {
-                ks = max(max(ks, s_s[w]), min(kb, s_b[w]));
-                kb = max(kb, s_b[w]);
+        if (warp == 0) {
+            unsigned long long kb = 0, ks = 0;
+            if (lane < RECHECK_T / 32) {
+                kb = s_b[lane];
+                ks = s_s[lane];
+            }
+            warp_top2_u64(kb, ks);
+            if (lane == 0) {
+                s_cta[0] = kb;
+                s_cta[1] = ks;
+            }
+        }
+        cluster.sync();
+        if (rank == 0 && threadIdx.x == 0) {
+            unsigned long long kb = s_cta[0], ks = s_cta[1];
+            for (int w = 1; w < RECHECK_C; ++w) {
+                const unsigned long long* o = cluster.map_shared_rank(s_cta, w);
+                ks = max(max(ks, o[1]), min(kb, o[0]));
+                kb = max(kb, o[0]);
             }
             const float f1 = sim_key_value(kb);
             const float f2 = ks ? sim_key_value(ks) : -INFINITY;
-            const int c1 = sim_key_column(kb);
-            if (fwd)
-                finish_f16_row(i, f1, f2, c1, ratio_sq, fbest, fpass, fdist);
-            else
-                finish_f16_row(i, f1, f2, c1, ratio_sq, bbest, bpass, bdist);
+            finish_f16_row(i, f1, f2, sim_key_column(kb), m.ratio_sq, z.best, z.pass, z.dist);
         }
-        __syncthreads();
+        cluster.sync();
     }
 }
 
@@ -1258,8 +1419,6 @@ static int run_match(int mode, const uint8_t* rows_a, int n1, const uint8_t* row
                      const float* sb = nullptr) {
     int* ctl = wsp<int>(ws, l.off_ctl);
     int* err = ctl;
-    const __half* ha = reinterpret_cast<const __half*>(rows_a);
-    const __half* hb = reinterpret_cast<const __half*>(rows_b);
     unsigned* maxnorm = reinterpret_cast<unsigned*>(ctl + 3);
     uint8_t* qa = wsp<uint8_t>(ws, l.off_qa);
     uint8_t* ta = wsp<uint8_t>(ws, l.off_ta);
@@ -1313,20 +1472,20 @@ static int run_match(int mode, const uint8_t* rows_a, int n1, const uint8_t* row
     m.side[1] = MergeSide{s.side[1].part, n2, s.side[1].nseg, rows_b, rows_a, n1, nb, na, hna ? hna + n1 : nullptr,
                           maxnorm, bbest, bpass, bdist, wsp<int>(ws, l.off_rl1), ctl + 2};
     m.ratio_sq = ratio_sq;
-    m.D = D;
     m.error = err;
     const int per = mode == SIM_I8 ? 256 : 8;  // rows of a block: one a thread, or one a warp
     m.blocks0 = ceil_div(n1, per);
     const int blocks = m.blocks0 + ceil_div(n2, per);
-    if (mode == SIM_F16) k_match_merge_f16<<<blocks, 256, 0, st>>>(m);
-    else if (mode == SIM_I8) k_match_merge_i8<<<blocks, 256, 0, st>>>(m);
-    else k_match_merge_u8<<<blocks, 256, 0, st>>>(m);
-    PYSIFT_LAUNCH_CHECK("k_match_merge");
     if (mode == SIM_F16) {
-        k_match_recheck_f16<<<sm_count(), RECHECK_T, 0, st>>>(wsp<int>(ws, l.off_rl0), wsp<int>(ws, l.off_rl1), ctl + 1,
-                                                             ha, n1, hb, n2, D, ratio_sq, fbest, fpass, fdist, bbest,
-                                                             bpass, bdist);
+        (D == 64 ? k_match_merge_f16<64> : k_match_merge_f16<128>)<<<blocks, 256, 0, st>>>(m);
+        PYSIFT_LAUNCH_CHECK("k_match_merge_f16");
+        (D == 64 ? k_match_recheck_f16<64> : k_match_recheck_f16<128>)<<<2 * sm_count() / RECHECK_C * RECHECK_C, RECHECK_T, 0,
+                                                                                    st>>>(m);
         PYSIFT_LAUNCH_CHECK("k_match_recheck_f16");
+    } else {
+        if (mode == SIM_I8) k_match_merge_i8<<<blocks, 256, 0, st>>>(m);
+        else (D == 64 ? k_match_merge_u8<64> : k_match_merge_u8<128>)<<<blocks, 256, 0, st>>>(m);
+        PYSIFT_LAUNCH_CHECK("k_match_merge");
     }
     k_match_mutual<<<1, 1024, 0, st>>>(fbest, fpass, fdist, bbest, bpass, n1, reinterpret_cast<int2*>(pairs), pdist,
                                        count);

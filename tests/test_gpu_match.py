@@ -102,6 +102,22 @@ def test_fp16_reference_mode_ties_and_rechecks():
     assert rechecked[0] >= np.count_nonzero(fb[:300] == np.arange(300))
 
 
+@pytest.mark.parametrize("n1,n2,D", [(40, 31, 64), (33, 33, 128), (70, 65, 64), (9, 2100, 128)])
+@pytest.mark.parametrize("scale", [0.125, 1.0, 2.0, 4.0, 8.0])
+def test_fp16_row_norms_and_ties_within_a_chunk(n1, n2, D, scale):
+    """Rows scaled by a power of two (exact in fp16), so that |a| max|b| lies on
+    both sides of the bound up to which the candidate columns are picked by
+    their fp32 value, with copies of a train row in the same 32-column chunk,
+    in the next one, and zero rows."""
+    xh, yh = _unit_f16_sets(n1, n2, D, seed=n1 + n2)
+    yh[3], yh[7] = yh[5], yh[5]
+    if n2 > 32:
+        yh[32] = yh[5]
+    yh[n2 - 1] = 0
+    xh[n1 - 1] = 0
+    _fp16_match_and_check((xh * np.float16(scale)).astype(np.float16), (yh * np.float16(scale)).astype(np.float16))
+
+
 def test_fp16_reference_mode_near_ties_of_the_rounding():
     """Rows built so that the best and second similarities sit within an
     fp32 accumulation error of an fp16 rounding boundary (two train rows that
