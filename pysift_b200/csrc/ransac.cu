@@ -59,8 +59,8 @@ __device__ __forceinline__ double ransac_exp(double x) {
 }
 
 // NV fixed-order pairwise trees at once, the same pairs as block_tree_sum
-// (t += t + s for s = 128, 64, ..., 1): the three top levels in shared
-// memory, the rest with warp shuffles.  out (shared) receives the NV sums.
+// (t += t + s for s = 128, 64, ..., 1): the two top levels in shared
+// memory, the rest a warp a value, with shuffles.  out (shared) receives the NV sums.
 template <int NV>
 __device__ __forceinline__ void block_tree_sums(const double (&v)[NV], double (*sh)[RT], double* out) {
     const int tid = threadIdx.x;
@@ -77,13 +77,15 @@ __device__ __forceinline__ void block_tree_sums(const double (&v)[NV], double (*
         for (int u = 0; u < NV; ++u) sh[u][tid] = sh[u][tid] + sh[u][tid + 64];
     }
     __syncthreads();
-    if (tid < 32) {
+    const int lane = tid & 31;
 #pragma unroll
-        for (int u = 0; u < NV; ++u) {
-            double x = sh[u][tid] + sh[u][tid + 32];
+    for (int u0 = 0; u0 < NV; u0 += RT / 32) {
+        const int u = u0 + (tid >> 5);
+        if (u < NV) {
+            double x = sh[u][lane] + sh[u][lane + 32];
 #pragma unroll
             for (int s = 16; s > 0; s >>= 1) x = x + __shfl_down_sync(FULL_MASK, x, s);
-            if (tid == 0) out[u] = x;
+            if (lane == 0) out[u] = x;
         }
     }
     __syncthreads();
@@ -356,93 +358,136 @@ __global__ void __launch_bounds__(256) k_ransac_hyp(const RansacArgs args) {
 }
 
 // Smallest-eigenvalue eigenvector of the symmetric 9x9 M (row-major, shared
-// memory) by parallel Jacobi, run by warp 0 (V: shared 9x9 eigenvectors).
+// memory) by parallel Jacobi, run by warp 0 (v: the eigenvector, shared).
 // Round-robin ordering of the 36 index pairs: round r = 0..8 rotates the 4
 // disjoint pairs {(r+i) mod 9, (r-i) mod 9}, i = 1..4 (p < q); index r rests.
 // The 4 angles of a round come from the matrix at the start of the round,
 // then all column rotations are applied, then all row rotations (exact, as
 // the pairs are disjoint).  Only pairs with |a_pq| > tol = 2^-52 trace
 // (the trace summed in index order) rotate; sweeps stop once no upper
-// off-diagonal element exceeds tol, at 15 at most.  Returns the index of the
-// smallest diagonal element (lowest on ties).
-__device__ int jacobi9_smallest(double (*M)[9], double (*V)[9]) {
-    __shared__ double s_cs[4][2];
-    __shared__ int s_pq[4][2];
-    __shared__ int s_act[4];
-    __shared__ int s_best;
+// off-diagonal element exceeds tol, at 15 at most.  The eigenvector is the one
+// of the smallest diagonal element (lowest index on ties).
+// A sweep is a chain of 9 rounds and a round one of two square roots and three
+// divisions, so a round holds nothing else that can be moved: lane 5 i + j
+// owns the 2x2 block of pair i's rows and pair j's columns (4: the resting
+// index), forms pair j's angle itself, takes pair i's by shuffle, and applies
+// both rotations in registers, with one barrier of the warp a round.  The
+// rotations are kept (`rot`, 15 x 9 rounds of 4, and a bit mask a round) and
+// applied to the eigenvector rows at the end, a row a lane.  1 / x is the
+// correctly rounded reciprocal, the same bits as the division.  A refit took
+// 53-59 us with the angles on 4 lanes and three passes over shared memory.
+constexpr int JACOBI_SWEEPS = 15;
+struct JacobiRot {
+    double2 cs[JACOBI_SWEEPS * 9][4];
+    int act[JACOBI_SWEEPS * 9];
+};
+
+// pair k of round r (k = 4: the resting index twice)
+__device__ __forceinline__ void jacobi_pair(int r, int k, int& p, int& q) {
+    int a = r + k + 1, b = r - k - 1;
+    a = a >= 9 ? a - 9 : a;
+    b = b < 0 ? b + 9 : b;
+    p = k == 4 ? r : min(a, b);
+    q = k == 4 ? r : max(a, b);
+}
+
+__device__ void jacobi9_smallest(double (*M)[9], JacobiRot& rot, double* v_out) {
     const int lane = threadIdx.x & 31;
     if (threadIdx.x < 32) {
-        for (int it = lane; it < 81; it += 32) V[it / 9][it % 9] = (it / 9 == it % 9) ? 1.0 : 0.0;
         double tr = 0.0;
         for (int k = 0; k < 9; ++k) tr = tr + M[k][k];
         const double tol = tr * 0x1p-52;
-        __syncwarp();
-        for (int sweep = 0; sweep < 15; ++sweep) {
-            // no upper off-diagonal element above tol -> converged
-            bool nz = false;
-            for (int it = lane; it < 81; it += 32) {
-                const int r = it / 9, c = it % 9;
-                if (c > r && fabs(M[r][c]) > tol) nz = true;
+        // the lane's upper off-diagonal elements (36 in all)
+        int er[2], ec[2];
+#pragma unroll
+        for (int u = 0; u < 2; ++u) {
+            int e = lane + 32 * u, r = 0;
+            if (e >= 36) e = lane;
+            while (e >= 8 - r) {
+                e -= 8 - r;
+                ++r;
             }
+            er[u] = r;
+            ec[u] = r + 1 + e;
+        }
+        const int i = min(lane / 5, 4), j = lane % 5;  // lanes 25.. repeat blocks 4, j
+        int n_rounds = 0;
+        __syncwarp();
+        for (int sweep = 0; sweep < JACOBI_SWEEPS; ++sweep) {
+            // no upper off-diagonal element above tol -> converged
+            const bool nz = fabs(M[er[0]][ec[0]]) > tol || fabs(M[er[1]][ec[1]]) > tol;
             if (!__any_sync(FULL_MASK, nz)) break;
-            for (int rnd = 0; rnd < 9; ++rnd) {
-                if (lane < 4) {
-                    const int a = (rnd + lane + 1) % 9, bb = (rnd + 9 - lane - 1) % 9;
-                    const int p = a < bb ? a : bb, q = a < bb ? bb : a;
-                    s_pq[lane][0] = p;
-                    s_pq[lane][1] = q;
-                    const double apq = M[p][q];
-                    int act = 0;
-                    if (fabs(apq) > tol) {
-                        const double app = M[p][p], aqq = M[q][q];
-                        const double theta = (aqq - app) / (2.0 * apq);
-                        const double tt = (theta >= 0.0 ? 1.0 : -1.0) / (fabs(theta) + sqrt(theta * theta + 1.0));
-                        const double c = 1.0 / sqrt(tt * tt + 1.0);
-                        s_cs[lane][0] = c;
-                        s_cs[lane][1] = tt * c;
-                        act = 1;
-                    }
-                    s_act[lane] = act;
+            for (int rnd = 0; rnd < 9; ++rnd, ++n_rounds) {
+                int pi, qi, pj, qj;
+                jacobi_pair(rnd, i, pi, qi);
+                jacobi_pair(rnd, j, pj, qj);
+                const double apq = M[pj][qj], app = M[pj][pj], aqq = M[qj][qj];
+                double pp = M[pi][pj], pq = M[pi][qj], qp = M[qi][pj], qq = M[qi][qj];
+                const bool act_j = j < 4 && fabs(apq) > tol;
+                const unsigned acts = __ballot_sync(FULL_MASK, act_j) & 15u;
+                if (lane == 0) rot.act[n_rounds] = (int)acts;
+                if (!acts) continue;
+                double c = 1.0, s = 0.0;
+                if (act_j) {
+                    const double theta = (aqq - app) / (2.0 * apq);
+                    const double d = __drcp_rn(fabs(theta) + sqrt(theta * theta + 1.0));
+                    const double tt = theta >= 0.0 ? d : -d;
+                    c = __drcp_rn(sqrt(tt * tt + 1.0));
+                    s = tt * c;
+                }
+                if (lane < 4) rot.cs[n_rounds][lane] = make_double2(c, s);
+                const double ci = __shfl_sync(FULL_MASK, c, i), si = __shfl_sync(FULL_MASK, s, i);
+                if (act_j) {
+                    const double a0 = c * pp - s * pq, a1 = s * pp + c * pq;
+                    const double b0 = c * qp - s * qq, b1 = s * qp + c * qq;
+                    pp = a0, pq = a1, qp = b0, qq = b1;
+                }
+                if (i < 4 && (acts >> i & 1u)) {
+                    const double a0 = ci * pp - si * qp, a1 = si * pp + ci * qp;
+                    const double b0 = ci * pq - si * qq, b1 = si * pq + ci * qq;
+                    pp = a0, qp = a1, pq = b0, qq = b1;
                 }
                 __syncwarp();
-                // column rotations: item = (pair j, row k)
-                for (int it = lane; it < 36; it += 32) {
-                    const int j = it / 9, k = it % 9;
-                    if (s_act[j]) {
-                        const int p = s_pq[j][0], q = s_pq[j][1];
-                        const double c = s_cs[j][0], s = s_cs[j][1];
-                        const double mkp = M[k][p], mkq = M[k][q];
-                        M[k][p] = c * mkp - s * mkq;
-                        M[k][q] = s * mkp + c * mkq;
-                    }
-                }
-                __syncwarp();
-                // row rotations and the eigenvector columns
-                for (int it = lane; it < 36; it += 32) {
-                    const int j = it / 9, k = it % 9;
-                    if (s_act[j]) {
-                        const int p = s_pq[j][0], q = s_pq[j][1];
-                        const double c = s_cs[j][0], s = s_cs[j][1];
-                        const double mpk = M[p][k], mqk = M[q][k];
-                        M[p][k] = c * mpk - s * mqk;
-                        M[q][k] = s * mpk + c * mqk;
-                        const double vkp = V[k][p], vkq = V[k][q];
-                        V[k][p] = c * vkp - s * vkq;
-                        V[k][q] = s * vkp + c * vkq;
-                    }
+                if (lane < 25) {
+                    M[pi][pj] = pp;
+                    M[pi][qj] = pq;
+                    M[qi][pj] = qp;
+                    M[qi][qj] = qq;
                 }
                 __syncwarp();
             }
         }
-        if (lane == 0) {
-            int best = 0;
-            for (int k = 1; k < 9; ++k)
-                if (M[k][k] < M[best][best]) best = k;
-            s_best = best;
+        int best = 0;
+        for (int k = 1; k < 9; ++k)
+            if (M[k][k] < M[best][best]) best = k;
+        if (lane < 9) {
+            double v[9];
+#pragma unroll
+            for (int k = 0; k < 9; ++k) v[k] = k == lane ? 1.0 : 0.0;
+            for (int n = 0; n < n_rounds; n += 9) {
+#pragma unroll
+                for (int rnd = 0; rnd < 9; ++rnd) {
+                    const int acts = rot.act[n + rnd];
+#pragma unroll
+                    for (int k = 0; k < 4; ++k) {
+                        const int a = (rnd + k + 1) % 9, b = (rnd + 8 - k) % 9;
+                        const int p = a < b ? a : b, q = a < b ? b : a;
+                        if (acts >> k & 1) {
+                            const double2 r = rot.cs[n + rnd][k];
+                            const double x = v[p], y = v[q];
+                            v[p] = r.x * x - r.y * y;
+                            v[q] = r.y * x + r.x * y;
+                        }
+                    }
+                }
+            }
+            double out = v[0];
+#pragma unroll
+            for (int k = 1; k < 9; ++k) out = best == k ? v[k] : out;
+            v_out[lane] = out;
         }
     }
     __syncthreads();
-    return s_best;
 }
 
 // Least-squares homography of the points idx[0..m): Hartley normalisation of
@@ -451,10 +496,11 @@ __device__ int jacobi9_smallest(double (*M)[9], double (*V)[9]) {
 // eigenvector by jacobi9_smallest, denormalised (pysift/core.py:2959-2981).
 __device__ void dlt_refit(const double* p1, const double* p2, const int* idx, int m, double* H, double* sh,
                           double* s_M) {
-    constexpr int NB = 9;  // tree sums run 9 at a time
+    constexpr int NB = 15;  // tree sums run 15 at a time
     __shared__ double s_part[NB][RT];
-    __shared__ double s_Mj[9][9], s_Vj[9][9];
-    __shared__ double s_red[NB];
+    __shared__ double s_Mj[9][9], s_v[9];
+    __shared__ double s_red[4];
+    __shared__ JacobiRot s_rot;
     Norm n1, n2;
     hartley2(p1, p2, idx, m, s_part, s_red, n1, n2);
     double acc[45];
@@ -492,10 +538,10 @@ __device__ void dlt_refit(const double* p1, const double* p2, const int* idx, in
         s_Mj[c][r] = s_M[it];
     }
     __syncthreads();
-    const int best = jacobi9_smallest(s_Mj, s_Vj);
+    jacobi9_smallest(s_Mj, s_rot, s_v);
     if (threadIdx.x == 0) {
         double hn[9], T1[9], T2inv[9];
-        for (int k = 0; k < 9; ++k) hn[k] = s_Vj[k][best];
+        for (int k = 0; k < 9; ++k) hn[k] = s_v[k];
         norm_mats(n1, n2, T1, T2inv);
         double t9[9];
         mat3_mul(T2inv, hn, t9);
