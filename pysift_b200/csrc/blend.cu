@@ -1206,6 +1206,29 @@ __global__ void __launch_bounds__(BF_T, 4) k_blend_final(const Level0 src, const
     }
 }
 
+// The start state of a blend in one launch (six memsets took longer than the
+// first kernel runs): the control block, the line flags and column ranges, and
+// the DP's directions.
+__global__ void __launch_bounds__(256) k_blend_clear(BlendCtl* ctl, int* __restrict__ rowf, int ch,
+                                                     int* __restrict__ colf, int* __restrict__ clo,
+                                                     int* __restrict__ chi, int cw, uint32_t* __restrict__ dir,
+                                                     long long dir_words) {
+    const long long i = (long long)blockIdx.x * 256 + threadIdx.x;
+    if (i < (long long)(sizeof(BlendCtl) / 4)) reinterpret_cast<uint32_t*>(ctl)[i] = 0;
+    if (i < ch) rowf[i] = 0;
+    if (i < cw) {
+        colf[i] = 0;
+        clo[i] = 0x7f7f7f7f;
+        chi[i] = -1;
+    }
+    // a block clears 4096 bytes of the directions
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+        const long long w = (long long)blockIdx.x * 1024 + k * 256 + threadIdx.x;
+        if (w < dir_words) dir[w] = 0;
+    }
+}
+
 __global__ void k_fill_i32(int* __restrict__ p, int n, int v) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i < n) p[i] = v;
@@ -1472,13 +1495,14 @@ int pysift_blend_multiband(const void* image1, int32_t image1_f32, const uint8_t
     int* rhi = bwp<int>(ws, l.off_rhi);
     int* clo = bwp<int>(ws, l.off_clo);
     int* chi = bwp<int>(ws, l.off_chi);
-    PYSIFT_CUDA_TRY(cudaMemsetAsync(ctl, 0, sizeof(BlendCtl), st));
-    PYSIFT_CUDA_TRY(cudaMemsetAsync(rowf, 0, (size_t)ch * 4, st));
-    PYSIFT_CUDA_TRY(cudaMemsetAsync(colf, 0, (size_t)cw * 4, st));
-    PYSIFT_CUDA_TRY(cudaMemsetAsync(clo, 0x7f, (size_t)cw * 4, st));
-    PYSIFT_CUDA_TRY(cudaMemsetAsync(chi, 0xff, (size_t)cw * 4, st));
     uint8_t* dir = bwp<uint8_t>(ws, l.off_dir);
-    PYSIFT_CUDA_TRY(cudaMemsetAsync(dir, 0, std::max(align_up(cw, 4) * ch, align_up(ch, 4) * cw), st));
+    static_assert(sizeof(BlendCtl) % 4 == 0, "cleared by words");
+    const long long dir_words = (long long)(std::max(align_up(cw, 4) * ch, align_up(ch, 4) * cw) / 4);
+    const long long n_clear = std::max({(long long)ceil_div(std::max(cw, ch), 256),
+                                        (long long)ceil_div((int)(sizeof(BlendCtl) / 4), 256), (dir_words + 1023) / 1024});
+    k_blend_clear<<<(unsigned int)n_clear, 256, 0, st>>>(ctl, rowf, ch, colf, clo, chi, cw,
+                                                         reinterpret_cast<uint32_t*>(dir), dir_words);
+    PYSIFT_LAUNCH_CHECK("k_blend_clear");
     GaussTaps w9;
     SeamTaps k25;
     for (int i = 0; i < 9; ++i) w9.w[i] = gauss_w9[i];

@@ -15,6 +15,8 @@
 //                   inner-rectangle crop (pysift/core.py:3627-3684)
 #include <cstdint>
 
+#include <algorithm>
+
 #include "common.cuh"
 
 namespace pysift {
@@ -263,9 +265,17 @@ __global__ void __launch_bounds__(256) k_warp_feather(const WarpArgs a) {
     for (int c = 0; c < 3; ++c) a.out[o + c] = res[c];
 }
 
-__global__ void k_fill_int(int* p, int n, int value) {
+// the extents of an empty coverage, all four arrays in one launch
+__global__ void k_extents_init(int* row_lo, int* row_hi, int n_rows, int* col_lo, int* col_hi, int n_cols) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < n) p[i] = value;
+    if (i < n_rows) {
+        row_lo[i] = 0x7fffffff;
+        row_hi[i] = -1;
+    }
+    if (i < n_cols) {
+        col_lo[i] = 0x7fffffff;
+        col_hi[i] = -1;
+    }
 }
 
 // rank[i] = #{j : (resp_j, j) precedes (resp_i, i)} under descending response,
@@ -414,14 +424,8 @@ int pysift_warp_feather(const uint8_t* img1, int32_t hs, int32_t ws, int32_t pit
     a.col_hi = col_hi;
     cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
     if (row_lo) {
-        k_fill_int<<<ceil_div(ch, 256), 256, 0, st>>>(row_lo, ch, 0x7fffffff);
-        PYSIFT_LAUNCH_CHECK("k_fill_int");
-        k_fill_int<<<ceil_div(ch, 256), 256, 0, st>>>(row_hi, ch, -1);
-        PYSIFT_LAUNCH_CHECK("k_fill_int");
-        k_fill_int<<<ceil_div(cw, 256), 256, 0, st>>>(col_lo, cw, 0x7fffffff);
-        PYSIFT_LAUNCH_CHECK("k_fill_int");
-        k_fill_int<<<ceil_div(cw, 256), 256, 0, st>>>(col_hi, cw, -1);
-        PYSIFT_LAUNCH_CHECK("k_fill_int");
+        k_extents_init<<<ceil_div(std::max(cw, ch), 256), 256, 0, st>>>(row_lo, row_hi, ch, col_lo, col_hi, cw);
+        PYSIFT_LAUNCH_CHECK("k_extents_init");
     }
     k_warp_feather<<<dim3(ceil_div(cw, 256), ch), 256, 0, st>>>(a);
     PYSIFT_LAUNCH_CHECK("k_warp_feather");

@@ -403,9 +403,9 @@ class GPUPyStitch:
 
     def _compose_enqueue(self, img1, img2, H, key="", max_canvas_px=400_000_000):
         """Canvas geometry on the host, then warp, composition and the
-        coverage extents on the current stream; the extents (and the seam
-        RMSE) are copied to pinned host memory (read them after the stream
-        has finished)."""
+        coverage extents on the current stream; the extents and the seam
+        RMSE are copied to pinned host memory (the extents can be read once
+        ext_done has passed, the RMSE after the stream has finished)."""
         hs, ws = img1.shape[:2]
         h2, w2 = img2.shape[:2]
         cw, ch, ox, oy = self._compute_canvas_size(img1.shape, img2.shape, H)
@@ -431,7 +431,14 @@ class GPUPyStitch:
                                                  float(np.float32(ox)), float(np.float32(oy)), iox, ioy, 1, *outs,
                                                  ext.data_ptr(), ext[ch:].data_ptr(), ext[2 * ch:].data_ptr(),
                                                  ext[2 * ch + cw:].data_ptr(), st), "pysift_warp_feather")
-        res = dict(out=out, canvas_w=cw, canvas_h=ch, ox=ox, oy=oy, seam_rmse_host=None)
+        # the crop depends on the extents alone: they go to the host while the
+        # images are blended
+        ext_host = torch.empty(ext.shape, dtype=torch.int32, pin_memory=True)
+        ext_host.copy_(ext, non_blocking=True)
+        ext_done = torch.cuda.Event()
+        ext_done.record()
+        res = dict(out=out, canvas_w=cw, canvas_h=ch, ox=ox, oy=oy, seam_rmse_host=None, ext_host=ext_host,
+                   ext_done=ext_done)
         if multiband:
             from . import blend as _blend
             canvas2 = self._dev.get(key + "canvas2", (ch, cw, 3), torch.uint8, dev)
@@ -447,9 +454,6 @@ class GPUPyStitch:
             rmse_host = torch.empty(1, dtype=torch.float64, pin_memory=True)
             rmse_host.copy_(rmse, non_blocking=True)
             res.update(seam_rmse_host=rmse_host, warped1=warped, mask1=m1, mask2=m2, canvas2=canvas2)
-        ext_host = torch.empty(ext.shape, dtype=torch.int32, pin_memory=True)
-        ext_host.copy_(ext, non_blocking=True)
-        res["ext_host"] = ext_host
         return res
 
     def _compose_crop(self, c):
@@ -467,7 +471,7 @@ class GPUPyStitch:
 
     def _compose(self, img1, img2, H, max_canvas_px=400_000_000):
         c = self._compose_enqueue(img1, img2, H, max_canvas_px=max_canvas_px)
-        torch.cuda.current_stream(self.device).synchronize()
+        c["ext_done"].synchronize()
         pano = self._to_host(self._compose_crop(c))
         self._last_compose = c
         return pano, dict(canvas_w=c["canvas_w"], canvas_h=c["canvas_h"], ox=c["ox"], oy=c["oy"],
