@@ -908,6 +908,7 @@ __device__ __forceinline__ void pyr_load(const Level0& src, const PyrLevel& in, 
 template <int NC, bool L0>
 __global__ void k_pyr_rows(const Level0 src, const PyrLevel in, int W, int H, float* __restrict__ t1,
                            float* __restrict__ t2, const GaussTaps w9) {
+    chain_begin();
     const int x = blockIdx.x * blockDim.x + threadIdx.x, yo = blockIdx.y;
     if (x >= W) return;
     const int y = 2 * yo;
@@ -938,6 +939,7 @@ __global__ void k_pyr_rows(const Level0 src, const PyrLevel in, int W, int H, fl
 template <int NC>
 __global__ void k_pyr_cols(const float* __restrict__ t1, const float* __restrict__ t2, int W, int Wo,
                            const GaussTaps w9, float* __restrict__ g1, float* __restrict__ g2) {
+    chain_begin();
     const int xo = blockIdx.x * blockDim.x + threadIdx.x, y = blockIdx.y;
     if (xo >= Wo) return;
     const int col = 2 * xo;
@@ -1023,34 +1025,50 @@ struct Zoom1 {
     }
 };
 
-// one blended Laplacian level k >= 1: m * (G1 - up(G1')) + (1 - m) * (G2 - up(G2'))
-// (pysift/core.py:3529-3541); the coarsest level blends the Gaussians
-__global__ void k_blend_level(const float* __restrict__ g1, const float* __restrict__ g2,
-                              const float* __restrict__ gm, const float* __restrict__ g1n,
-                              const float* __restrict__ g2n, int H, int W, int hn, int wn, ZoomF zf,
-                              float* __restrict__ out) {
-    const int x = blockIdx.x * blockDim.x + threadIdx.x, y = blockIdx.y;
-    if (x >= W) return;
-    const long long p = (long long)y * W + x;
-    const float m = gm[p];
+// The blended Laplacian levels k >= 1: m * (G1 - up(G1')) + (1 - m) * (G2 - up(G2'))
+// (pysift/core.py:3529-3541); the coarsest level blends the Gaussians.  The
+// levels do not depend on one another: one launch, a run of blocks a level
+// (five launches took 23 us and their gaps on a 2112x1213 canvas, one 16).
+struct BlendLevel {
+    const float *g1, *g2, *gm, *g1n, *g2n;  // g1n, g2n null: the coarsest
+    float* out;
+    int H, W, hn, wn;
+    ZoomF zf;
+    int block0;  // the level's first block
+};
+struct BlendLevels {
+    BlendLevel l[7];
+    int n;
+};
+
+__global__ void __launch_bounds__(256) k_blend_levels(const __grid_constant__ BlendLevels a) {
+    int k = 0;
+    while (k + 1 < a.n && (int)blockIdx.x >= a.l[k + 1].block0) ++k;
+    const BlendLevel& v = a.l[k];
+    const int i = (int)blockIdx.x - v.block0, bx = (v.W + 255) / 256;
+    const int y = i / bx, x = (i - y * bx) * 256 + threadIdx.x;
+    if (x >= v.W) return;
+    const long long p = (long long)y * v.W + x;
+    const float m = v.gm[p];
     const float mc = 1.0f - m;
-    if (g1n) {
-        const Zoom1 z(hn, wn, zf, y, x);
+    if (v.g1n) {
+        const Zoom1 z(v.hn, v.wn, v.zf, y, x);
 #pragma unroll
         for (int c = 0; c < 3; ++c) {
-            const float l1 = g1[p * 3 + c] - z.at(g1n, 3, c);
-            const float l2 = g2[p * 3 + c] - z.at(g2n, 3, c);
-            out[p * 3 + c] = m * l1 + mc * l2;
+            const float l1 = v.g1[p * 3 + c] - z.at(v.g1n, 3, c);
+            const float l2 = v.g2[p * 3 + c] - z.at(v.g2n, 3, c);
+            v.out[p * 3 + c] = m * l1 + mc * l2;
         }
     } else {
 #pragma unroll
-        for (int c = 0; c < 3; ++c) out[p * 3 + c] = m * g1[p * 3 + c] + mc * g2[p * 3 + c];
+        for (int c = 0; c < 3; ++c) v.out[p * 3 + c] = m * v.g1[p * 3 + c] + mc * v.g2[p * 3 + c];
     }
 }
 
 // reconstruction step (pysift/core.py:3544-3547): out = up(res) + lb
 __global__ void k_blend_reconstruct(const float* __restrict__ res, int hn, int wn, const float* __restrict__ lb,
                                     int H, int W, ZoomF zf, float* __restrict__ out) {
+    chain_begin();
     const int x = blockIdx.x * blockDim.x + threadIdx.x, y = blockIdx.y;
     if (x >= W) return;
     const long long p = (long long)y * W + x;
@@ -1582,7 +1600,9 @@ int pysift_blend_multiband(const void* image1, int32_t image1_f32, const uint8_t
     PYSIFT_LAUNCH_CHECK("k_seam_rows");
     k_seam_cols<<<dim3(ceil_div(cw, SC_T), ceil_div(ch, SC_L)), SC_T, 0, st>>>(srow, mask1, mask2, k25, gm0, cw, ch);
     PYSIFT_LAUNCH_CHECK("k_seam_cols");
-    // Gaussian pyramid of the seam mask, then join the image pyramids
+    // Gaussian pyramid of the seam mask, then join the image pyramids; its
+    // small launches and the reconstruction's overlap the ends of the ones
+    // before them
     {
         float* tm = bwp<float>(ws, l.off_tm);
         for (int k = 0; k + 1 < n_levels; ++k) {
@@ -1591,10 +1611,10 @@ int pysift_blend_multiband(const void* image1, int32_t image1_f32, const uint8_t
             in.g2 = nullptr;
             in.gm = bwp<float>(ws, l.off_gm[k]);
             const int ho = l.h[k + 1], wo = l.w[k + 1];
-            k_pyr_rows<1, false><<<dim3(ceil_div(l.w[k], 128), ho), 128, 0, st>>>(src, in, l.w[k], l.h[k], tm, nullptr,
-                                                                                  w9);
-            k_pyr_cols<1><<<dim3(ceil_div(wo, 128), ho), 128, 0, st>>>(tm, nullptr, l.w[k], wo, w9,
-                                                                       bwp<float>(ws, l.off_gm[k + 1]), nullptr);
+            launch_chained(k_pyr_rows<1, false>, dim3(ceil_div(l.w[k], 128), ho), 128, 0, st, src, in, l.w[k], l.h[k],
+                           tm, nullptr, w9);
+            launch_chained(k_pyr_cols<1>, dim3(ceil_div(wo, 128), ho), 128, 0, st, tm, nullptr, l.w[k], wo, w9,
+                           bwp<float>(ws, l.off_gm[k + 1]), nullptr);
         }
         PYSIFT_LAUNCH_CHECK("k_pyr mask");
     }
@@ -1602,21 +1622,36 @@ int pysift_blend_multiband(const void* image1, int32_t image1_f32, const uint8_t
     cudaEventDestroy(fork_ev);
     cudaEventDestroy(join_ev);
     // blended Laplacian levels 1 .. n - 1 and the reconstruction down to level 1
-    for (int k = 1; k < n_levels; ++k) {
-        const bool top = k + 1 == n_levels;
-        k_blend_level<<<dim3(ceil_div(l.w[k], 256), l.h[k]), 256, 0, st>>>(
-            bwp<float>(ws, l.off_g1[k]), bwp<float>(ws, l.off_g2[k]), bwp<float>(ws, l.off_gm[k]),
-            top ? nullptr : bwp<float>(ws, l.off_g1[k + 1]), top ? nullptr : bwp<float>(ws, l.off_g2[k + 1]), l.h[k],
-            l.w[k], top ? 0 : l.h[k + 1], top ? 0 : l.w[k + 1],
-            top ? ZoomF{1.0, 1.0} : zoom_factors(l.h[k + 1], l.w[k + 1], l.h[k], l.w[k]), bwp<float>(ws, l.off_lb[k]));
+    if (n_levels > 1) {
+        BlendLevels bl;
+        bl.n = n_levels - 1;
+        long long blocks = 0;
+        for (int k = 1; k < n_levels; ++k) {
+            const bool top = k + 1 == n_levels;
+            BlendLevel& v = bl.l[k - 1];
+            v.g1 = bwp<float>(ws, l.off_g1[k]);
+            v.g2 = bwp<float>(ws, l.off_g2[k]);
+            v.gm = bwp<float>(ws, l.off_gm[k]);
+            v.g1n = top ? nullptr : bwp<float>(ws, l.off_g1[k + 1]);
+            v.g2n = top ? nullptr : bwp<float>(ws, l.off_g2[k + 1]);
+            v.out = bwp<float>(ws, l.off_lb[k]);
+            v.H = l.h[k];
+            v.W = l.w[k];
+            v.hn = top ? 0 : l.h[k + 1];
+            v.wn = top ? 0 : l.w[k + 1];
+            v.zf = top ? ZoomF{1.0, 1.0} : zoom_factors(v.hn, v.wn, v.H, v.W);
+            v.block0 = (int)blocks;
+            blocks += (long long)ceil_div(v.W, 256) * v.H;
+        }
+        k_blend_levels<<<(unsigned int)blocks, 256, 0, st>>>(bl);
     }
-    PYSIFT_LAUNCH_CHECK("k_blend_level");
+    PYSIFT_LAUNCH_CHECK("k_blend_levels");
     const float* res = n_levels > 1 ? bwp<float>(ws, l.off_lb[n_levels - 1]) : nullptr;
     int rh = l.h[n_levels - 1], rw = l.w[n_levels - 1];
     for (int k = n_levels - 2; k >= 1; --k) {
         float* out = bwp<float>(ws, l.off_res[k & 1]);
-        k_blend_reconstruct<<<dim3(ceil_div(l.w[k], 256), l.h[k]), 256, 0, st>>>(
-            res, rh, rw, bwp<float>(ws, l.off_lb[k]), l.h[k], l.w[k], zoom_factors(rh, rw, l.h[k], l.w[k]), out);
+        launch_chained(k_blend_reconstruct, dim3(ceil_div(l.w[k], 256), l.h[k]), 256, 0, st, res, rh, rw,
+                       bwp<float>(ws, l.off_lb[k]), l.h[k], l.w[k], zoom_factors(rh, rw, l.h[k], l.w[k]), out);
         res = out;
         rh = l.h[k];
         rw = l.w[k];
