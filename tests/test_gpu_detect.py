@@ -100,6 +100,17 @@ def test_extrema_strip_edges(H, W, n_scales, oracle_lib):
     _compare(out, ref)
 
 
+@pytest.mark.parametrize("dsp", [False, True])
+@pytest.mark.parametrize("H,W", [(24, 40), (60, 90), (150, 200), (260, 330), (420, 560)])
+def test_descriptor_parts_and_orientation_groups(H, W, dsp, oracle_lib):
+    """Keypoint counts from a handful, whose descriptor entries are cut into as
+    many parts as they can be, to several thousand, which are not cut, and
+    both sides of the orientation's block sizes."""
+    img = synthetic.dense_texture(H, W, seed=H + W, sigma=1.5)
+    sift, out, ref = _run_both(img, oracle_lib, n_octaves=4, dsp=dsp)
+    _compare(out, ref)
+
+
 def test_no_doubling(oracle_lib):
     img = synthetic.scene(480, 640, seed=3)
     sift, out, ref = _run_both(img, oracle_lib, double_image=False)

@@ -39,6 +39,27 @@ def _zoom_gpu(img, fp16):
     return got[:, :2 * W]
 
 
+@pytest.mark.parametrize("shape", [(7, 31), (8, 32), (17, 1000), (255, 255), (256, 257), (1023, 640), (1100, 1344)])
+@pytest.mark.parametrize("pad", [0, 1])
+def test_zoom2x_walk_lengths(shape, pad, oracle_lib):
+    """Sizes from the shortest to the longest walks down the rows, at the edges
+    of their tiles, with rows that take paired stores and rows that do not."""
+    import torch
+    from oracle import oracle
+    from pysift_b200 import _lib
+    H, W = shape
+    img = (np.random.default_rng(H * W).random(shape) * 256).astype(np.uint8)
+    g = torch.from_numpy(img).cuda()
+    coef = torch.empty(H * W, dtype=torch.float64, device="cuda")
+    out = torch.full((2 * H, 2 * W + pad), float("nan"), dtype=torch.float32, device="cuda")
+    assert _lib.load().pysift_zoom2x_u8(g.data_ptr(), H, W, W, 0, coef.data_ptr(), out.data_ptr(), 2 * W + pad,
+                                        torch.cuda.current_stream().cuda_stream) == 0
+    got = out.cpu().numpy()
+    ref = oracle.zoom2x(img.astype(np.float32) / np.float32(255.0))
+    assert np.array_equal(got[:, :2 * W].view(np.int32), ref.view(np.int32))
+    assert np.isnan(got[:, 2 * W:]).all()
+
+
 @pytest.mark.parametrize("shape", SHAPES)
 @pytest.mark.parametrize("fp16", [False, True])
 def test_zoom2x_matches_oracle(shape, fp16, oracle_lib):
