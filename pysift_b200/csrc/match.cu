@@ -66,7 +66,13 @@ namespace pysift {
 constexpr int MT = 128;           // query rows per CTA = UMMA M = TMEM lanes
 constexpr int NT = 128;           // train rows per tile = UMMA N
 constexpr int MATCH_THREADS = 256;  // the scan's reducer threads: 2 warps per TMEM lane quadrant, each half the tile's columns
-constexpr unsigned SPIN_LIMIT = 1u << 22;  // bounded waits on the pipeline barriers
+// Bounded waits: on the scan's pipeline barriers (a build can shorten them to
+// make every scan give up), and for a CTA's own copies and MMAs in flight
+// before it exits.
+#ifndef PYSIFT_MATCH_SPIN_LIMIT
+#define PYSIFT_MATCH_SPIN_LIMIT (1u << 22)
+#endif
+constexpr unsigned SPIN_LIMIT = PYSIFT_MATCH_SPIN_LIMIT, DRAIN_LIMIT = 1u << 22;
 
 enum MatchMode { SIM_F16 = 0, DIST_U8 = 1, SPLIT_FP8 = 2, SIM_I8 = 3 };
 
@@ -194,10 +200,11 @@ __host__ __device__ __forceinline__ size_t tiled_off(int r, int c, int RB) {
 }
 
 // Bounded mbarrier wait that also gives up once another role of the CTA has
-// raised the abort flag.
+// raised the abort flag; without a flag, the wait before an exit.
 __device__ __forceinline__ bool mbar_wait_bounded(uint64_t* bar, uint32_t parity, const volatile int* abort_flag) {
     uint32_t done = 0;
-    for (unsigned spins = 0; spins < SPIN_LIMIT; ++spins) {
+    const unsigned limit = abort_flag ? SPIN_LIMIT : DRAIN_LIMIT;
+    for (unsigned spins = 0; spins < limit; ++spins) {
         asm volatile(
             "{\n\t.reg .pred p;\n\t"
             "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
@@ -621,7 +628,8 @@ struct MergeArgs {
 };
 
 // SIM_I8: merge the column-level segments of one scan (in index order),
-// ratio test on the similarities (pysift/core.py:2676-2680, float32).
+// ratio test on the similarities (pysift/core.py:2676-2680, float32).  A scan
+// that gave up left its segments unwritten: no result.
 __global__ void k_match_merge_i8(const __grid_constant__ MergeArgs m) {
     const int sd = (int)blockIdx.x >= m.blocks0 ? 1 : 0;
     const MergeSide& z = m.side[sd];
@@ -641,9 +649,10 @@ __global__ void k_match_merge_i8(const __grid_constant__ MergeArgs m) {
         i1 = p.k1 > k1 ? p.i1 : i1;
         k1 = fmaxf(k1, p.k1);
     }
+    const bool bad = *m.error || !(k1 > -INFINITY) || i1 < 0 || i1 >= z.n_t;
     int ok = 0;
     float d = 0.0f;
-    if (k2 > -INFINITY) {
+    if (!bad && k2 > -INFINITY) {
         float db = 2.0f - 2.0f * k1;
         float ds = 2.0f - 2.0f * k2;
         db = db < 0.0f ? 0.0f : db;
@@ -651,7 +660,7 @@ __global__ void k_match_merge_i8(const __grid_constant__ MergeArgs m) {
         ok = (ds > 1e-10f) && (db < ratio_sq * ds);
         d = sqrtf(db);
     }
-    best[i] = (k1 > -INFINITY) ? i1 : -1;
+    best[i] = bad ? -1 : i1;
     pass[i] = ok;
     if (dist) dist[i] = d;
 }
@@ -1112,7 +1121,8 @@ __global__ void __cluster_dims__(RECHECK_C, 1, 1) __launch_bounds__(RECHECK_T)
 // lane with both gathers of all of them in flight), ballots place the pairs.
 __global__ void __launch_bounds__(1024) k_match_mutual(const int* __restrict__ fbest, const int* __restrict__ fpass,
                                                        const float* __restrict__ fdist, const int* __restrict__ bbest,
-                                                       const int* __restrict__ bpass, int n1, int2* __restrict__ pairs,
+                                                       const int* __restrict__ bpass, int n1, int n2,
+                                                       int2* __restrict__ pairs,
                                                        float* __restrict__ pdist, int* __restrict__ count) {
     __shared__ int sh[33];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -1133,7 +1143,7 @@ __global__ void __launch_bounds__(1024) k_match_mutual(const int* __restrict__ f
         }
 #pragma unroll
         for (int k = 0; k < K; ++k) {
-            const bool ok = p[k] && j[k] >= 0;
+            const bool ok = p[k] && j[k] >= 0 && j[k] < n2;
             p[k] = ok ? bpass[j[k]] : 0;
             b[k] = ok ? bbest[j[k]] : -1;
         }
@@ -1487,8 +1497,8 @@ static int run_match(int mode, const uint8_t* rows_a, int n1, const uint8_t* row
         else (D == 64 ? k_match_merge_u8<64> : k_match_merge_u8<128>)<<<blocks, 256, 0, st>>>(m);
         PYSIFT_LAUNCH_CHECK("k_match_merge");
     }
-    k_match_mutual<<<1, 1024, 0, st>>>(fbest, fpass, fdist, bbest, bpass, n1, reinterpret_cast<int2*>(pairs), pdist,
-                                       count);
+    k_match_mutual<<<1, 1024, 0, st>>>(fbest, fpass, fdist, bbest, bpass, n1, n2, reinterpret_cast<int2*>(pairs),
+                                       pdist, count);
     PYSIFT_LAUNCH_CHECK("k_match_mutual");
     return PYSIFT_OK;
 }

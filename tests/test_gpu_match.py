@@ -267,3 +267,65 @@ def test_stitch_int8_matching_end_to_end():
     assert np.array_equal(st._last["pairs"].cpu().numpy(), orc["pairs"])
     rel = np.max(np.abs(st._last["H"] - orc["H"]) / np.maximum(np.abs(orc["H"]), 1e-6))
     assert rel < 1e-6, rel
+
+
+_GIVE_UP_HOST = r'''
+#include <cstdarg>
+namespace pysift {
+void set_error(const char*, ...) {}
+void count_launch() {}
+}
+'''
+
+
+@pytest.fixture(scope="module")
+def giving_up_lib(tmp_path_factory):
+    """match.cu with pipeline waits of no length (the waits for copies and MMAs
+    in flight before a block exits keep theirs): every scan gives up, sets its
+    error flag and leaves its segments unwritten."""
+    import ctypes
+    import os
+    import subprocess
+    from pysift_b200 import _lib, build
+    d = tmp_path_factory.mktemp("give_up")
+    (d / "host.cpp").write_text(_GIVE_UP_HOST)
+    so = d / "libgiveup.so"
+    subprocess.check_call([build.nvcc(), *build.ARCH, "-O3", "--fmad=false", "-std=c++17", "-Xcompiler", "-fPIC",
+                           "-DPYSIFT_MATCH_SPIN_LIMIT=0", "-shared", "-o", str(so),
+                           os.path.join(build.HERE, "csrc", "match.cu"), str(d / "host.cpp")])
+    lib = ctypes.CDLL(str(so))
+    for name in ("pysift_match_fp16", "pysift_match_u8_exact", "pysift_match_u8_split_fp8", "pysift_match_i8"):
+        getattr(lib, name).restype, getattr(lib, name).argtypes = _lib.EXPORTS[name]
+    return lib
+
+
+@pytest.mark.parametrize("n1,n2", [(1, 1), (130, 257), (1500, 300)])
+@pytest.mark.parametrize("mode", ["fp16", "u8_exact", "u8_split_fp8", "i8"])
+def test_scan_that_gives_up_matches_nothing(mode, n1, n2, giving_up_lib):
+    """Segments left over in the workspace from an earlier use (here: finite
+    keys with indices past both sets) are not read as a result."""
+    import torch
+    from pysift_b200 import match
+    from pysift_b200._lib import load
+    D = 64
+    dt = {"fp16": torch.float16, "i8": torch.int8}.get(mode, torch.uint8)
+    d1, d2 = torch.ones((n1, D), device="cuda").to(dt), torch.ones((n2, D), device="cuda").to(dt)
+    s1, s2 = torch.ones(n1, device="cuda"), torch.ones(n2, device="cuda")
+    ws = match._ws(load(), n1, n2, D, {"u8_exact": 1, "u8_split_fp8": 2}.get(mode, 0), d1.device)
+    ws.fill_(0x3f)  # keys 0.747, indices 0x3f3f3f3f
+    wp, wn = match._aligned(ws)
+    outs = [torch.full((n,), 7, dtype=torch.int32, device="cuda") for n in (n1, n1, n2, n2)]
+    pairs = torch.full((n1, 2), 7, dtype=torch.int32, device="cuda")
+    dist = torch.full((n1,), 7.0, device="cuda")
+    count = torch.full((1,), 7, dtype=torch.int32, device="cuda")
+    fn = getattr(giving_up_lib, f"pysift_match_{mode}")
+    sets = (d1.data_ptr(), s1.data_ptr(), n1, d2.data_ptr(), s2.data_ptr(), n2) if mode == "i8" else \
+        (d1.data_ptr(), n1, d2.data_ptr(), n2)
+    rc = fn(*sets, D, 0.75, wp, wn, *[o.data_ptr() for o in outs], pairs.data_ptr(), dist.data_ptr(),
+            count.data_ptr(), torch.cuda.current_stream().cuda_stream)
+    assert rc == 0
+    torch.cuda.synchronize()
+    assert (outs[0] == -1).all() and (outs[2] == -1).all()
+    assert (outs[1] == 0).all() and (outs[3] == 0).all()
+    assert count.item() == 0
+    assert (pairs == 7).all() and (dist == 7.0).all()
