@@ -1000,6 +1000,49 @@ struct F16Row {
             }
         }
     }
+    // One chunk of a row that takes every column: columns that the exact keys so
+    // far rule out are left, and when many remain, as repeated rows give them, a
+    // column a lane, where a chain of warp-wide sums would be longer.
+    static constexpr int F16_FEW = 8;
+    __device__ __forceinline__ void chunk_of_run(int c0) {
+        const int col = c0 + chunk_row<LPR>(lane);
+        bool cand = col < n_t;
+        if (fast) {
+            const float v = rough(c0);
+            float b1 = cand ? v : -INFINITY, b2 = -INFINITY;
+#pragma unroll
+            for (int o = 16; o > 0; o >>= 1) {
+                const float o1 = __shfl_xor_sync(FULL_MASK, b1, o), o2 = __shfl_xor_sync(FULL_MASK, b2, o);
+                b2 = fmaxf(fmaxf(b2, o2), fminf(b1, o1));
+                b1 = fmaxf(b1, o1);
+            }
+            m2 = fmaxf(fmaxf(m2, b2), fminf(m1, b1));
+            m1 = fmaxf(m1, b1);
+            const float margin = e2 + (0x1p-9f * (fabsf(m1) + e2) + 0x1p-23f);
+            cand = cand && !(v < m2 - margin);
+            if (ks) {
+                // nothing to gain either from a column whose similarity can
+                // neither pass the second value nor, being later, take a tie
+                const float f1 = sim_key_value(kb), f2 = sim_key_value(ks);
+                const float u = round_half(__fadd_ru(v, e2));
+                cand = cand && !(u <= f2 && (u < f1 || col > sim_key_column(kb)));
+            }
+            unsigned todo = __ballot_sync(FULL_MASK, cand);
+            if (__popc(todo) <= F16_FEW) {
+                while (todo) {
+                    const int l = __ffs(todo) - 1;
+                    todo &= todo - 1;
+                    exact(c0 + chunk_row<LPR>(l));
+                }
+                return;
+            }
+        }
+        unsigned long long b = 0, s = 0;
+        if (cand) b = sim_key(f16_round_f64(dot_f16_exact(q, t + (size_t)col * D, D)), col);
+        if (fast) warp_top2_u64(b, s);
+        take(b);
+        take(s);
+    }
     // the two largest over the warp
     __device__ __forceinline__ void join() {
         if (!fast) warp_top2_u64(kb, ks);
@@ -1065,16 +1108,19 @@ __global__ void k_match_merge_f16(const __grid_constant__ MergeArgs m) {
 // the lowest index.  Sets of 8000 x 64 with a few such rows: 40 -> 7 us
 // against one CTA a row that formed every column in float64.
 constexpr int RECHECK_T = 512, RECHECK_C = 8;
+constexpr int RECHECK_FEW = 4 * 2 * 148 / RECHECK_C;  // rows left to the clusters: a few each
 
 template <int D>
 __global__ void __cluster_dims__(RECHECK_C, 1, 1) __launch_bounds__(RECHECK_T)
     k_match_recheck_f16(const __grid_constant__ MergeArgs m) {
+    chain_begin();
     __shared__ unsigned long long s_b[RECHECK_T / 32], s_s[RECHECK_T / 32];
     __shared__ unsigned long long s_cta[2];
     namespace cg = cooperative_groups;
     cg::cluster_group cluster = cg::this_cluster();
     const int rank = (int)cluster.block_rank();
     const int c0 = *m.side[0].n_recheck, call = c0 + *m.side[1].n_recheck;
+    if (call > RECHECK_FEW) return;  // k_match_recheck_runs_f16
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     for (int v = blockIdx.x / RECHECK_C; v < call; v += gridDim.x / RECHECK_C) {
         const MergeSide& z = m.side[v < c0 ? 0 : 1];
@@ -1116,14 +1162,54 @@ __global__ void __cluster_dims__(RECHECK_C, 1, 1) __launch_bounds__(RECHECK_T)
     }
 }
 
+// More such rows than the clusters take, as sets with repeated rows leave them
+// by the thousand: a CTA takes a row, which spares the cluster's barriers, and
+// with a row for every warp each warp takes rows of its own, so that the warps
+// of a CTA walk the same columns and read them from the L1 cache.  Two sets of
+// 5000 x 64 with 10 distinct rows match in 1.2 ms, by clusters 4.9.
+template <int D>
+__global__ void __launch_bounds__(RECHECK_T) k_match_recheck_runs_f16(const __grid_constant__ MergeArgs m) {
+    chain_begin();
+    constexpr int W = RECHECK_T / 32;
+    __shared__ unsigned long long s_b[W], s_s[W];
+    const int c0 = *m.side[0].n_recheck, call = c0 + *m.side[1].n_recheck;
+    if (call <= RECHECK_FEW) return;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int team = call < (int)gridDim.x * W ? W : 1, member = warp % team;  // warps a row
+    for (int v = ((int)blockIdx.x * W + warp) / team; v < call; v += (int)gridDim.x * W / team) {
+        const MergeSide& z = m.side[v < c0 ? 0 : 1];
+        const int i = v < c0 ? z.recheck[v] : z.recheck[v - c0];
+        F16Row<D> row(z, i);
+        for (int c = member * 32; c < z.n_t; c += 32 * team) row.chunk_of_run(c);
+        row.join();
+        unsigned long long kb = row.kb, ks = row.ks;
+        if (team > 1) {
+            if (lane == 0) {
+                s_b[warp] = kb;
+                s_s[warp] = ks;
+            }
+            __syncthreads();
+            if (warp == 0) {
+                kb = lane < W ? s_b[lane] : 0;
+                ks = lane < W ? s_s[lane] : 0;
+                warp_top2_u64(kb, ks);
+            }
+            __syncthreads();
+        }
+        if (member == 0 && lane == 0)
+            finish_f16_row(i, sim_key_value(kb), ks ? sim_key_value(ks) : -INFINITY, sim_key_column(kb), m.ratio_sq,
+                           z.best, z.pass, z.dist);
+    }
+}
+
 // Mutual matches in query order: fwd[i] = j passes, bwd[j] = i passes.  One
 // CTA: a warp covers 256 consecutive rows a round (coalesced loads, 8 rows a
 // lane with both gathers of all of them in flight), ballots place the pairs.
-__global__ void __launch_bounds__(1024) k_match_mutual(const int* __restrict__ fbest, const int* __restrict__ fpass,
-                                                       const float* __restrict__ fdist, const int* __restrict__ bbest,
-                                                       const int* __restrict__ bpass, int n1, int n2,
-                                                       int2* __restrict__ pairs,
-                                                       float* __restrict__ pdist, int* __restrict__ count) {
+__global__ void __launch_bounds__(1024) k_match_mutual(const int* fbest, const int* fpass, const float* fdist,
+                                                       const int* bbest, const int* bpass, int n1, int n2,
+                                                       int2* __restrict__ pairs, float* __restrict__ pdist,
+                                                       int* __restrict__ count) {
+    chain_begin();
     __shared__ int sh[33];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const unsigned below = (1u << lane) - 1u;
@@ -1143,7 +1229,7 @@ __global__ void __launch_bounds__(1024) k_match_mutual(const int* __restrict__ f
         }
 #pragma unroll
         for (int k = 0; k < K; ++k) {
-            const bool ok = p[k] && j[k] >= 0 && j[k] < n2;
+            const bool ok = p[k] && (unsigned)j[k] < (unsigned)n2;
             p[k] = ok ? bpass[j[k]] : 0;
             b[k] = ok ? bbest[j[k]] : -1;
         }
@@ -1489,16 +1575,18 @@ static int run_match(int mode, const uint8_t* rows_a, int n1, const uint8_t* row
     if (mode == SIM_F16) {
         (D == 64 ? k_match_merge_f16<64> : k_match_merge_f16<128>)<<<blocks, 256, 0, st>>>(m);
         PYSIFT_LAUNCH_CHECK("k_match_merge_f16");
-        (D == 64 ? k_match_recheck_f16<64> : k_match_recheck_f16<128>)<<<2 * sm_count() / RECHECK_C * RECHECK_C, RECHECK_T, 0,
-                                                                                    st>>>(m);
+        const dim3 grid(2 * sm_count() / RECHECK_C * RECHECK_C);
+        launch_chained(D == 64 ? k_match_recheck_f16<64> : k_match_recheck_f16<128>, grid, RECHECK_T, 0, st, m);
         PYSIFT_LAUNCH_CHECK("k_match_recheck_f16");
+        launch_chained(D == 64 ? k_match_recheck_runs_f16<64> : k_match_recheck_runs_f16<128>, grid, RECHECK_T, 0, st, m);
+        PYSIFT_LAUNCH_CHECK("k_match_recheck_runs_f16");
     } else {
         if (mode == SIM_I8) k_match_merge_i8<<<blocks, 256, 0, st>>>(m);
         else (D == 64 ? k_match_merge_u8<64> : k_match_merge_u8<128>)<<<blocks, 256, 0, st>>>(m);
         PYSIFT_LAUNCH_CHECK("k_match_merge");
     }
-    k_match_mutual<<<1, 1024, 0, st>>>(fbest, fpass, fdist, bbest, bpass, n1, n2, reinterpret_cast<int2*>(pairs),
-                                       pdist, count);
+    launch_chained(k_match_mutual, dim3(1), 1024, 0, st, (const int*)fbest, (const int*)fpass, (const float*)fdist,
+                   (const int*)bbest, (const int*)bpass, n1, n2, reinterpret_cast<int2*>(pairs), pdist, count);
     PYSIFT_LAUNCH_CHECK("k_match_mutual");
     return PYSIFT_OK;
 }

@@ -329,3 +329,29 @@ def test_scan_that_gives_up_matches_nothing(mode, n1, n2, giving_up_lib):
     assert (outs[1] == 0).all() and (outs[3] == 0).all()
     assert count.item() == 0
     assert (pairs == 7).all() and (dist == 7.0).all()
+
+
+@pytest.mark.parametrize("D", [64, 128])
+@pytest.mark.parametrize("n1,n2,distinct,ulps", [
+    (60, 70, 3, 0),        # fewer rechecked rows than the clusters take together
+    (700, 900, 1, 0),      # every similarity equal
+    (600, 4200, 3, 0),     # chunks full of candidates; more chunks than warps
+    (1000, 2100, 40, 0),
+    (900, 1300, 5, 1),     # copies that differ by one unit in the last place
+])
+def test_fp16_repeated_rows(n1, n2, distinct, ulps, D):
+    """Sets with few distinct rows: more than two best columns a row, so most
+    rows are recomputed over every column; the lowest index wins."""
+    rng = np.random.default_rng(n1 + distinct + D)
+    base = rng.standard_normal((distinct, D)).astype(np.float32)
+    base = (base / np.linalg.norm(base, axis=1, keepdims=True)).astype(np.float16)
+    sets = []
+    for n in (n1, n2):
+        x = base[rng.integers(0, distinct, n)]
+        for _ in range(ulps):
+            k = rng.integers(0, D, n)
+            v = x[np.arange(n), k]
+            x[np.arange(n), k] = np.nextafter(v, np.where(rng.random(n) < 0.5, np.inf, -np.inf).astype(np.float16))
+        sets.append(x)
+    _, _, rechecked = _fp16_match_and_check(*sets)
+    assert rechecked.sum() > (0 if n1 < 100 else 500)
