@@ -518,6 +518,34 @@ struct DpBand {
 // halo[parity][side][warp]: the DP_B values left (side 0) / right (side 1) of a warp's net positions
 typedef double DpHalo[2][2][DP_WARPS][DP_B];
 
+// One line: the costs c of the lane's E positions on it, D of the line before
+// in p (replaced); d gets the directions.
+template <int E>
+__device__ __forceinline__ void dp_line(const float4 (&c)[E / 4], double (&p)[E], unsigned (&d)[E / 4]) {
+    // the outermost lanes read themselves: those positions are stale by now
+    const double left = __shfl_up_sync(0xffffffffu, p[E - 1], 1);
+    const double right = __shfl_down_sync(0xffffffffu, p[0], 1);
+    double o[E];
+#pragma unroll
+    for (int k = 0; k < E / 4; ++k) {
+        const float v[4] = {c[k].x, c[k].y, c[k].z, c[k].w};
+        d[k] = 0u;
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+            const int i = 4 * k + e;
+            const double pl = i ? p[i - 1] : left, pm = p[i], pr = i + 1 < E ? p[i + 1] : right;
+            unsigned m = 0u;
+            double best = pl;
+            if (pm < best) { best = pm; m = 1u << (8 * e); }
+            if (pr < best) { best = pr; m = 2u << (8 * e); }
+            d[k] |= m;
+            o[i] = v[e] >= 0.0f ? (double)v[e] + best : BL_INF;
+        }
+    }
+#pragma unroll
+    for (int i = 0; i < E; ++i) p[i] = o[i];
+}
+
 template <int E>
 __device__ __forceinline__ void dp_band(const DpBand& a, DpHalo& halo) {
     constexpr int NET = dp_net<E>(), NQ = E / 4, HL = DP_B / E;  // HL lanes hold a halo
@@ -563,29 +591,8 @@ __device__ __forceinline__ void dp_band(const DpBand& a, DpHalo& halo) {
         for (int t = 0; t < DP_B; ++t) {
             if (q0 + t >= a.nL) break;
             const int line = __shfl_sync(0xffffffffu, ids, t);
-            // the outermost lanes read themselves: those positions are stale by now
-            const double left = __shfl_up_sync(0xffffffffu, p[E - 1], 1);
-            const double right = __shfl_down_sync(0xffffffffu, p[0], 1);
-            double o[E];
             unsigned d[NQ];
-#pragma unroll
-            for (int k = 0; k < NQ; ++k) {
-                const float v[4] = {ring[t][k].x, ring[t][k].y, ring[t][k].z, ring[t][k].w};
-                d[k] = 0u;
-#pragma unroll
-                for (int e = 0; e < 4; ++e) {
-                    const int i = 4 * k + e;
-                    const double pl = i ? p[i - 1] : left, pm = p[i], pr = i + 1 < E ? p[i + 1] : right;
-                    unsigned m = 0u;
-                    double best = pl;
-                    if (pm < best) { best = pm; m = 1u << (8 * e); }
-                    if (pr < best) { best = pr; m = 2u << (8 * e); }
-                    d[k] |= m;
-                    o[i] = v[e] >= 0.0f ? (double)v[e] + best : BL_INF;
-                }
-            }
-#pragma unroll
-            for (int i = 0; i < E; ++i) p[i] = o[i];
+            dp_line<E>(ring[t], p, d);
             if (net) {
                 uint8_t* row = a.dir + (long long)line * a.Mp + pos;
 #pragma unroll
@@ -635,32 +642,79 @@ __device__ __forceinline__ void dp_band(const DpBand& a, DpHalo& halo) {
     }
 }
 
-// Bands wider than the cluster's registers: one CTA, the two DP lines in
-// global memory, a block barrier per line.
-__device__ __noinline__ void dp_wide(const DpBand& a, double* prev, double* cur) {
-    const int tid = threadIdx.x;
-    for (int q = 0; q < a.nL; ++q) {
-        const long long row = (long long)a.ovl[q] * a.Mp;
-        for (int j = a.lo + tid; j <= a.hi; j += DP_T) {
-            const float c = a.dpc[row + j];
-            double best = 0.0;
-            if (q > 0) {
-                const double pl = j > a.lo ? prev[j - 1] : BL_INF, pm = prev[j], pr = j < a.hi ? prev[j + 1] : BL_INF;
-                int m = 0;
-                best = pl;
-                if (pm < best) { best = pm; m = 1; }
-                if (pr < best) { best = pr; m = 2; }
-                a.dir[row + j] = (uint8_t)m;
+// Bands wider than the cluster's registers: the same blocks of DP_B lines, the
+// cluster's warps taking the band's pieces in turn, with D of a block's last
+// line in global memory (in L2, two lines in turn) for the next block.  A blend
+// with two overlaps 10,000 columns apart on 700 lines took 29.1 ms with one CTA
+// walking the whole band a line at a time, 14.4 walking each line's own window,
+// 1.9 so.
+template <int E>
+__device__ __noinline__ void dp_wide(const DpBand& a, double* prev) {
+    constexpr int NET = dp_net<E>(), NQ = E / 4, HL = DP_B / E;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int nseg = (a.hi - a.lo) / NET + 1, stored = min(a.M, a.lo + nseg * NET);
+    double* cur = a.end;
+    if (((a.nL - 1 + DP_B - 1) / DP_B & 1) == 0 && a.nL > 1) {  // the last block writes a.end
+        cur = prev;
+        prev = a.end;
+    }
+    for (int q0 = 1; q0 == 1 || q0 < a.nL; q0 += DP_B) {
+        const int ids = lane < DP_B && q0 + lane < a.nL ? a.ovl[q0 + lane] : -1;
+        for (int seg = (int)dp_cluster_rank() * DP_WARPS + warp; seg < nseg; seg += DP_CTAS * DP_WARPS) {
+            const int pos = a.lo + seg * NET - DP_B + lane * E;
+            const bool net = lane >= HL && lane < 32 - HL;
+            auto load = [&](int line, float4 c[NQ]) {
+                const float* src = a.dpc + (long long)line * a.Mp + pos;
+#pragma unroll
+                for (int k = 0; k < NQ; ++k)
+                    c[k] = pos + 4 * k >= 0 && pos + 4 * k < a.Mp ? __ldg(reinterpret_cast<const float4*>(src) + k)
+                                                                  : make_float4(-1.0f, -1.0f, -1.0f, -1.0f);
+            };
+            float4 ring[DP_B][NQ];
+#pragma unroll
+            for (int t = 0; t < DP_B; ++t) {
+                const int line = __shfl_sync(0xffffffffu, ids, t);
+                if (line >= 0) load(line, ring[t]);
             }
-            cur[j] = c >= 0.0f ? (double)c + best : BL_INF;
+            double p[E];
+            if (q0 == 1) {
+                float4 c[NQ];
+                load(a.ovl[0], c);
+#pragma unroll
+                for (int k = 0; k < NQ; ++k) {
+                    const float v[4] = {c[k].x, c[k].y, c[k].z, c[k].w};
+#pragma unroll
+                    for (int e = 0; e < 4; ++e) p[4 * k + e] = v[e] >= 0.0f ? (double)v[e] : BL_INF;
+                }
+            } else {
+#pragma unroll
+                for (int i = 0; i < E; ++i)
+                    p[i] = pos + i >= a.lo && pos + i < stored ? __ldcg(prev + pos + i) : BL_INF;
+            }
+#pragma unroll
+            for (int t = 0; t < DP_B; ++t) {
+                const int line = __shfl_sync(0xffffffffu, ids, t);
+                if (line < 0) break;
+                unsigned d[NQ];
+                dp_line<E>(ring[t], p, d);
+                if (net) {
+                    uint8_t* row = a.dir + (long long)line * a.Mp + pos;
+#pragma unroll
+                    for (int k = 0; k < NQ; ++k)
+                        if (pos + 4 * k < a.Mp) reinterpret_cast<unsigned*>(row)[k] = d[k];
+                }
+            }
+            if (net) {
+#pragma unroll
+                for (int i = 0; i < E; ++i)
+                    if (pos + i < stored) __stcg(cur + pos + i, p[i]);
+            }
         }
-        __syncthreads();
+        dp_cluster_sync();
         double* t = prev;
         prev = cur;
         cur = t;
     }
-    if (prev != a.end)
-        for (int j = a.lo + tid; j <= a.hi; j += DP_T) a.end[j] = prev[j];
 }
 
 __global__ void __cluster_dims__(DP_CTAS, 1, 1) __launch_bounds__(DP_T)
@@ -686,7 +740,7 @@ __global__ void __cluster_dims__(DP_CTAS, 1, 1) __launch_bounds__(DP_T)
     const int width = a.hi - a.lo + 1;
     if (width <= DP_CTAS * DP_WARPS * dp_net<4>()) dp_band<4>(a, halo);
     else if (width <= DP_CTAS * DP_WARPS * dp_net<8>()) dp_band<8>(a, halo);
-    else if (rank == 0) dp_wide(a, gB, gA);
+    else dp_wide<8>(a, gB);
     dp_cluster_sync();
     if (rank != 0) return;
     // first minimum of the last overlap line (non-overlap positions count as INF)

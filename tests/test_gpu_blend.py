@@ -437,3 +437,13 @@ def test_blend_in_a_cuda_graph():
         g.replay()
         torch.cuda.synchronize()
         assert np.array_equal(pano.cpu().numpy(), eager[1 - k])
+
+
+@pytest.mark.parametrize("rows,lo,na,gap,nb", [
+    (17, 3, 8, 7200, 8), (18, 4, 8, 7200, 8), (33, 5, 16, 7200, 16), (34, 1, 17, 7200, 17),
+    (40, 2, 20, 14296, 20), (40, 2, 20, 14297, 20),   # 14336 and 14337: two and three pieces a warp
+    (520, 7, 500, 6900, 20),                           # an overlap across several pieces
+])
+def test_blend_seam_wide_bands(rows, lo, na, gap, nb):
+    """Bands past the registers of the DP's cluster, over its line blocks."""
+    test_blend_seam_band_edges(rows, lo, na, gap, nb)
