@@ -457,6 +457,7 @@ __device__ void jacobi9_smallest(double (*M)[9], JacobiRot& rot, double* v_out) 
                 __syncwarp();
             }
         }
+        __syncwarp();  // rot.act of rounds without a rotation, which take no barrier
         int best = 0;
         for (int k = 1; k < 9; ++k)
             if (M[k][k] < M[best][best]) best = k;

@@ -166,6 +166,32 @@ def test_dlt_matches_oracle_and_svd():
     assert np.max(np.abs(Hg - Hs) / np.maximum(np.abs(Hs), 1e-9)) < 1e-6
 
 
+@pytest.mark.parametrize("side", [2, 3, 8])
+def test_dlt_of_symmetric_grids(side):
+    """Centred grids under a shift, a scale and a reflection: the normal matrix
+    starts with most of its off-diagonal zero, so that whole rounds of the
+    Jacobi sweeps rotate nothing, the last ones among them.  Each follows the
+    refit of an irregular set, whose rotations are not to be seen."""
+    import torch
+    from oracle import stitch_oracle as so
+    L, lib = _lib()
+    idx = torch.empty(400, dtype=torch.int32, device="cuda")
+    H = torch.empty(9, dtype=torch.float64, device="cuda")
+
+    def refit(p1, p2):
+        d1, d2 = torch.from_numpy(p1).cuda(), torch.from_numpy(p2).cuda()
+        assert lib.pysift_dlt_homography(d1.data_ptr(), d2.data_ptr(), len(p1), idx.data_ptr(), H.data_ptr(),
+                                         _st()) == 0
+        assert np.array_equal(H.cpu().numpy().reshape(3, 3), so.dlt(p1, p2))
+
+    g = np.stack(np.meshgrid(np.arange(side), np.arange(side)), -1).reshape(-1, 2) * 2.0 - (side - 1)
+    for k, f in enumerate((lambda p: p, lambda p: p + [3.0, -5.0], lambda p: 4.0 * p, lambda p: p * [-1.0, 1.0],
+                           lambda p: p[:, ::-1] * 0.5 + 7.0)):
+        p1, p2, _ = _correspondences(20 + k, n=400, outliers=0.0)
+        refit(p1, p2)
+        refit(g, np.ascontiguousarray(f(g)))
+
+
 def test_warp_feather_bit_exact_and_grid_sample():
     import torch
     import torch.nn.functional as F
