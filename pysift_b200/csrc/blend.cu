@@ -991,7 +991,7 @@ __global__ void k_pyr_rows(const Level0 src, const PyrLevel in, int W, int H, fl
 }
 
 template <int NC>
-__global__ void k_pyr_cols(const float* __restrict__ t1, const float* __restrict__ t2, int W, int Wo,
+__global__ void k_pyr_cols(const float* t1, const float* t2, int W, int Wo,
                            const GaussTaps w9, float* __restrict__ g1, float* __restrict__ g2) {
     chain_begin();
     const int xo = blockIdx.x * blockDim.x + threadIdx.x, y = blockIdx.y;
@@ -1120,8 +1120,8 @@ __global__ void __launch_bounds__(256) k_blend_levels(const __grid_constant__ Bl
 }
 
 // reconstruction step (pysift/core.py:3544-3547): out = up(res) + lb
-__global__ void k_blend_reconstruct(const float* __restrict__ res, int hn, int wn, const float* __restrict__ lb,
-                                    int H, int W, ZoomF zf, float* __restrict__ out) {
+__global__ void k_blend_reconstruct(const float* res, int hn, int wn, const float* lb, int H, int W, ZoomF zf,
+                                    float* __restrict__ out) {
     chain_begin();
     const int x = blockIdx.x * blockDim.x + threadIdx.x, y = blockIdx.y;
     if (x >= W) return;

@@ -53,6 +53,10 @@ void count_launch();
 // its launch then overlaps the end of the one before, and chain_begin() waits
 // for that one's completion and for its writes.  It also lets the kernel
 // after it be launched.  A no-op in a kernel launched the ordinary way.
+// What the kernel before may still write while this one starts is not read-only
+// for this one's lifetime: such an input is no `const T* __restrict__` parameter
+// and not read with __ldg, which would let its loads go by the read-only path or
+// before the wait.
 __device__ __forceinline__ void chain_begin() {
     asm volatile("griddepcontrol.wait;\n\tgriddepcontrol.launch_dependents;" ::: "memory");
 }

@@ -514,7 +514,7 @@ constexpr int ZI_T = 256, ZI_W = ZI_T / 32;
 constexpr int ZI_MAX_PAIRS = 16;                       // row pairs of a warp, at most
 constexpr int ZI_CC = 36;
 
-__global__ void __launch_bounds__(ZI_T, 3) k_zoom_interp(const double* __restrict__ coef, int H, int W, double zy,
+__global__ void __launch_bounds__(ZI_T, 3) k_zoom_interp(const double* coef, int H, int W, double zy,
                                                       double zx, int fp16, int pairs, float* __restrict__ out, int out_pitch) {
     chain_begin();
     __shared__ __align__(16) double rw[2 * ZI_W * ZI_MAX_PAIRS][4];  // weights of output rows 2 j0 - 1 + i
@@ -1329,7 +1329,9 @@ __device__ __forceinline__ void extrema_strips(const ExtArgs& a, int block, floa
     if (r0 >= H) return;
     const int r1 = min(r0 + a.rows, H);  // rows r0 .. r1 - 1
     const int c = (unit - ry * ncx) * EX_COLS - 2 + 2 * lane;
-    // columns outside the row read any value: their pixels lie in the border
+    // columns outside the row read any value: their pixels lie in the border.
+    // (__ldg: the levels are complete before the first pass, which is launched
+    // the ordinary way, so in the chained retry too)
     const long long pitch = v.pitch, plane = v.lev[1] - v.lev[0];
     const float* src = v.lev[0] + (long long)max(r0 - 1, 0) * pitch + max(0, min(c, v.pitch - 2));
     float2 D[3][ND], g[NL];
@@ -2592,9 +2594,8 @@ __global__ void __launch_bounds__(DESC_T, DESC_OCC) k_descriptor(const DescArgs 
 
 // Response of every output row (rows are the (x, y) ranks of the oriented
 // entries), counted into the output-limit order's buckets.
-__global__ void k_row_resp(const int* __restrict__ ent_kp, const float* __restrict__ kp_resp,
-                           const int* __restrict__ rank, float* __restrict__ row_resp, int* __restrict__ resp_cnt,
-                           const Ctrl* ctrl) {
+__global__ void k_row_resp(const int* ent_kp, const float* kp_resp, const int* rank, float* __restrict__ row_resp,
+                           int* __restrict__ resp_cnt, const Ctrl* ctrl) {
     chain_begin();
     const int n = ctrl->n_oriented;
     for (int e = blockIdx.x * blockDim.x + threadIdx.x; e < n; e += gridDim.x * blockDim.x) {

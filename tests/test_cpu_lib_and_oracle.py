@@ -208,3 +208,23 @@ def test_ransac_samples_equal_torch_randint(n_points, n_hyp):
     gen.manual_seed(42)
     want = torch.randint(0, n_points, (n_hyp, 4), generator=gen).numpy().ravel()
     assert np.array_equal((host % np.uint32(n_points)).astype(np.int64), want)
+
+
+def test_chained_kernels_wait_first_and_claim_no_read_only_inputs():
+    """A kernel that may start while the one before it still writes (launched
+    with launch_chained, directly or through the blur and extrema tables) waits
+    before anything else, and no parameter promises that its data is read-only
+    for the kernel's whole life."""
+    kernels, chained = {}, {"k_blur", "k_extrema_mask"}
+    csrc = os.path.join(ROOT, "pysift_b200", "csrc")
+    for name in sorted(f for f in os.listdir(csrc) if f.endswith(".cu")):
+        src = re.sub(r"//[^\n]*", "", open(os.path.join(csrc, name)).read())
+        for m in re.finditer(r"__global__[^;{]*?\b(k_\w+)\s*\(([^{;]*)\)\s*\{\s*([^;]*;)", src):
+            kernels[m.group(1)] = (m.group(2), m.group(3))
+        for m in re.finditer(r"\blaunch_chained\(([^,]*),", src):
+            chained.update(re.findall(r"\bk_\w+", m.group(1)))
+    assert len(chained) > 20
+    for k in sorted(chained):
+        params, first = kernels[k]
+        assert first == "chain_begin();", k
+        assert not re.search(r"\bconst\b[^,]*__restrict__", params), k
