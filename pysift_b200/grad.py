@@ -81,7 +81,7 @@ def _levels_plan(kps, sift, shape):
         sizes.append(nxt)
     if kps.shape[0] == 0:
         return torch.empty((0, 4)), 1, S, sizes
-    k = kps.detach().cpu().numpy()
+    k = kps.detach().double().cpu().numpy()  # any real type, also those numpy does not have
     o, si = k[:, 0].astype(np.int64), k[:, 1].astype(np.int64)
     o = np.where(o < 0, o + len(sizes), o)
     if o.min() < 0 or o.max() >= len(sizes) or si.min() < 0 or si.max() > S + 2:

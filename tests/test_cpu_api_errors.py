@@ -85,3 +85,19 @@ def test_c_abi_argument_checks_without_a_device():
     assert lib.pysift_match_u8_exact(odd, 10, fake, 10, 128, *args) == -1
     assert lib.pysift_match_u8_split_fp8(fake, 10, odd, 10, 128, *args) == -1
     assert "aligned" in lib.pysift_last_error().decode()
+
+
+@pytest.mark.parametrize("dtype", [torch.float64, torch.float32, torch.float16, torch.bfloat16, torch.int64])
+def test_differentiable_keypoint_tables_of_any_type(dtype):
+    """Rows [octave, scale index, row, column, angle] of a table as torch holds
+    them, in the library's layout; types numpy lacks too."""
+    from types import SimpleNamespace
+    from pysift_b200 import _lib, grad
+    from pysift_b200.core import build_detect_config
+    sift = SimpleNamespace(_cfg=build_detect_config(5, 3, 1.6, 0.04, 10.0, False, 3, False, False, True, True))
+    table = torch.tensor([[0, 1, 30, 40, 90], [2, 3, 5, 9, 12], [1, 2, 17, 128, 250]], dtype=torch.float64).to(dtype)
+    rows, n_oct, top, sizes = grad._levels_plan(table, sift, (96, 130))
+    assert rows.dtype == torch.float32
+    assert (rows[:, 0] == torch.tensor([1, 2 * _lib.MAX_LEVELS + 3, _lib.MAX_LEVELS + 2])).all()
+    assert torch.equal(rows[:, 1:], table[:, 2:].float())
+    assert (n_oct, top) == (3, 3) and sizes[:3] == [(96, 130), (48, 65), (24, 33)]
