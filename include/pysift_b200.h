@@ -341,17 +341,20 @@ int pysift_blur_adjoint(const float* gout, int32_t gout_pitch, float* gin, int32
  * PYSIFT_MAX_LEVELS + scale index, centre row, centre column, angle in
  * degrees]; octaves 0 .. n_octaves - 1 and levels 0 .. top (n_scales <= top <=
  * n_scales + 2) of img (float, pitch in floats) are built in the workspace (a
- * row of another level yields zeros).  backward rebuilds them and writes
+ * row of another level yields zeros).  levels: n_octaves * PYSIFT_MAX_LEVELS
+ * host bytes, non-zero where kp has rows (NULL: anywhere); backward keeps a map
+ * of gradients only for those.  backward rebuilds the levels and writes
  * dL/dimg (gimg; each blur radius must be below both sides of its octave). */
 int pysift_desc_levels_workspace_size(const pysift_detect_config* cfg, int32_t H, int32_t W, int32_t n_octaves,
-                                      int32_t top, int32_t backward, size_t* bytes);
+                                      int32_t top, const uint8_t* levels, int32_t backward, size_t* bytes);
 int pysift_desc_levels_forward(const pysift_detect_config* cfg, const float* img, int32_t H, int32_t W, int32_t pitch,
-                               const float* kp, int32_t n, int32_t n_octaves, int32_t top, void* workspace,
-                               size_t workspace_bytes, float* hist, float* desc, pysift_stream_t stream);
+                               const float* kp, int32_t n, int32_t n_octaves, int32_t top, const uint8_t* levels,
+                               void* workspace, size_t workspace_bytes, float* hist, float* desc,
+                               pysift_stream_t stream);
 int pysift_desc_levels_backward(const pysift_detect_config* cfg, const float* img, int32_t H, int32_t W, int32_t pitch,
-                                const float* kp, int32_t n, int32_t n_octaves, int32_t top, void* workspace,
-                                size_t workspace_bytes, const float* hist, const float* gdesc, float* gimg,
-                                int32_t gimg_pitch, pysift_stream_t stream);
+                                const float* kp, int32_t n, int32_t n_octaves, int32_t top, const uint8_t* levels,
+                                void* workspace, size_t workspace_bytes, const float* hist, const float* gdesc,
+                                float* gimg, int32_t gimg_pitch, pysift_stream_t stream);
 int pysift_warp_f32_forward(const float* img1, int32_t hs, int32_t ws, int32_t C, const float* img2, int32_t h2,
                             int32_t w2, int32_t cw, int32_t ch, const double* hinv_host, double ox, double oy,
                             int32_t iox, int32_t ioy, float* out, pysift_stream_t stream);

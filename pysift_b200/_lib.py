@@ -114,14 +114,14 @@ EXPORTS.update({
                                                 c_void_p, c_void_p, c_void_p, c_void_p]),
     "pysift_blur_adjoint": (ctypes.c_int, [c_void_p, c_int32, c_void_p, c_int32, c_void_p, c_int32, c_int32, c_int32,
                                            c_void_p, c_int32, c_int32, c_void_p]),
-    "pysift_desc_levels_workspace_size": (ctypes.c_int, [c_void_p, c_int32, c_int32, c_int32, c_int32, c_int32,
-                                                         ctypes.POINTER(c_size_t)]),
+    "pysift_desc_levels_workspace_size": (ctypes.c_int, [c_void_p, c_int32, c_int32, c_int32, c_int32, c_void_p,
+                                                         c_int32, ctypes.POINTER(c_size_t)]),
     "pysift_desc_levels_forward": (ctypes.c_int, [c_void_p, c_void_p, c_int32, c_int32, c_int32, c_void_p, c_int32,
-                                                  c_int32, c_int32, c_void_p, c_size_t, c_void_p, c_void_p,
+                                                  c_int32, c_int32, c_void_p, c_void_p, c_size_t, c_void_p, c_void_p,
                                                   c_void_p]),
     "pysift_desc_levels_backward": (ctypes.c_int, [c_void_p, c_void_p, c_int32, c_int32, c_int32, c_void_p, c_int32,
-                                                   c_int32, c_int32, c_void_p, c_size_t, c_void_p, c_void_p, c_void_p,
-                                                   c_int32, c_void_p]),
+                                                   c_int32, c_int32, c_void_p, c_void_p, c_size_t, c_void_p, c_void_p,
+                                                   c_void_p, c_int32, c_void_p]),
     "pysift_warp_f32_forward": (ctypes.c_int, [c_void_p, c_int32, c_int32, c_int32, c_void_p, c_int32, c_int32,
                                                c_int32, c_int32, c_void_p, c_double, c_double, c_int32, c_int32,
                                                c_void_p, c_void_p]),

@@ -472,10 +472,14 @@ static int launch_adjoint_axes(const AdjArgs& a, int R, float* tmp, int tmp_pitc
 
 // The tiled kernel for the taps it is right and compiled for (the Gaussian
 // tables are symmetric bit for bit), the two-pass form for the others.
-static int launch_adjoint(const AdjArgs& a, int R, float* tmp, int tmp_pitch, cudaStream_t st) {
+static bool adjoint_tiled(const float* w, int R) {
     bool tiled = R <= ADJ_MAX_R;
-    for (int k = 0; k < R; ++k) tiled = tiled && a.w[k] == a.w[2 * R - k];
-    if (!tiled) return launch_adjoint_axes(a, R, tmp, tmp_pitch, st);
+    for (int k = 0; k < R; ++k) tiled = tiled && w[k] == w[2 * R - k];
+    return tiled;
+}
+
+static int launch_adjoint(const AdjArgs& a, int R, float* tmp, int tmp_pitch, cudaStream_t st) {
+    if (!adjoint_tiled(a.w, R)) return launch_adjoint_axes(a, R, tmp, tmp_pitch, st);
     switch (R) {
         case 0: adj_launch<0>(a, st); break;
         case 1: adj_launch<1>(a, st); break;
@@ -516,18 +520,21 @@ static int launch_desc_bwd(const DescTable& tab, const float* kp, int n, bool le
 }
 
 // Workspace of pysift_desc_levels_*: the Gaussian levels 0 .. top of every
-// octave in use, and backward a map per level from 0 .. top, each octave's
-// level-0 gradient and three buffers for the chain of adjoints.
+// octave in use, and backward a map for each level that keypoints sit on (all,
+// when `levels` is null).  Once the maps are filled the levels are not needed
+// any more: the chain of adjoints runs in their planes (0 and 1 in turn, plane
+// min(2, top) for the octave's level-0 gradient).
 struct LevelsLayout {
     int n_oct, top;
     int H[PYSIFT_MAX_OCTAVES], W[PYSIFT_MAX_OCTAVES], P[PYSIFT_MAX_OCTAVES];
-    size_t off_lev[PYSIFT_MAX_OCTAVES], off_map[PYSIFT_MAX_OCTAVES], off_g0[PYSIFT_MAX_OCTAVES], off_chain[3];
+    bool used[GD_LEVELS];
+    size_t off_lev[PYSIFT_MAX_OCTAVES], off_map[GD_LEVELS], off_tmp;
     size_t map_begin, map_end, total;
     size_t plane(int o) const { return (size_t)H[o] * P[o]; }
 };
 
-static int levels_layout(const pysift_detect_config* cfg, int H, int W, int n_oct, int top, bool backward,
-                         LevelsLayout& l) {
+static int levels_layout(const pysift_detect_config* cfg, int H, int W, int n_oct, int top, const uint8_t* levels,
+                         bool backward, LevelsLayout& l) {
     PYSIFT_CHECK_ARG(cfg, "config is NULL");
     PYSIFT_CHECK_ARG(H > 2 && W > 2, "image size %dx%d too small", H, W);
     PYSIFT_CHECK_ARG(n_oct >= 1 && n_oct <= PYSIFT_MAX_OCTAVES, "n_octaves %d outside 1..%d", n_oct,
@@ -554,12 +561,16 @@ static int levels_layout(const pysift_detect_config* cfg, int H, int W, int n_oc
     }
     for (int o = 0; o < n_oct; ++o) l.off_lev[o] = take((size_t)(top + 1) * l.plane(o) * sizeof(float));
     l.map_begin = off;
-    if (backward) {
-        for (int o = 0; o < n_oct; ++o) l.off_map[o] = take((size_t)(top + 1) * l.plane(o) * sizeof(float2));
-        l.map_end = off;
-        for (int o = 0; o < n_oct; ++o) l.off_g0[o] = take(l.plane(o) * sizeof(float));
-        for (size_t& c : l.off_chain) c = take(l.plane(0) * sizeof(float));
-    }
+    for (int o = 0; o < n_oct; ++o)
+        for (int s = 0; s <= top; ++s) {
+            const int e = o * PYSIFT_MAX_LEVELS + s;
+            l.used[e] = !levels || levels[e];
+            if (backward && l.used[e]) l.off_map[e] = take(l.plane(o) * sizeof(float2));
+        }
+    l.map_end = off;
+    bool tmp = false;  // a plane more for the two-pass adjoint
+    for (int s = -1; backward && s < top; ++s) tmp = tmp || !adjoint_tiled(cfg->blur_weights[2 + s], cfg->blur_radius[2 + s]);
+    if (tmp) l.off_tmp = take(l.plane(0) * sizeof(float));
     l.total = off;
     return PYSIFT_OK;
 }
@@ -568,7 +579,8 @@ static float* lev_at(void* ws, const LevelsLayout& l, int o, int s) {
     return reinterpret_cast<float*>(static_cast<char*>(ws) + l.off_lev[o]) + (size_t)s * l.plane(o);
 }
 static float2* map_at(void* ws, const LevelsLayout& l, int o, int s) {
-    return reinterpret_cast<float2*>(static_cast<char*>(ws) + l.off_map[o]) + (size_t)s * l.plane(o);
+    const int e = o * PYSIFT_MAX_LEVELS + s;
+    return l.used[e] ? reinterpret_cast<float2*>(static_cast<char*>(ws) + l.off_map[e]) : nullptr;
 }
 
 // Gaussian levels of the non-doubled image (pysift/core.py:1288-1343)
@@ -599,7 +611,7 @@ static void levels_table(const pysift_detect_config* cfg, void* ws, const Levels
     for (int o = 0; o < l.n_oct; ++o)
         for (int s = 0; s <= l.top; ++s) {
             const int ph = (int)cfg->desc_ph[s];
-            if (ph < 1 || ph > 200) continue;
+            if (ph < 1 || ph > 200 || !l.used[o * PYSIFT_MAX_LEVELS + s]) continue;
             DescLevel& v = tab.lv[o * PYSIFT_MAX_LEVELS + s];
             v.G = lev_at(ws, l, o, s);
             v.map = backward ? map_at(ws, l, o, s) : nullptr;
@@ -864,20 +876,21 @@ int pysift_blur_adjoint(const float* gout, int32_t gout_pitch, float* gin, int32
 }
 
 int pysift_desc_levels_workspace_size(const pysift_detect_config* cfg, int32_t H, int32_t W, int32_t n_octaves,
-                                      int32_t top, int32_t backward, size_t* bytes) {
+                                      int32_t top, const uint8_t* levels, int32_t backward, size_t* bytes) {
     PYSIFT_CHECK_ARG(bytes != nullptr, "bytes is NULL");
     LevelsLayout l = {};
-    const int rc = levels_layout(cfg, H, W, n_octaves, top, backward != 0, l);
+    const int rc = levels_layout(cfg, H, W, n_octaves, top, levels, backward != 0, l);
     if (rc) return rc;
     *bytes = l.total;
     return PYSIFT_OK;
 }
 
 int pysift_desc_levels_forward(const pysift_detect_config* cfg, const float* img, int32_t H, int32_t W, int32_t pitch,
-                               const float* kp, int32_t n, int32_t n_octaves, int32_t top, void* workspace,
-                               size_t workspace_bytes, float* hist, float* desc, pysift_stream_t stream) {
+                               const float* kp, int32_t n, int32_t n_octaves, int32_t top, const uint8_t* levels,
+                               void* workspace, size_t workspace_bytes, float* hist, float* desc,
+                               pysift_stream_t stream) {
     LevelsLayout l = {};
-    int rc = levels_layout(cfg, H, W, n_octaves, top, false, l);
+    int rc = levels_layout(cfg, H, W, n_octaves, top, levels, false, l);
     if (rc) return rc;
     PYSIFT_CHECK_ARG(img && workspace && pitch >= W && n >= 0 && (n == 0 || (kp && hist && desc)), "bad arguments");
     PYSIFT_CHECK_ARG((reinterpret_cast<uintptr_t>(workspace) & 255) == 0, "workspace must be 256-byte aligned");
@@ -895,11 +908,11 @@ int pysift_desc_levels_forward(const pysift_detect_config* cfg, const float* img
 }
 
 int pysift_desc_levels_backward(const pysift_detect_config* cfg, const float* img, int32_t H, int32_t W, int32_t pitch,
-                                const float* kp, int32_t n, int32_t n_octaves, int32_t top, void* workspace,
-                                size_t workspace_bytes, const float* hist, const float* gdesc, float* gimg,
-                                int32_t gimg_pitch, pysift_stream_t stream) {
+                                const float* kp, int32_t n, int32_t n_octaves, int32_t top, const uint8_t* levels,
+                                void* workspace, size_t workspace_bytes, const float* hist, const float* gdesc,
+                                float* gimg, int32_t gimg_pitch, pysift_stream_t stream) {
     LevelsLayout l = {};
-    int rc = levels_layout(cfg, H, W, n_octaves, top, true, l);
+    int rc = levels_layout(cfg, H, W, n_octaves, top, levels, true, l);
     if (rc) return rc;
     PYSIFT_CHECK_ARG(img && workspace && gimg && pitch >= W && gimg_pitch >= W && n >= 0 &&
                          (n == 0 || (kp && hist && gdesc)),
@@ -933,13 +946,12 @@ int pysift_desc_levels_backward(const pysift_detect_config* cfg, const float* im
             t.map = map_at(ws, l, o, s);
             t.map_pitch = P;
             if (s == cfg->n_scales && o + 1 < n_octaves) {
-                t.sub = reinterpret_cast<float*>(ws + l.off_g0[o + 1]);
+                t.sub = lev_at(ws, l, o + 1, std::min(2, top));
                 t.sub_pitch = l.P[o + 1];
             }
             return t;
         };
-        float* const chain[2] = {reinterpret_cast<float*>(ws + l.off_chain[0]),
-                                 reinterpret_cast<float*>(ws + l.off_chain[1])};
+        float* const chain[2] = {lev_at(ws, l, o, 0), lev_at(ws, l, o, 1)};
         float* cur = chain[0];
         k_adjoint_tail<<<dim3(ceil_div(Wo, 256), Ho), 256, 0, st>>>(cur, P, Ho, Wo, tail(top));
         PYSIFT_LAUNCH_CHECK("k_adjoint_tail");
@@ -948,14 +960,14 @@ int pysift_desc_levels_backward(const pysift_detect_config* cfg, const float* im
             AdjArgs a = {};
             a.in = cur;
             a.in_pitch = P;
-            a.out = s == 0 ? gimg : (s == 1 ? reinterpret_cast<float*>(ws + l.off_g0[o]) : chain[(top - s + 1) & 1]);
+            a.out = s == 0 ? gimg : (s == 1 ? lev_at(ws, l, o, std::min(2, top)) : chain[(top - s + 1) & 1]);
             a.out_pitch = s == 0 ? gimg_pitch : P;
             a.H = Ho;
             a.W = Wo;
             const int R = cfg->blur_radius[1 + s];
             for (int k = 0; k <= 2 * R; ++k) a.w[k] = cfg->blur_weights[1 + s][k];
             if (s > 0) a.tail = tail(s - 1);
-            rc = launch_adjoint(a, R, reinterpret_cast<float*>(ws + l.off_chain[2]), P, st);
+            rc = launch_adjoint(a, R, reinterpret_cast<float*>(ws + l.off_tmp), P, st);
             if (rc) return rc;
             cur = a.out;
         }

@@ -70,8 +70,9 @@ def _blur_adjoint(g, w, r, accumulate_into=None):
 def _levels_plan(kps, sift, shape):
     """What the library needs to know of a keypoint table: its rows [octave *
     MAX_LEVELS + scale index, row, column, angle] (float32, host), the octaves
-    and the top level in use, and the (rows, columns) of every octave the
-    image has (the pyramid ends before a side falls below 8)."""
+    and the top level in use, the (rows, columns) of every octave the image has
+    (the pyramid ends before a side falls below 8), and a byte per level of the
+    octaves in use, set where keypoints sit."""
     n_oct, S = sift._cfg.n_octaves, sift._cfg.n_scales
     sizes = [tuple(shape)]
     while len(sizes) < n_oct:
@@ -80,25 +81,29 @@ def _levels_plan(kps, sift, shape):
             break
         sizes.append(nxt)
     if kps.shape[0] == 0:
-        return torch.empty((0, 4)), 1, S, sizes
+        return torch.empty((0, 4)), 1, S, sizes, bytes(_lib.MAX_LEVELS)
     k = kps.detach().double().cpu().numpy()  # any real type, also those numpy does not have
     o, si = k[:, 0].astype(np.int64), k[:, 1].astype(np.int64)
     o = np.where(o < 0, o + len(sizes), o)
     if o.min() < 0 or o.max() >= len(sizes) or si.min() < 0 or si.max() > S + 2:
         raise IndexError("keypoint on an octave or level the pyramid does not have")
-    for s in np.unique(si).tolist():
+    lev = o * _lib.MAX_LEVELS + si
+    n_used = int(o.max()) + 1
+    used = np.bincount(lev, minlength=n_used * _lib.MAX_LEVELS) > 0
+    for s in np.flatnonzero(used.reshape(n_used, _lib.MAX_LEVELS).any(0)).tolist():
         if not 1 <= int(sift._cfg.desc_ph[s]) <= 200:
             raise ValueError(f"patch half-width {sift._cfg.desc_ph[s]} of scale index {s} is outside 1..200")
     rows = np.empty((k.shape[0], 4), np.float32)
-    rows[:, 0] = o * _lib.MAX_LEVELS + si
+    rows[:, 0] = lev
     rows[:, 1:] = k[:, 2:5]
-    return torch.from_numpy(rows), int(o.max()) + 1, max(int(si.max()), S), sizes
+    return torch.from_numpy(rows), n_used, max(int(si.max()), S), sizes, used.tobytes()
 
 
-def _levels_workspace(lib, sift, shape, n_oct, top, backward, device):
+def _levels_workspace(lib, sift, shape, n_oct, top, used, backward, device):
     size = ctypes.c_size_t()
-    _lib.check(lib.pysift_desc_levels_workspace_size(ctypes.byref(sift._cfg), shape[0], shape[1], n_oct, top, backward,
-                                                     ctypes.byref(size)), "pysift_desc_levels_workspace_size")
+    _lib.check(lib.pysift_desc_levels_workspace_size(ctypes.byref(sift._cfg), shape[0], shape[1], n_oct, top,
+                                                     used, backward, ctypes.byref(size)),
+               "pysift_desc_levels_workspace_size")
     # torch's blocks are 512-byte aligned
     return torch.empty(int(size.value), dtype=torch.uint8, device=device)
 
@@ -127,27 +132,28 @@ class _Descriptors(torch.autograd.Function):
     def forward(ctx, img, kps, sift):
         x = img.detach().contiguous().float()
         H, W = x.shape
-        rows, n_oct, top, sizes = _levels_plan(kps, sift, (H, W))
+        rows, n_oct, top, sizes, used = _levels_plan(kps, sift, (H, W))
         n = rows.shape[0]
         rows = rows.pin_memory().to(img.device, non_blocking=True) if n else rows.to(img.device)
         desc = torch.empty((n, 128), dtype=torch.float32, device=img.device)
         hist = torch.empty_like(desc)
         if n:
             lib = _lib.load()
-            ws = _levels_workspace(lib, sift, (H, W), n_oct, top, 0, img.device)
+            ws = _levels_workspace(lib, sift, (H, W), n_oct, top, used, 0, img.device)
             _lib.check(lib.pysift_desc_levels_forward(ctypes.byref(sift._cfg), x.data_ptr(), H, W, W, rows.data_ptr(),
-                                                      n, n_oct, top, ws.data_ptr(), ws.numel(), hist.data_ptr(),
-                                                      desc.data_ptr(), _st()), "pysift_desc_levels_forward")
+                                                      n, n_oct, top, used, ws.data_ptr(), ws.numel(),
+                                                      hist.data_ptr(), desc.data_ptr(), _st()),
+                       "pysift_desc_levels_forward")
         ctx.save_for_backward(img, hist, rows)
         ctx.sift = sift
-        ctx.plan = (n_oct, top, sizes)
+        ctx.plan = (n_oct, top, sizes, used)
         return desc
 
     @staticmethod
     def backward(ctx, gdesc):
         img, hist, rows = ctx.saved_tensors
         sift = ctx.sift
-        n_oct, top, sizes = ctx.plan
+        n_oct, top, sizes, used = ctx.plan
         x = img.detach().contiguous().float()
         H, W = x.shape
         for o, size in enumerate(sizes):
@@ -156,12 +162,12 @@ class _Descriptors(torch.autograd.Function):
                     raise ValueError(f"pysift_desc_levels_backward: radius {r} must be below both image sides")
         lib = _lib.load()
         gdesc = gdesc.contiguous().float()
-        ws = _levels_workspace(lib, sift, (H, W), n_oct, top, 1, img.device)   # levels recomputed, not stored
+        ws = _levels_workspace(lib, sift, (H, W), n_oct, top, used, 1, img.device)  # levels recomputed, not stored
         gx = torch.empty_like(x)
         _lib.check(lib.pysift_desc_levels_backward(ctypes.byref(sift._cfg), x.data_ptr(), H, W, W, rows.data_ptr(),
-                                                   rows.shape[0], n_oct, top, ws.data_ptr(), ws.numel(),
-                                                   hist.data_ptr(), gdesc.data_ptr(), gx.data_ptr(), W, _st()),
-                   "pysift_desc_levels_backward")
+                                                   rows.shape[0], n_oct, top, used, ws.data_ptr(),
+                                                   ws.numel(), hist.data_ptr(), gdesc.data_ptr(), gx.data_ptr(), W,
+                                                   _st()), "pysift_desc_levels_backward")
         return gx.to(img.dtype), None, None
 
 

@@ -96,8 +96,33 @@ def test_differentiable_keypoint_tables_of_any_type(dtype):
     from pysift_b200.core import build_detect_config
     sift = SimpleNamespace(_cfg=build_detect_config(5, 3, 1.6, 0.04, 10.0, False, 3, False, False, True, True))
     table = torch.tensor([[0, 1, 30, 40, 90], [2, 3, 5, 9, 12], [1, 2, 17, 128, 250]], dtype=torch.float64).to(dtype)
-    rows, n_oct, top, sizes = grad._levels_plan(table, sift, (96, 130))
+    rows, n_oct, top, sizes, used = grad._levels_plan(table, sift, (96, 130))
     assert rows.dtype == torch.float32
     assert (rows[:, 0] == torch.tensor([1, 2 * _lib.MAX_LEVELS + 3, _lib.MAX_LEVELS + 2])).all()
     assert torch.equal(rows[:, 1:], table[:, 2:].float())
     assert (n_oct, top) == (3, 3) and sizes[:3] == [(96, 130), (48, 65), (24, 33)]
+    assert [i for i, b in enumerate(used) if b] == [1, _lib.MAX_LEVELS + 2, 2 * _lib.MAX_LEVELS + 3]
+
+
+def test_differentiable_descriptors_keep_maps_of_named_levels_only():
+    """The backward workspace: the levels, and two floats a pixel for each level
+    the table names (the adjoint chain needs nothing beside them)."""
+    import ctypes
+    from pysift_b200 import _lib
+    from pysift_b200.core import build_detect_config
+    cfg = build_detect_config(4, 3, 1.6, 0.04, 10.0, False, 3, False, False, True, True)
+    H, W, n_oct, top = 300, 416, 3, 3
+
+    def size(used, backward):
+        n = ctypes.c_size_t()
+        assert _lib.load().pysift_desc_levels_workspace_size(ctypes.byref(cfg), H, W, n_oct, top, used, backward,
+                                                             ctypes.byref(n)) == _lib.OK
+        return n.value
+
+    planes = [-(-H >> o) * -(-(-(-W >> o)) // 32) * 32 * 4 for o in range(n_oct)]  # 256-byte multiples
+    used = (ctypes.c_uint8 * (n_oct * _lib.MAX_LEVELS))()
+    assert size(used, 0) == size(None, 0) == sum((top + 1) * p for p in planes)
+    assert size(used, 1) == size(used, 0)
+    used[1] = used[2] = used[_lib.MAX_LEVELS + 3] = 1
+    assert size(used, 1) == size(used, 0) + 2 * (2 * planes[0] + planes[1])
+    assert size(None, 1) == size(None, 0) + 2 * sum((top + 1) * p for p in planes)

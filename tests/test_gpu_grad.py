@@ -90,6 +90,40 @@ def test_descriptor_levels_match_torch_autograd(H, W, n_oct, sigma0, n):
     assert _rel(x.grad.cpu(), x64.grad.cpu()) < 1e-4
 
 
+@pytest.mark.parametrize("levels", [[(0, 2)], [(1, 1)], [(0, 0), (1, 3)], [(1, 5)], [(0, 1), (0, 2), (0, 3), (1, 2)]])
+@pytest.mark.parametrize("n_scales,sigma0", [(3, 1.6), (1, 1.6), (3, 4.0)])
+def test_descriptor_levels_named_by_the_table(n_scales, sigma0, levels, monkeypatch):
+    """Maps are kept for the levels in the table alone and the adjoint chain
+    runs in the planes of the levels: few and single levels, an octave without
+    any, the shortest chain (one scale an octave), radii of the two-pass form.
+    The same as with a map for every level, up to the order of the atomics
+    (1,000 float32 terms at most meet in a pixel: 1000 * 2^-24 = 6e-5)."""
+    import torch
+    from pysift_b200 import PySIFT, grad
+    levels = [(o, min(s, n_scales + 2)) for o, s in levels]
+    if sigma0 > 2:
+        levels = [(o, min(s, 3)) for o, s in levels]  # higher levels blur past the image
+    rng = np.random.default_rng(len(levels))
+    H, W = 101, 130
+    sift = PySIFT(double_image=False, n_octaves=2, n_scales=n_scales, sigma0=sigma0)
+    img = torch.from_numpy(_img(H, W, 7)).cuda()
+    kps = torch.tensor(np.array([[*levels[i % len(levels)], rng.integers(4, 46), rng.integers(4, 60), rng.uniform(0, 360)]
+                                 for i in range(12)], np.float64))
+    r = torch.from_numpy(rng.standard_normal((12, 128)).astype(np.float32)).cuda()
+    out = []
+    for every in (False, True):
+        if every:
+            plan = grad._levels_plan
+            monkeypatch.setattr(grad, "_levels_plan", lambda *a: (*plan(*a)[:4], b"\1" * len(plan(*a)[4])))
+        x = img.clone().requires_grad_(True)
+        d = grad.descriptors(x, kps, sift)
+        (d * r).sum().backward()
+        out.append((d.detach().cpu(), x.grad.cpu()))
+    assert torch.equal(out[0][0], out[1][0])
+    assert float(out[0][1].abs().max()) > 0
+    assert _rel(out[0][1], out[1][1]) < 6e-5
+
+
 def test_descriptor_levels_refuse_what_the_pyramid_lacks():
     import torch
     from pysift_b200 import grad
