@@ -124,6 +124,44 @@ def test_descriptor_levels_named_by_the_table(n_scales, sigma0, levels, monkeypa
     assert _rel(out[0][1], out[1][1]) < 6e-5
 
 
+@pytest.mark.parametrize("s,n", [(1, 1), (2, 40), (3, 700)])
+def test_single_level_descriptor_entry_points(s, n):
+    """pysift_desc_f32_forward / _backward on one Gaussian level against the
+    call over all levels: the same descriptor bytes, and through the adjoints
+    of the blurs the same gradient of the image up to the order of the atomics
+    (6e-5, see above)."""
+    import torch
+    from pysift_b200 import _lib, grad
+    lib, st = _lib.load(), torch.cuda.current_stream().cuda_stream
+    rng = np.random.default_rng(n)
+    H, W = 90, 117
+    sift = _sift(1)
+    _, _, base, incs = grad.pyramid_params(sift)
+    blurs = [base, *incs[:s]]
+    x = torch.from_numpy(_img(H, W, 9)).cuda().requires_grad_(True)
+    at = np.stack([rng.integers(0, H, n), rng.integers(0, W, n), rng.uniform(0, 360, n)], 1)  # the rim too
+    kps = torch.tensor(np.concatenate([np.tile([0.0, s], (n, 1)), at], 1))
+    d = grad.descriptors(x, kps, sift)
+    r = torch.from_numpy(rng.standard_normal(d.shape).astype(np.float32)).cuda()
+    (d * r).sum().backward()
+
+    level = x.detach()
+    for w, radius in blurs:
+        level = grad._blur(level, w, radius)
+    kp = torch.from_numpy(at.astype(np.float32)).cuda()
+    hist, desc = torch.empty((n, 128), device="cuda"), torch.empty((n, 128), device="cuda")
+    ph = int(sift._cfg.desc_ph[s])
+    _lib.check(lib.pysift_desc_f32_forward(level.data_ptr(), H, W, W, kp.data_ptr(), n, ph, hist.data_ptr(),
+                                           desc.data_ptr(), st), "forward")
+    assert torch.equal(desc, d.detach())
+    g = torch.zeros_like(level)
+    _lib.check(lib.pysift_desc_f32_backward(level.data_ptr(), H, W, W, kp.data_ptr(), n, ph, hist.data_ptr(),
+                                            r.data_ptr(), g.data_ptr(), st), "backward")
+    for w, radius in reversed(blurs):
+        g = grad._blur_adjoint(g, w, radius)
+    assert _rel(g.cpu(), x.grad.cpu()) < 6e-5
+
+
 def test_descriptor_levels_refuse_what_the_pyramid_lacks():
     import torch
     from pysift_b200 import grad
