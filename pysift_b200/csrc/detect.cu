@@ -501,14 +501,16 @@ __global__ void __launch_bounds__(PR_NT) k_prefilter_rows(double* __restrict__ c
 // float32.  On the 2x grid the output columns 2k-1 and 2k interpolate the
 // same 4 input columns (their input coordinates share the floor k-1), and
 // likewise the output rows 2j-1 and 2j, so the grid splits into 2x2 quads of
-// common support.  A lane owns a column pair and its warp walks down the row
+// common support (the coordinates of 2k-1 and 2k lie (n-k)/(2n-1) above k-1 and
+// k/(2n-1) below k on n inputs, far more than their rounding, and the last one
+// is n-1 exactly).  A lane owns a column pair and its warp walks down the row
 // pairs of a tile: of the 16 coefficients 4 are new at each step (the window
 // in shared memory holds mirrored rows and columns past the image's edges, so
 // that every support is contiguous), the column weights stay in registers,
 // and each c * wy_a serves both columns.  What is left is the 160 float64
 // operations of a quad (108 us for the 48 Mpixel of a doubled 4000x3000 image
 // at 64 a cycle and SM); with all 16 coefficients and both axes' weights
-// fetched from shared memory per quad it was issue-bound: 283 -> 196 us there.
+// fetched from shared memory per quad it was issue-bound: 283 -> 178 us there.
 // Three blocks an SM (80 registers) hide the chains' latency best.
 constexpr int ZI_T = 256, ZI_W = ZI_T / 32;
 constexpr int ZI_MAX_PAIRS = 16;                       // row pairs of a warp, at most
@@ -553,8 +555,6 @@ __global__ void __launch_bounds__(ZI_T, 3) k_zoom_interp(const double* coef, int
     const bool cva = xa >= 0 && xa < OW && zoom_axis(xa, W, zx, sa, wxa);
     const bool cvb = xb < OW && zoom_axis(xb, W, zx, sb, wxb);
     const int col = cva ? sa - xlo : (cvb ? sb - xlo : 0);
-    // both columns of a pair share their support wherever both exist
-    const bool odd_pair = cva && cvb && sa != sb;
     asm volatile("cp.async.wait_all;" ::: "memory");
     __syncthreads();
     const bool pair_stores = (out_pitch & 1) == 0 && (reinterpret_cast<uintptr_t>(out) & 7) == 0;
@@ -599,25 +599,6 @@ __global__ void __launch_bounds__(ZI_T, 3) k_zoom_interp(const double* coef, int
                     t[1][0] += p1 * wxa[b];
                     t[1][1] += p1 * wxb[b];
                 }
-            }
-            if (odd_pair || (ya >= 0 && yb >= 0 && ya != yb)) {
-                // supports that differ: each output from its own
-                for (int u = 0; u < 2; ++u)
-                    for (int w = 0; w < 2; ++w) {
-                        const int y0 = u ? yb : ya, x0 = (w ? sb : sa) - xlo;
-                        double s = 0.0;
-                        if (y0 >= 0 && (w ? cvb : cva))
-                            for (int a = 0; a < 4; ++a)
-                                for (int b = 0; b < 4; ++b) {
-                                    double coeff = win[y0 + a][x0 + b] * rw[i + u][a];
-                                    coeff *= w ? wxb[b] : wxa[b];
-                                    s += coeff;
-                                }
-                        if (u == 0 && w == 0) t[0][0] = s;
-                        if (u == 0 && w == 1) t[0][1] = s;
-                        if (u == 1 && w == 0) t[1][0] = s;
-                        if (u == 1 && w == 1) t[1][1] = s;
-                    }
             }
 #pragma unroll
             for (int u = 0; u < 2; ++u) {
@@ -1309,8 +1290,10 @@ __device__ __forceinline__ float min3(float a, float b, float c) {
 // scales come from registers, the neighbours' by shuffle.  Extrema are rare
 // (0.2 % of the pixels), so their bits go into the zeroed mask by atomics.
 // Bound by the latency of the level loads (24 bytes a pixel): eight blocks an
-// SM at 64 registers (a few spills on the rare path) beat five with two rows
-// in flight.  Staging 32 x 32 tiles in shared memory instead cost the halo's
+// SM at 64 registers beat five with two rows in flight; the spills this costs (0,
+// 48, 160, 228 and 496 bytes loaded for 1 .. 5 scales, by the compiler's count)
+// leave every scale count faster than the staged tiles: whole detections at
+// 1023x767 1.05, 1.10, 1.19, 1.17 and 1.13 times as fast.  Staging 32 x 32 tiles in shared memory instead cost the halo's
 // sectors, a store and a load per value and a barrier: both launches of a
 // 4000x3000 detection (1.54 GB of levels, 235 us at the copy rate, and the
 // retry's empty grid) 411 -> 280 us, of a 640x480 one 19 -> 13.

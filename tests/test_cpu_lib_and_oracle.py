@@ -228,3 +228,15 @@ def test_chained_kernels_wait_first_and_claim_no_read_only_inputs():
         params, first = kernels[k]
         assert first == "chain_begin();", k
         assert not re.search(r"\bconst\b[^,]*__restrict__", params), k
+
+
+@pytest.mark.parametrize("sizes", [range(2, 2000), [4096, 9973, 65536, 100003, 1 << 20]])
+def test_zoom2x_pairs_share_their_support(sizes):
+    """What the 2x zoom kernel relies on, in its arithmetic: the coordinate
+    k * ((n - 1) / (2 n - 1)) of outputs 2 j - 1 and 2 j has the floor j - 1 (0 for
+    output 0, and n - 1 for the last), and none passes n - 1."""
+    for n in sizes:
+        c = np.arange(2 * n, dtype=np.float64) * ((n - 1) / (2 * n - 1))
+        want = (np.arange(2 * n) + 1) // 2 - 1
+        want[0], want[-1] = 0, n - 1
+        assert np.array_equal(np.floor(c).astype(np.int64), want) and c[-1] == n - 1
