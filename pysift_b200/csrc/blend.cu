@@ -24,14 +24,6 @@ namespace pysift {
 
 constexpr double BL_INF = 1e18;
 
-__device__ __forceinline__ int refl_half(int i, int n) {
-    while (i < 0 || i >= n) {
-        if (i < 0) i = -i - 1;
-        if (i >= n) i = 2 * n - 1 - i;
-    }
-    return i;
-}
-
 __device__ __forceinline__ int refl_101(int i, int n) {
     if (n == 1) return 0;
     while (i < 0 || i >= n) {
@@ -445,8 +437,8 @@ __global__ void k_sobel_cost(const float* __restrict__ avg, const float* __restr
         return;
     }
     const long long p = (long long)y * W + x;
-    const int xl = refl_half(x - 1, W), xr = refl_half(x + 1, W);
-    const int yu = refl_half(y - 1, H), yd = refl_half(y + 1, H);
+    const int xl = reflect_idx(x - 1, W), xr = reflect_idx(x + 1, W);
+    const int yu = reflect_idx(y - 1, H), yd = reflect_idx(y + 1, H);
     auto dxr = [&](int r) {  // the axis-1 derivative on row r, as float32
         return (double)(float)((double)avg[(long long)r * W + xr] - (double)avg[(long long)r * W + xl]);
     };
@@ -972,8 +964,8 @@ __global__ void k_pyr_rows(const Level0 src, const PyrLevel in, int W, int H, fl
     for (int c = 0; c < NC; ++c) s[c] = w9.w[4] * a[c];
 #pragma unroll
     for (int k = 4; k >= 1; --k) {
-        pyr_load<NC, L0>(src, in, (long long)refl_half(y - k, H) * W + x, a);
-        pyr_load<NC, L0>(src, in, (long long)refl_half(y + k, H) * W + x, b);
+        pyr_load<NC, L0>(src, in, (long long)reflect_idx(y - k, H) * W + x, a);
+        pyr_load<NC, L0>(src, in, (long long)reflect_idx(y + k, H) * W + x, b);
         const double w = w9.w[4 - k];
 #pragma unroll
         for (int c = 0; c < NC; ++c) s[c] = s[c] + (a[c] + b[c]) * w;
@@ -1016,8 +1008,8 @@ __global__ void k_pyr_cols(const float* t1, const float* t2, int W, int Wo,
     for (int c = 0; c < NC; ++c) s[c] = w9.w[4] * a[c];
 #pragma unroll
     for (int k = 4; k >= 1; --k) {
-        load(refl_half(col - k, W), a);
-        load(refl_half(col + k, W), b);
+        load(reflect_idx(col - k, W), a);
+        load(reflect_idx(col + k, W), b);
         const double w = w9.w[4 - k];
 #pragma unroll
         for (int c = 0; c < NC; ++c) s[c] = s[c] + (a[c] + b[c]) * w;

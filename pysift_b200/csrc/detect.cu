@@ -1290,13 +1290,14 @@ __device__ __forceinline__ float min3(float a, float b, float c) {
 // scales come from registers, the neighbours' by shuffle.  Extrema are rare
 // (0.2 % of the pixels), so their bits go into the zeroed mask by atomics.
 // Bound by the latency of the level loads (24 bytes a pixel): eight blocks an
-// SM at 64 registers beat five with two rows in flight; the spills this costs (0,
-// 48, 160, 228 and 496 bytes loaded for 1 .. 5 scales, by the compiler's count)
-// leave every scale count faster than the staged tiles: whole detections at
-// 1023x767 1.05, 1.10, 1.19, 1.17 and 1.13 times as fast.  Staging 32 x 32 tiles in shared memory instead cost the halo's
-// sectors, a store and a load per value and a barrier: both launches of a
-// 4000x3000 detection (1.54 GB of levels, 235 us at the copy rate, and the
-// retry's empty grid) 411 -> 280 us, of a 640x480 one 19 -> 13.
+// SM at 64 registers beat five with two rows in flight; the spills this costs
+// (0, 48, 160, 228 and 496 bytes loaded for 1 .. 5 scales, by the compiler's
+// count) leave every scale count faster than with staged tiles: whole
+// detections at 1023x767 1.05, 1.10, 1.19, 1.17 and 1.13 times as fast.
+// Staging 32 x 32 tiles in shared memory cost the halo's sectors, a store and a
+// load per value and a barrier: both launches of a 4000x3000 detection (1.54 GB
+// of levels, 235 us at the copy rate, and the retry's empty grid) 411 -> 280
+// us, of a 640x480 one 19 -> 13.
 constexpr int EX_T = 128, EX_COLS = 62;
 
 template <int NL>

@@ -701,7 +701,8 @@ __global__ void k_warp_f32_fwd(const WarpF32Args a) {
 // gradients to the next lane when that lane's left-hand corners are the same
 // pixels: half the float atomics.  66.7 -> 46.7 us for the 1024x768x3 views of
 // a canvas of 1 Mpixel, whose images, gradients and output gradient are 12 us
-// of DRAM traffic.
+// of DRAM traffic.  Eight blocks an SM leave 64 registers; three channels spill
+// 132 bytes under that.
 constexpr int WB_T = 128;
 template <int C>
 __global__ void __launch_bounds__(WB_T, 8) k_warp_f32_bwd(const __grid_constant__ WarpF32Args a) {

@@ -15,9 +15,11 @@
 // issues tcgen05.mma (kind::f16 / f8f6f4 / i8, fp32 or s32 accumulator in
 // tensor memory, two accumulators of 128 columns) and eight warps reduce the
 // finished accumulator, read back with tcgen05.ld (two warps per TMEM lane
-// quadrant, each half of the tile's columns); mbarriers link the three roles.  Train tiles are split into segments so that the grid fills the
-// SMs; a merge kernel combines the segments of each row and applies the ratio
-// test; k_match_mutual keeps mutual matches (pysift/core.py:2574-2701,
+// quadrant, each half of the tile's columns); mbarriers link the three roles.
+// Train tiles are split into segments so that the grid fills the SMs; a merge
+// kernel combines the segments of each row and applies the ratio test (rows of
+// the fp16 mode that it cannot settle go through k_match_recheck_f16, or
+// k_match_recheck_runs_f16 when there are many); k_match_mutual keeps mutual matches (pysift/core.py:2574-2701,
 // 2840-2940).
 //
 // The reduction works on 32-column chunks: a chunk's key is its largest
@@ -52,7 +54,8 @@
 //             division does not commute with the maximum): column-level top-2.
 // Ties are broken towards the lower index in every direction: a scan visits
 // train entries in increasing index order and replaces the best only on a
-// strictly larger key; segments merge in index order.
+// strictly larger key; SIM_I8 merges its segments in index order, the others
+// merge states that carry the index, in any order.
 #include <algorithm>
 #include <climits>
 #include <cstdint>
@@ -675,8 +678,7 @@ __device__ __forceinline__ void warp_top2_u64(unsigned long long& kb, unsigned l
     }
 }
 
-// Segments of one chunk-level scan, merged in segment order (every lane
-// reads the same parts).
+// The state of the lane at distance o in a butterfly of the warp.
 __device__ __forceinline__ Top3 shfl_xor_top3(const Top3& t, int o) {
     Top3 r;
     r.k1 = __shfl_xor_sync(FULL_MASK, t.k1, o);
@@ -713,8 +715,8 @@ __device__ __forceinline__ Top3 merge_parts(const Top3* __restrict__ part, int i
 // Rows of a 32-column chunk read by a warp with consecutive lanes on one row:
 // LPR lanes hold a row's 16-byte words, so a load instruction covers 32 / LPR
 // rows of a few cache lines.  A row a lane touches 32 lines each time, which
-// bound both merges: 24.8 -> 11.7 us for two 8192x128 uint8 sets.  get(j, row) is the lane's share of row j's sum;
-// the LPR shares of each row are then added by halves across the lanes, so
+// bound both merges: 24.8 -> 11.7 us for two 8192x128 uint8 sets.  get(j) is the
+// lane's share of row j's sum; the LPR shares of each row are then added by halves across the lanes, so
 // that lane l ends with the whole sum of row chunk_row<LPR>(l).
 template <int LPR>
 __device__ __forceinline__ int chunk_row(int lane) {
@@ -1049,10 +1051,10 @@ struct F16Row {
     }
 };
 
-// Merge the chunk-level segments of one SIM_F16 scan (in segment order) and
-// settle the row from its two best chunks (one warp per row): the two largest
-// of their columns give the exact best F1 (lowest index on ties) and second F2
-// among them.  Every column of the other chunks has an fp32 value <= k3 (the
+// Merge the chunk-level segments of one SIM_F16 scan (merge_parts) and settle
+// the row from its two best chunks (one warp per row): the two largest of their
+// columns give the exact best F1 (lowest index on ties) and second F2 among
+// them.  Every column of the other chunks has an fp32 value <= k3 (the
 // third chunk's largest), so its exact value is <= k3 + e and its fp16
 // similarity <= U = fp16(k3 + e); the row is settled when U <= F2 and U < F1
 // (a column tying F1 could have a lower index).  Unsettled rows are appended
