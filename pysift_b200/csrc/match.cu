@@ -255,6 +255,9 @@ struct ScanSide {
     const float* scale_t;  //         and per train row
     int nseg, seg_tiles;   // segments of the train side and their tiles
     void* part;            // [n_q][nseg] Top3 (chunk level; SIM_I8: Top2 of columns)
+    const unsigned* blockmax;  // SIM_F16: the largest query norm of each preparation block, as float bits,
+    int n_blockmax;
+    unsigned* maxnorm;         //          and where the largest of all goes
 };
 
 struct RowScanArgs {
@@ -383,6 +386,7 @@ __global__ void __launch_bounds__(SCAN_THREADS, 2) k_match_rows(const __grid_con
     __shared__ __align__(8) uint64_t bar_full[NS], bar_empty[NS], bar_acc_full[2], bar_acc_empty[2], bar_q, bar_done;
     __shared__ uint32_t tmem_base;
     __shared__ volatile int s_abort;
+    __shared__ unsigned s_max;
     __shared__ Top3 s_half[MT];  // Top2 in the first 16 bytes for SIM_I8
 
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
@@ -413,6 +417,7 @@ __global__ void __launch_bounds__(SCAN_THREADS, 2) k_match_rows(const __grid_con
         mbar_init(&bar_q, 1);
         mbar_init(&bar_done, 1);
         s_abort = 0;
+        s_max = 0u;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
@@ -517,6 +522,16 @@ __global__ void __launch_bounds__(SCAN_THREADS, 2) k_match_rows(const __grid_con
         int i1 = 0x7fffffff, j1 = 0x7fffffff;
         Top3 tc;  // chunk-level state (CHUNKED)
         top3_init(tc);
+        if (MODE == SIM_F16 && bl == 0) {
+            // the side's largest query norm, for the merges, while the first
+            // accumulator is on its way (an atomic maximum in the preparation
+            // wanted a memset before it)
+            unsigned m = 0u;
+            for (int i = tid; i < args.n_blockmax; i += MATCH_THREADS) m = max(m, args.blockmax[i]);
+            atomicMax(&s_max, m);
+            asm volatile("bar.sync 1, %0;" ::"n"(MATCH_THREADS) : "memory");
+            if (tid == 0) *args.maxnorm = s_max;
+        }
         bool fail = false;
         for (int p = 0; p < nt; ++p) {
             const int a = p & 1;
@@ -1262,10 +1277,9 @@ __global__ void __launch_bounds__(1024) k_match_mutual(const int* fbest, const i
 // into the tiled layout with zero rows up to whole tiles, and what the mode
 // needs of each row.  A 16-byte chunk a thread, a row's chunks in adjacent
 // lanes.
-//   SIM_F16    row L2 norms and the largest of each set, rounded up with a
-//              relative margin of 2^-20, the largest as float bits
-//              (non-negative floats order as their bits); maxnorm is zeroed
-//              beforehand
+//   SIM_F16    row L2 norms, rounded up with a relative margin of 2^-20, and the
+//              largest of each block as float bits (non-negative floats order
+//              as their bits)
 //   SIM_I8     the rows alone
 //   DIST_U8    |row|^2 as int32
 //   SPLIT_FP8  |row|^2 as int32 and float32 (exact: below 2^24), and
@@ -1281,13 +1295,13 @@ struct PrepSide {
     uint8_t* t;   // SPLIT_FP8: the train side
     int* norm;
     float* fnorm;
-    unsigned* maxnorm;
+    unsigned* blockmax;  // one entry a block of the side
 };
 struct PrepArgs {
     PrepSide side[2];
     int blocks0;
     int RB;       // bytes of a row
-    int* ctl;     // zeroed by the first block except for SIM_F16
+    int* ctl;     // zeroed by the first block
 };
 constexpr int PREP_T = 256, CTL_INTS = 8;
 
@@ -1317,9 +1331,8 @@ __global__ void __launch_bounds__(PREP_T) k_match_prep(const __grid_constant__ P
     if (MODE == SIM_F16) {
         if (threadIdx.x == 0) s_max = 0u;
         __syncthreads();
-    } else if (blockIdx.x == 0 && threadIdx.x < CTL_INTS) {
-        a.ctl[threadIdx.x] = 0;
     }
+    if (blockIdx.x == 0 && threadIdx.x < CTL_INTS) a.ctl[threadIdx.x] = 0;
     uint4 v = make_uint4(0u, 0u, 0u, 0u);
     if (r < z.n) v = reinterpret_cast<const uint4*>(z.rows)[g];
     const bool in = r < z.n_pad;
@@ -1366,7 +1379,7 @@ __global__ void __launch_bounds__(PREP_T) k_match_prep(const __grid_constant__ P
             atomicMax(&s_max, __float_as_uint(nrm));
         }
         __syncthreads();
-        if (threadIdx.x == 0 && s_max) atomicMax(z.maxnorm, s_max);
+        if (threadIdx.x == 0) z.blockmax[(int)blockIdx.x - (sd ? a.blocks0 : 0)] = s_max;
     }
 }
 
@@ -1440,9 +1453,9 @@ static int launch_scan_mode(int mode, const RowScanArgs& a, int D, int blocks, c
 
 struct MatchLayout {
     // off_ctl: int[8] = error flag, SIM_F16 recheck counts (forward, backward),
-    // max row norms (set 1, set 2) as float bits
+    // max row norms (set 1, set 2) as float bits (written by the scan)
     size_t off_fpart, off_bpart, off_fbest, off_fpass, off_fdist, off_bbest, off_bpass, off_bdist, off_ctl;
-    size_t off_rl0, off_rl1, off_nrm;
+    size_t off_rl0, off_rl1, off_nrm, off_bmax;
     size_t off_na, off_nb, off_fna, off_fnb;
     // the scan operands in the tiled layout (rows padded to whole tiles):
     // query side and train side of each set (the same buffer except for the
@@ -1452,6 +1465,7 @@ struct MatchLayout {
 };
 
 static int pad_rows(int n) { return ceil_div(n, MT) * MT; }
+static int prep_blocks(int n, int RB) { return (int)ceil_div_ll((long long)pad_rows(n) * (RB / 16), PREP_T); }
 
 // exact: 0 = fp16 similarity (and int8 similarity, whose D-byte rows fit in
 // its buffers), 1 = exact via unsigned 8-bit MMAs, 2 = exact via split e4m3
@@ -1475,11 +1489,12 @@ static MatchLayout match_layout(int n1, int n2, int D, int exact) {
     l.off_bpass = take((size_t)n2 * 4);
     l.off_bdist = take((size_t)n2 * 4);
     l.off_ctl = take(CTL_INTS * sizeof(int));
-    l.off_rl0 = l.off_rl1 = l.off_nrm = 0;
+    l.off_rl0 = l.off_rl1 = l.off_nrm = l.off_bmax = 0;
     if (exact == 0) {
         l.off_rl0 = take((size_t)n1 * 4);
         l.off_rl1 = take((size_t)n2 * 4);
         l.off_nrm = take(((size_t)n1 + n2) * 4);
+        l.off_bmax = take(((size_t)prep_blocks(n1, 2 * D) + prep_blocks(n2, 2 * D)) * 4);
     }
     l.off_na = l.off_nb = l.off_fna = l.off_fnb = 0;
     if (exact == 1 || exact == 2) {  // |row|^2 as int32 and as float32, padded to whole tiles
@@ -1529,17 +1544,16 @@ static int run_match(int mode, const uint8_t* rows_a, int n1, const uint8_t* row
     float* fna = !sim ? wsp<float>(ws, l.off_fna) : nullptr;
     float* fnb = !sim ? wsp<float>(ws, l.off_fnb) : nullptr;
     float* hna = mode == SIM_F16 ? wsp<float>(ws, l.off_nrm) : nullptr;
+    unsigned* bmax = mode == SIM_F16 ? wsp<unsigned>(ws, l.off_bmax) : nullptr;
     {
         PrepArgs pa;
         pa.RB = mode == SIM_F16 ? 2 * D : D;
         pa.ctl = ctl;
-        pa.side[0] = PrepSide{rows_a, n1, p1, qa, ta, na, mode == SIM_F16 ? hna : fna, maxnorm};
-        pa.side[1] = PrepSide{rows_b, n2, p2, qb, tb, nb, mode == SIM_F16 ? hna + n1 : fnb, maxnorm + 1};
-        const int KC = pa.RB / 16;
-        pa.blocks0 = (int)ceil_div_ll((long long)p1 * KC, PREP_T);
-        const int blocks = pa.blocks0 + (int)ceil_div_ll((long long)p2 * KC, PREP_T);
+        pa.blocks0 = prep_blocks(n1, pa.RB);
+        pa.side[0] = PrepSide{rows_a, n1, p1, qa, ta, na, mode == SIM_F16 ? hna : fna, bmax};
+        pa.side[1] = PrepSide{rows_b, n2, p2, qb, tb, nb, mode == SIM_F16 ? hna + n1 : fnb, bmax ? bmax + pa.blocks0 : nullptr};
+        const int blocks = pa.blocks0 + prep_blocks(n2, pa.RB);
         if (mode == SIM_F16) {
-            PYSIFT_CUDA_TRY(cudaMemsetAsync(ctl, 0, CTL_INTS * sizeof(int), st));
             k_match_prep<SIM_F16><<<blocks, PREP_T, 0, st>>>(pa);
         } else if (mode == SIM_I8) {
             k_match_prep<SIM_I8><<<blocks, PREP_T, 0, st>>>(pa);
@@ -1557,8 +1571,10 @@ static int run_match(int mode, const uint8_t* rows_a, int n1, const uint8_t* row
     float* fdist = wsp<float>(ws, l.off_fdist);
     float* bdist = wsp<float>(ws, l.off_bdist);
     RowScanArgs s;
-    s.side[0] = ScanSide{qa, tb, n1, n2, fnb, nb, sa, sb, 1, 1, wsp<void>(ws, l.off_fpart)};
-    s.side[1] = ScanSide{qb, ta, n2, n1, fna, na, sb, sa, 1, 1, wsp<void>(ws, l.off_bpart)};
+    const int b1 = prep_blocks(n1, 2 * D), b2 = prep_blocks(n2, 2 * D);
+    s.side[0] = ScanSide{qa, tb, n1, n2, fnb, nb, sa, sb, 1, 1, wsp<void>(ws, l.off_fpart), bmax, b1, maxnorm};
+    s.side[1] = ScanSide{qb, ta, n2, n1, fna, na, sb, sa, 1, 1, wsp<void>(ws, l.off_bpart), bmax ? bmax + b1 : nullptr, b2,
+                         maxnorm + 1};
     s.error = err;
     scan_split(s.side);
     s.blocks0 = ceil_div(n1, MT) * s.side[0].nseg;
@@ -1580,8 +1596,10 @@ static int run_match(int mode, const uint8_t* rows_a, int n1, const uint8_t* row
         const dim3 grid(2 * sm_count() / RECHECK_C * RECHECK_C);
         launch_chained(D == 64 ? k_match_recheck_f16<64> : k_match_recheck_f16<128>, grid, RECHECK_T, 0, st, m);
         PYSIFT_LAUNCH_CHECK("k_match_recheck_f16");
-        launch_chained(D == 64 ? k_match_recheck_runs_f16<64> : k_match_recheck_runs_f16<128>, grid, RECHECK_T, 0, st, m);
-        PYSIFT_LAUNCH_CHECK("k_match_recheck_runs_f16");
+        if (n1 + (long long)n2 > RECHECK_FEW) {
+            launch_chained(D == 64 ? k_match_recheck_runs_f16<64> : k_match_recheck_runs_f16<128>, grid, RECHECK_T, 0, st, m);
+            PYSIFT_LAUNCH_CHECK("k_match_recheck_runs_f16");
+        }
     } else {
         if (mode == SIM_I8) k_match_merge_i8<<<blocks, 256, 0, st>>>(m);
         else (D == 64 ? k_match_merge_u8<64> : k_match_merge_u8<128>)<<<blocks, 256, 0, st>>>(m);
